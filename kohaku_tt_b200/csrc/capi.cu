@@ -289,6 +289,8 @@ extern "C" int ktt_b200_sdpa_backward_supported(const ktt_b200_attn_args* a) {
     return 1;
 }
 
+static bool row_per_query(const AttnParams& p) { return p.mask_dtype != KTT_B200_MASK_NONE && p.ms[2] != 0 && p.sq > 1; }
+
 extern "C" int ktt_b200_sdpa_forward(const ktt_b200_attn_args* a, void* stream) {
     if (const char* why = forward_refusal(a)) {
         note_call(4);
@@ -321,6 +323,12 @@ extern "C" int ktt_b200_sdpa_forward(const ktt_b200_attn_args* a, void* stream) 
         p.fwd_done_counter = (usable && a->workspace_bytes >= 256) ? static_cast<int32_t*>(a->workspace) + 1 : nullptr;
         return launch_forward_tc5(p, st);
     }
+    // What is left for AUTO: head dims those kernels are not built for and masks with a row per
+    // query. The latter need their workspace; a caller that brings none keeps the warp-MMA kernel.
+    if (a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_takes(p) && (!row_per_query(p) || a->workspace_bytes >= forward_pair_workspace(p))) {
+        note_call(0);
+        return launch_forward_pair(p, a->workspace, a->workspace_bytes, st);
+    }
     note_call(1);
     return launch_forward_mma(p, st);
 }
@@ -334,8 +342,9 @@ extern "C" int64_t ktt_b200_sdpa_forward_workspace(const ktt_b200_attn_args* a) 
     AttnParams p;
     to_params(a, p);
     const char* why = nullptr;
-    if (!forward_tc5_takes(p, &why)) return 0;   // the warp-MMA kernel has no use for one
-    return forward_row_workspace(p);             // the same 256 bytes for both tcgen05 kernels
+    if (forward_tc5_takes(p, &why)) return forward_row_workspace(p);   // the same 256 bytes for both
+    if (a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_takes(p)) return forward_pair_workspace(p);
+    return 0;                                                          // the warp-MMA kernel has no use for one
 }
 
 extern "C" int ktt_b200_forward_streams_per_sm(void) { return forward_row_occupancy(); }

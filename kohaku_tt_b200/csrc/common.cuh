@@ -204,6 +204,13 @@ bool forward_row_takes(const AttnParams& p, const char** why);
 int64_t forward_row_workspace(const AttnParams& p);
 int launch_forward_row(const AttnParams& p, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
 int forward_row_occupancy();
+// Head dims up to 128 that are multiples of 8, masks of any shape (fwd_pair.cu). The workspace
+// (optional without a mask that has a row per query; forward_pair_workspace() bytes) starts with
+// the work counter, which must be zero and is left zero; the plan of such a mask behind it is
+// written by the call, which then clears the counter itself.
+bool forward_pair_takes(const AttnParams& p);
+int64_t forward_pair_workspace(const AttnParams& p);
+int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
 // 0, or KTT_B200_ERR_DEVICE_WAIT with the code of the first wait that ran out (cleared).
 int device_status(int* code);
 // Test support: launches one warp whose bounded wait runs out after ~1e5 cycles.

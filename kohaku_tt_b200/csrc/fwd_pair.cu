@@ -1,0 +1,1280 @@
+// Forward on the Blackwell tensor path for what the other two tcgen05 kernels are not built for:
+// head dims that are any multiple of 8 up to 128, and masks with a row per query. TMA tile
+// loads, tcgen05.mma with accumulators in tensor memory, online softmax with one thread per
+// query row.
+//
+// A persistent CTA per SM works on two 128-row query tiles at a time, A and B:
+//
+//   warps 0-3, 4-7     softmax of tile A and of tile B: thread r owns query row r and all 128
+//                      keys of a block, with its own running maximum and sum; it writes P (bf16)
+//                      to tensor memory and rescales O only when the maximum moved by more than
+//                      2^8 (the lazy rescale of ktt_flash/compute.cpp, flash.md "row reference").
+//                      No two threads ever exchange anything inside the loop.
+//   warps 8, 9         issue S = Q K^T and O += P V (P read from tensor memory) of A and of B: while
+//                      one tile is in its exponentials the tensor core serves the other
+//   warp 10            TMA loads of Q and of a ring of K and V tiles, and the draw of the work
+//
+// These calls ran on the warp-MMA kernel before (mma.sync, 64-row CTAs). Measured on B200: 16 x
+// 16 heads x 257 rows, D 80: 220 -> 55 us; 2 x 16 heads x 2048, D 64, a causal mask with padding
+// as a bf16 tensor: 577 -> 104 us, of which the plan of the mask is 5.
+//
+// Tensor memory (512 columns): S_A, S_B (128 each); head dims up to 64: P_A, P_B (64 each) and
+// O_A, O_B (64 each), so that the next scores can be computed while P V still reads P; up to 128:
+// P overwrites the scores it came from, O_A, O_B (128 each). Head dims between two sizes are
+// zero-filled by TMA; the products run over ceil(D / 16) steps and ceil(Dv / 16) columns only.
+//
+// Two ways to use the two tiles:
+//   pair   A and B are neighbours in the list of (query tile, head) of one K / V head: one
+//          K / V stream serves both, which halves the traffic from L2
+//   dual   (few tiles per SM) A and B are the same query tile, A working on the first half of
+//          its key blocks and B on the rest; A's threads then read B's unnormalised O straight
+//          out of tensor memory. The longest tile's serial chain is halved. Always A then B:
+//          the bits do not depend on timing.
+//
+// Masks. One row per (batch, head): the 128 terms of a block are fetched by 128 threads and
+// shared through shared memory. A row per query: a small kernel in front (mask_plan_kernel)
+// sorts the mask into 32-row x 128-key pieces - hidden, without effect, yes / no, values -
+// and lays the pieces that matter out so that a warp reads them with coalesced 16-byte loads;
+// blocks hidden from a whole tile are not visited at all.
+//
+// Arithmetic contract as in the reference's flash forward (ktt_flash/compute.cpp:193-491):
+// base-2 softmax with fp32 statistics, P rounded to bf16 before P V, fp32 accumulation, O / l
+// and lse = ln2 (m + log2 l) at the end.
+//
+// Every wait on an mbarrier is bounded: when one runs out the CTA records a code in a
+// host-visible status word, stops waiting everywhere, frees its tensor memory and exits.
+// Launched with programmatic stream serialization: everything before `griddepcontrol.wait`
+// may overlap the tail of the previous kernel in the stream.
+#include <cstdlib>
+
+#include "tc5.cuh"
+
+namespace ktt {
+using namespace tc5;
+namespace {
+
+constexpr float kRescaleGap = 8.f;   // log2 units
+// Three warpgroups; warp 11 has no role. Registers can only be moved between whole warpgroups: the
+// softmax threads, which hold 128 scores each, take 208, the last group keeps 88.
+constexpr int kPairThreads = 384;
+constexpr int kSoftmaxRegs = 208, kRoleRegs = 3 * 168 - 2 * kSoftmaxRegs;
+static_assert(2 * kSoftmaxRegs + kRoleRegs <= 3 * 168, "an increase beyond what the block started with waits for ever");
+constexpr int kMmaWarp = 8, kProducerWarp = 10;   // kMmaWarp + t: tile t
+
+template <int DP>
+struct PairPlan {
+    static constexpr int kSub = DP / 64;              // 64-column sub-tiles of an operand
+    static constexpr int kTile = 128 * 128;           // one [128][64] bf16 sub-tile, 128-byte swizzled rows
+    static constexpr int kOperand = kSub * kTile;
+    static constexpr int kSlots = DP == 64 ? 12 : 5;  // ring of K and V tiles (K, V, K, V, ...)
+    static constexpr int kQ = 0;                      // Q_A, Q_B
+    static constexpr int kRing = 2 * kOperand;
+    static constexpr int kMaskRow = kRing + kSlots * kOperand;   // float [tile][parity][128]: a block's mask terms
+    static constexpr int kBars = kMaskRow + 2 * 2 * 128 * 4;
+    static constexpr int kBarBytes = 512;
+    static constexpr int kBytes = kBars + kBarBytes;
+    static_assert(kBytes <= 232448, "shared memory per CTA");
+    // dual: float2 [128] of B's (m, l); Q_B is idle then
+    static constexpr int kPartial = kQ + kOperand;
+    // tensor memory columns
+    static constexpr bool kPOverS = DP == 128;        // P overwrites the scores it came from
+    static constexpr int kP = kPOverS ? 0 : 256;      // S_A 0, S_B 128
+    static constexpr int kPStep = kPOverS ? 128 : 64; // from P_A to P_B
+    static constexpr int kO = kPOverS ? 256 : 384;    // + DP per tile
+    static_assert(kO + 2 * DP <= 512, "tensor memory columns");
+    // Exponentials per 8 pairs that take the FMA-pipe polynomial instead of MUFU.
+    static constexpr int kPolyPairs = 2;   // measured: 0, 1, 2, 3 of 8 take 161, 153, 151, 153 us on 2 x 10 heads x 4096
+    // barriers (8 bytes each); "+ t": tile
+    static constexpr int bQFull = 0;                   // + t
+    static constexpr int bQFree = 2;                   // + t
+    static constexpr int bSFull = 4;                   // + t
+    static constexpr int bSFree = 6;                   // + t: the scores are in registers
+    static constexpr int bPFull = 8;                   // + 2 t + half of the keys (64 each; one phase for all where P has columns of its own)
+    static constexpr int bPVDone = 12;                 // + t
+    static constexpr int bOFree = 14;                  // + t
+    static constexpr int bWorkFull = 16;               // + slot
+    static constexpr int bWorkFree = 18;               // + slot
+    static constexpr int bMask = 20;                   // + t: the block's mask terms are written
+    static constexpr int bPartial = 22;                // dual: B's half is final
+    static constexpr int bKVFull = 23;                 // + ring slot
+    static constexpr int bKVEmpty = bKVFull + kSlots;  // + ring slot
+    static constexpr int bCount = bKVEmpty + kSlots;
+    static_assert(bCount * 8 + 32 <= kBarBytes, "barrier area");
+};
+
+// What mask_plan_kernel leaves behind, per plane (a (batch, head) of the mask's own sizes),
+// 32-row group and 128-key block. `active`: bit per block, set unless the block is hidden from
+// the group. `kind`: see PieceKind. `bits`: uint4 per row (bit = visible). `values`: 128 terms
+// per row as they were given (16-bit: bf16; else fp32), [16-byte chunk][row].
+struct MaskPlan {
+    uint32_t* active;
+    uint8_t* kind;
+    uint4* bits;
+    uint4* values;
+    int groups, blocks, words;   // 32-row groups, key blocks, active words per group
+    int heads;                   // planes per batch entry
+    int batched;                 // 0: every batch entry shares the planes
+    int wide;                    // values are fp32
+};
+enum PieceKind : uint8_t { kHidden = 0, kNoEffect = 1, kYesNo = 2, kValues = 3, kAllFloor = 4 };
+constexpr int kMaxPlanBlocks = 1024;
+
+struct PairParams {
+    AttnParams a;
+    int* status;
+    int dim_of[3][3];     // per operand (q, k, v): tensor-map slot (1..3) of the row, head and batch dims
+    int work;             // items = levels * batch * kv_heads
+    int dual;
+    int* work_counter;    // null: a fixed deal
+    int* done_counter;    // with it: the last producer to finish puts both back to zero
+    int grouped;          // item order (decode_item)
+    Divisor by_batch, by_kv_heads, by_group, by_levels;
+    MaskPlan plan;
+};
+
+struct Item {
+    int b, hk;
+    int h[2], q0[2], kend[2];   // per tile; kend: keys any of its rows sees
+    int n[2];                   // key blocks per tile (dual: its share); n[0] >= n[1]
+    bool valid[2];
+    SeqInfo si;
+};
+
+// Items of one (batch, K / V head) are neighbours in its list of (query tile, head), longest
+// causal tiles first, heads fastest. Two orders of the items: with the level slowest every deal
+// in rounds hands out similar lengths; `grouped` (needs the counter) keeps all items of one
+// (batch, K / V head) together, so that the items in flight share the K / V of a few heads in L2
+// (measured on a packed 65,536-token batch with 537 MB of K / V: 4.85 -> 0.81 GB of DRAM reads).
+__device__ __forceinline__ Item decode_item(const PairParams& tp, int w) {
+    const AttnParams& p = tp.a;
+    Item k;
+    int level;
+    if (tp.grouped) {
+        const int plane = div_by(w, tp.by_levels);
+        level = w - plane * static_cast<int>(tp.by_levels.d);
+        k.b = div_by(plane, tp.by_kv_heads);
+        k.hk = plane - k.b * p.kv_heads;
+    } else {
+        const int t = div_by(w, tp.by_kv_heads);
+        k.hk = w - t * p.kv_heads;
+        level = div_by(t, tp.by_batch);
+        k.b = t - level * p.batch;
+    }
+    k.si = seq_info(p, k.b);
+    const int group = static_cast<int>(tp.by_group.d);
+    const int tiles = (k.si.lq + kBM - 1) >> 7;
+    const int units = tiles * group;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int u = tp.dual ? level : 2 * level + t;
+        k.valid[t] = u < units;
+        const int back = div_by(u, tp.by_group);
+        k.h[t] = k.hk * group + (u - back * group);
+        k.q0[t] = (tiles - 1 - back) * kBM;
+        int kend = k.si.klen;
+        if (p.causal) kend = min(kend, min(k.q0[t] + kBM, k.si.lq) + k.si.shift);
+        k.kend[t] = max(kend, 0);
+        k.n[t] = k.valid[t] ? (k.kend[t] + kBN - 1) >> 7 : 0;
+    }
+    if (tp.dual) {
+        k.n[1] = k.n[0] >> 1;
+        k.n[0] -= k.n[1];
+    }
+    return k;
+}
+
+// Walks the key blocks of an item. Without a plan that is 0, 1, 2, ...; with one it is the
+// blocks that are not hidden from both tiles (a dual item: from the tile).
+template <bool kPlan>
+struct BlockIter {
+    int at;
+    __device__ __forceinline__ void start(const PairParams&, const Item&, int first) { at = first; }
+    __device__ __forceinline__ int next() { return at++; }
+};
+// The active word `w` of an item (converged warp): lanes 0-7 fetch the words of the two tiles'
+// eight 32-row groups.
+__device__ __forceinline__ uint32_t active_word(const PairParams& tp, const Item& k, int w) {
+    const MaskPlan& m = tp.plan;
+    const int lane = threadIdx.x & 31, t = (lane >> 2) & 1;
+    uint32_t word = 0;
+    if (lane < 8 && k.valid[t]) {
+        const int g = (k.q0[t] >> 5) + (lane & 3);
+        const int plane = (m.batched ? k.b * m.heads : 0) + (m.heads > 1 ? k.h[t] : 0);
+        if (g < m.groups) word = m.active[(static_cast<int64_t>(plane) * m.groups + g) * m.words + w];
+    }
+    return __reduce_or_sync(0xffffffffu, word);
+}
+template <>
+struct BlockIter<true> {
+    const PairParams* tp;
+    const Item* k;
+    uint32_t word;
+    int w;
+    __device__ __forceinline__ void start(const PairParams& tp_, const Item& k_, int first) {
+        tp = &tp_;
+        k = &k_;
+        w = 0;
+        word = active_word(tp_, k_, 0);
+        for (int i = 0; i < first; ++i) next();
+    }
+    __device__ __forceinline__ int next() {
+        while (!word) {
+            ++w;
+            if (w >= tp->plan.words) return 0;   // not reached: callers take as many as there are
+            word = active_word(*tp, *k, w);
+        }
+        const int bit = __ffs(word) - 1;
+        word &= word - 1;
+        return w * 32 + bit;
+    }
+};
+// With a plan both tiles of an item walk the blocks that either of them needs.
+__device__ __forceinline__ void apply_plan(const PairParams& tp, Item& k) {
+    int n = 0;
+    for (int w = 0; w < tp.plan.words; ++w) n += __popc(active_word(tp, k, w));
+    if (tp.dual) {
+        k.n[1] = n >> 1;
+        k.n[0] = n - k.n[1];
+    } else {
+        k.n[0] = k.valid[0] ? n : 0;
+        k.n[1] = k.valid[1] ? n : 0;
+    }
+}
+
+__device__ __forceinline__ int snake(int round, int cta, int ctas) {
+    return round * ctas + ((round & 1) ? ctas - 1 - cta : cta);
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));   // one three-input instruction
+    return d;
+}
+
+// ---- the kernel ------------------------------------------------------------------------
+
+// kMask: 0 none, 1 a row per (batch, head), 2 a plan (a row per query).
+template <int DP, int kMask>
+__global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_v, const PairParams tp) {
+    using P = PairPlan<DP>;
+    using Iter = BlockIter<kMask == 2>;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const uint32_t sbase = smem_u32(smem);
+    if (sbase & 1023u) {   // swizzled tiles need a 1024-byte aligned base
+        if (threadIdx.x == 0) atomicCAS_system(tp.status, 0, 900);
+        return;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t bars = sbase + P::kBars;
+    auto bar = [&](int i) { return bars + 8u * i; };
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + P::kBars + P::bCount * 8);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + P::kBars + P::bCount * 8 + 8);
+    volatile int* work_slot = reinterpret_cast<volatile int*>(smem + P::kBars + P::bCount * 8 + 16);   // [2]
+    const AttnParams& p = tp.a;
+
+    if (warp == kProducerWarp) {
+        for (int i = lane; i < P::bCount; i += 32) {
+            uint32_t count = 1;
+            // Softmax threads arrive once per warp (mbar_arrive_warp).
+            if ((i >= P::bSFree && i < P::bSFree + 2) || (i >= P::bPFull && i < P::bPFull + 4) ||
+                (i >= P::bOFree && i < P::bOFree + 2) || (i >= P::bMask && i < P::bMask + 2) || i == P::bPartial) count = 4;
+            if (i >= P::bWorkFree && i < P::bWorkFree + 2) count = 10;   // the softmax and the MMA warps
+            // Pair: both tiles release every ring tile. Dual: each has one user, but they share Q.
+            if (i >= P::bKVEmpty && !tp.dual) count = 2;
+            if (i == P::bQFree && tp.dual) count = 2;
+            mbar_init(bar(i), count);
+        }
+        if (lane == 0) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+            *abort_flag = 0;
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+        __syncwarp();
+    } else if (warp == kMmaWarp) {
+        tmem_alloc(smem_u32(tmem_slot), 512);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // Nothing of this launch has touched global memory yet, and nothing will before the previous
+    // kernel in the stream has completed; the next one may start its own set-up.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+    const bool dual = tp.dual != 0;
+
+    // The n-th item of this CTA: -1 = no more, -2 = nothing at this position. Without a counter
+    // every role computes the same snake order by itself; with one, the producer warp draws the
+    // items and hands them to the other roles through a two-slot queue in shared memory.
+    const bool dynamic = tp.work_counter != nullptr;
+    auto static_item = [&](int n) -> int {
+        if (static_cast<int64_t>(n) * gridDim.x >= tp.work) return -1;
+        const int w = snake(n, blockIdx.x, gridDim.x);
+        return w < tp.work ? w : -2;
+    };
+    auto draw_item = [&](int n, bool& ok) -> int {   // producer warp, converged
+        if (!dynamic) return static_item(n);
+        const int slot = n & 1;
+        if (n >= 2) {
+            ok = __all_sync(0xffffffffu, mbar_wait_inline(bar(P::bWorkFree + slot), ((n >> 1) - 1) & 1, abort_flag, 120 + slot, tp.status));
+            if (!ok) return -1;
+        }
+        int w;
+        while (true) {   // positions past the end of a short sequence are skipped here
+            w = 0;
+            if (lane == 0) w = atomicAdd(tp.work_counter, 1);
+            w = __shfl_sync(0xffffffffu, w, 0);
+            if (w >= tp.work) {
+                w = -1;
+                break;
+            }
+            if (decode_item(tp, w).valid[0]) break;
+        }
+        if (lane == 0) {
+            work_slot[slot] = w;
+            __threadfence_block();
+            mbar_arrive(bar(P::bWorkFull + slot));
+        }
+        return w;
+    };
+    auto take_item = [&](int n, bool& ok) -> int {   // the other roles
+        if (!dynamic) return static_item(n);
+        const int slot = n & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait_inline(bar(P::bWorkFull + slot), (n >> 1) & 1, abort_flag, 130 + slot, tp.status));
+        if (!ok) return -1;
+        const int w = work_slot[slot];
+        mbar_arrive_warp(bar(P::bWorkFree + slot));
+        return w;
+    };
+    // Tensor-map coordinate of slot `slot` (1..3): row, head and batch sit where the host sorted
+    // them by stride.
+    auto coord = [&](int operand, int slot, int row, int head, int batch) {
+        return tp.dim_of[operand][0] == slot ? row : tp.dim_of[operand][1] == slot ? head : batch;
+    };
+
+    // The register counts are set inside the roles' branches: in code that both reach, the compiler
+    // would have to keep to the smaller one.
+    if (warp >= kMmaWarp) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRoleRegs));
+      if (warp == kProducerWarp) {
+        // ---------------- producer (whole warp, converged) ----------------
+        int items_of[2] = {0, 0};   // Q tiles loaded so far
+        int slot = 0, lap = 0;      // next ring slot, times round the ring
+        bool ok = true;
+        auto wait_for = [&](int b, int parity, int code) {
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_inline(bar(b), parity, abort_flag, code, tp.status));
+        };
+        auto load_q = [&](const Item& k, int t) {
+            if (items_of[t] > 0) wait_for(P::bQFree + t, (items_of[t] - 1) & 1, 110 + t);
+            if (!ok) return;
+            const int r = k.si.q_off + k.q0[t], b = p.cu_q ? 0 : k.b;
+            const int c1 = coord(0, 1, r, k.h[t], b), c2 = coord(0, 2, r, k.h[t], b), c3 = coord(0, 3, r, k.h[t], b);
+            mbar_expect_tx(bar(P::bQFull + t), P::kOperand);
+            for (int s = 0; s < P::kSub; ++s) {
+                tma_load_4d(sbase + P::kQ + t * P::kOperand + s * P::kTile, &map_q, bar(P::bQFull + t), s * 64, c1, c2, c3);
+            }
+            ++items_of[t];
+        };
+        auto load_kv = [&](const Item& k, const CUtensorMap* map, int operand, int block) {
+            if (lap > 0) wait_for(P::bKVEmpty + slot, (lap - 1) & 1, 100);
+            if (!ok) return;
+            const int r = k.si.k_off + block * kBN, b = p.cu_q ? 0 : k.b;
+            const int c1 = coord(operand, 1, r, k.hk, b), c2 = coord(operand, 2, r, k.hk, b), c3 = coord(operand, 3, r, k.hk, b);
+            mbar_expect_tx(bar(P::bKVFull + slot), P::kOperand);
+            for (int s = 0; s < P::kSub; ++s) {
+                tma_load_4d(sbase + P::kRing + slot * P::kOperand + s * P::kTile, map, bar(P::bKVFull + slot), s * 64, c1, c2, c3);
+            }
+            if (++slot == P::kSlots) {
+                slot = 0;
+                ++lap;
+            }
+        };
+        // In the grouped order items are fetched one ahead: the trip to the counter, and the
+        // positions a draw skips, hide behind an item's loads. Otherwise an item is drawn when
+        // its loads start: committing earlier evens the CTAs out less well at the end.
+        const bool ahead = tp.grouped != 0;
+        int w_next = ahead ? draw_item(0, ok) : 0;
+        for (int n = 0; ok; ++n) {
+            const int w = ahead ? w_next : draw_item(n, ok);
+            if (w == -1) break;
+            if (ahead) w_next = draw_item(n + 1, ok);
+            if (!ok) break;
+            if (w == -2) continue;
+            Item k = decode_item(tp, w);
+            if constexpr (kMask == 2) apply_plan(tp, k);
+            if (k.n[0] == 0) continue;
+            Iter it[2];
+            it[0].start(tp, k, 0);
+            if (dual) it[1].start(tp, k, k.n[0]);
+            load_q(k, 0);
+            const int entries = dual ? k.n[0] + k.n[1] : k.n[0];
+            for (int e = 0; ok && e < entries; ++e) {
+                const int block = (dual && (e & 1)) ? it[1].next() : it[0].next();
+                load_kv(k, &map_k, 1, block);
+                if (e == 0 && !dual && k.n[1] > 0) load_q(k, 1);
+                load_kv(k, &map_v, 2, block);
+            }
+        }
+        if (*abort_flag) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < 4000000) {   // let copies in flight land
+            }
+        } else if (dynamic && tp.done_counter && lane == 0) {
+            // This producer draws no more. The last one to say so puts the counters back to zero.
+            __threadfence();
+            const int done = atomicAdd(tp.done_counter, 1);
+            if (done == static_cast<int>(gridDim.x) - 1) {
+                *tp.work_counter = 0;
+                *tp.done_counter = 0;
+                __threadfence();
+            }
+        }
+      } else if (warp < kMmaWarp + 2) {
+        // ---------------- MMA issuer of tile t (whole warp, converged) ----------------
+        // What stands between two products is this warp's scalar work, at the pace of one warp
+        // beside two in their softmax: no divisions, no state in memory, one vote per pair of waits.
+        const int t = warp - kMmaWarp;
+        const uint64_t q_desc = smem_desc(sbase + P::kQ + (tp.dual ? 0 : t) * P::kOperand, 16, 1024);
+        const uint64_t k_desc = smem_desc(sbase + P::kRing, 16, 1024);
+        const uint64_t v_desc = smem_desc(sbase + P::kRing, P::kTile, 1024);
+        const int d_steps = (p.d + 15) >> 4;
+        const uint32_t d_s = tmem + t * 128, a_p = tmem + P::kP + t * P::kPStep, d_o = tmem + P::kO + t * DP;
+        const int q_bar = dual ? 0 : t;
+        const int stride = dual ? 4 : 2;    // ring tiles from one of this tile's blocks to its next
+        int blk = 0, items = 0;             // this tile's blocks and items so far: parities
+        int q_items = 0;                    // Q tiles so far
+        int base = 0, base_lap = 0;         // ring position of the item's first tile
+        bool ok = true;
+        // Waits for two barriers at once (their polls overlap).
+        auto wait_two = [&](uint32_t b0, uint32_t par0, uint32_t b1, uint32_t par1, int code) {
+            const bool got = mbar_try_wait(b0, par0) & mbar_try_wait(b1, par1);
+            if (!__all_sync(0xffffffffu, got)) {
+                ok = ok && __all_sync(0xffffffffu, mbar_wait_inline(b0, par0, abort_flag, code, tp.status) && mbar_wait_inline(b1, par1, abort_flag, code + 1, tp.status));
+            }
+        };
+        auto advance = [](int& slot, int& lap, int by) {
+            slot += by;
+            if (slot >= P::kSlots) {
+                slot -= P::kSlots;
+                lap ^= 1;
+            }
+        };
+        for (int n = 0; ok; ++n) {
+            const int w = take_item(n, ok);
+            if (w == -1) break;
+            if (w == -2) continue;
+            Item k = decode_item(tp, w);
+            if constexpr (kMask == 2) apply_plan(tp, k);
+            if (k.n[0] == 0) continue;
+            const int nb = t ? k.n[1] : k.n[0], kend = t ? k.kend[1] : k.kend[0], klen = k.si.klen;
+            const int entries = dual ? k.n[0] + k.n[1] : k.n[0];
+            Iter it;
+            it.start(tp, k, dual && t ? k.n[0] : 0);
+            int s_slot = base, s_lap = base_lap;    // K of the next score product; V is one further
+            if (dual && t) advance(s_slot, s_lap, 2);
+            int v_slot = s_slot, v_lap = s_lap;
+            advance(v_slot, v_lap, 1);
+            int block = 0, s_block = 0;             // of the P V and of the score product at hand
+            // Scores of block j + 1 go out ahead of P V of block j where P has columns of its own
+            // (they only need the scores' columns free), behind it where P overwrites them.
+#pragma unroll 1
+            for (int j = -1; ok && j < nb; ++j) {
+                const bool more = j + 1 < nb;
+                if (more) s_block = it.next();
+                auto scores = [&]() {
+                    const int gb = blk + j + 1;     // this tile's score products so far
+                    if (j < 0) {
+                        wait_two(bar(P::bQFull + q_bar), q_items & 1, bar(P::bKVFull + s_slot), s_lap, 200 + 2 * t);
+                        if (!P::kPOverS && gb > 0) wait_two(bar(P::bSFree + t), (gb - 1) & 1, bar(P::bSFree + t), (gb - 1) & 1, 210);
+                    } else if (P::kPOverS) {
+                        wait_two(bar(P::bKVFull + s_slot), s_lap, bar(P::bKVFull + s_slot), s_lap, 220 + t);
+                    } else {
+                        wait_two(bar(P::bKVFull + s_slot), s_lap, bar(P::bSFree + t), (gb - 1) & 1, 222 + 2 * t);
+                    }
+                    if (!ok) return;
+                    tc_fence_after();
+                    const int keys = min(kBN, (kend - s_block * kBN + 15) & ~15);   // in the MMA's steps of 16
+                    const uint64_t kd = k_desc + static_cast<uint32_t>(s_slot * (P::kOperand >> 4));
+                    if (d_steps == DP / 16 && keys == kBN) {
+#pragma unroll
+                        for (int ks = 0; ks < DP / 16; ++ks) {
+                            const uint32_t off = ((ks / 4) * P::kTile + (ks % 4) * 32) >> 4;
+                            tc_mma(d_s, q_desc + off, kd + off, instr_desc(kBN, false), ks > 0);
+                        }
+                    } else {
+                        const uint32_t idesc = instr_desc(keys, false);
+#pragma unroll 1
+                        for (int ks = 0; ks < d_steps; ++ks) {
+                            const uint32_t off = ((ks / 4) * P::kTile + (ks % 4) * 32) >> 4;
+                            tc_mma(d_s, q_desc + off, kd + off, idesc, ks > 0);
+                        }
+                    }
+                    tc_commit(bar(P::bSFull + t));
+                    tc_commit(bar(P::bKVEmpty + s_slot));
+                    if (j + 2 == nb) tc_commit(bar(P::bQFree + q_bar));
+                    advance(s_slot, s_lap, stride);
+                };
+                auto values = [&]() {
+                    const int gb = blk + j, keys = min(kBN, (kend - block * kBN + 15) & ~15), seen = klen - block * kBN;
+                    wait_two(bar(P::bKVFull + v_slot), v_lap, bar(P::bPFull + 2 * t), gb & 1, 230 + 2 * t);
+                    if (j == 0 && items > 0) wait_two(bar(P::bOFree + t), (items - 1) & 1, bar(P::bOFree + t), (items - 1) & 1, 250 + t);
+                    if (!ok) return;
+                    if (seen < keys) {
+                        // Rows past the sequence's keys may hold anything (a cache past its length, a
+                        // packed neighbour), and P = 0 times an infinity would still poison the
+                        // output. (Pair: both tiles' warps write the same zeros.)
+                        unsigned char* vt = smem + P::kRing + v_slot * P::kOperand;
+                        const int rows = keys - seen;
+#pragma unroll 1
+                        for (int i = lane; i < P::kSub * rows * 8; i += 32) {
+                            const int sub = i >= rows * 8 ? 1 : 0, rem = i - sub * (rows * 8);
+                            *reinterpret_cast<uint4*>(vt + sub * P::kTile + (seen + (rem >> 3)) * 128 + (rem & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                        }
+                        fence_async_smem();
+                        __syncwarp();
+                    }
+                    tc_fence_after();
+                    const uint64_t vd = v_desc + static_cast<uint32_t>(v_slot * (P::kOperand >> 4));
+                    // A: P, 8 TMEM columns per 16 keys. B: V MN-major, 16 keys = 16 rows of 128 bytes;
+                    // the second 64 columns of Dv are one sub-tile further (LBO).
+                    const bool whole = keys == kBN && p.dv == DP;
+                    if (whole) {
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks) {
+                            tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), instr_desc(DP, true), (j > 0 || ks > 0) ? 1u : 0u);
+                        }
+                    }
+                    if constexpr (P::kPOverS) {
+                        wait_two(bar(P::bPFull + 2 * t + 1), gb & 1, bar(P::bPFull + 2 * t + 1), gb & 1, 240 + t);
+                        if (!ok) return;
+                        tc_fence_after();
+                    }
+                    if (whole) {
+#pragma unroll
+                        for (int ks = 4; ks < 8; ++ks) {
+                            tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), instr_desc(DP, true), 1u);
+                        }
+                    } else {
+                        const uint32_t idesc = instr_desc((p.dv + 15) & ~15, true);
+#pragma unroll 1
+                        for (int ks = 0; ks < keys >> 4; ++ks) {
+                            tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), idesc, (j > 0 || ks > 0) ? 1u : 0u);
+                        }
+                    }
+                    tc_commit(bar(P::bPVDone + t));
+                    tc_commit(bar(P::bKVEmpty + v_slot));
+                    advance(v_slot, v_lap, stride);
+                };
+                if constexpr (P::kPOverS) {
+                    if (j >= 0) values();
+                    if (more) scores();
+                } else {
+                    if (more) scores();
+                    if (j >= 0) values();
+                }
+                block = s_block;
+            }
+            if (!dual && t && nb < entries) {
+                // Blocks that only tile A sees: this warp's release of their ring tiles. (Not before
+                // they have been loaded: the arrival must not fall into the slot's previous use.)
+                for (int e = 0; ok && e < 2 * (entries - nb); ++e) {
+                    wait_two(bar(P::bKVFull + s_slot), s_lap, bar(P::bKVFull + s_slot), s_lap, 260);
+                    if (lane == 0) mbar_arrive(bar(P::bKVEmpty + s_slot));
+                    __syncwarp();
+                    advance(s_slot, s_lap, 1);
+                }
+            }
+            if (dual && nb == 0) {   // Q is released by both
+                wait_two(bar(P::bQFull), q_items & 1, bar(P::bQFull), q_items & 1, 204);
+                if (lane == 0) mbar_arrive(bar(P::bQFree));
+                __syncwarp();
+            }
+            if (nb > 0) ++items;
+            if (nb > 0 || dual) ++q_items;
+            blk += nb;
+            // 2 * entries can be several times round the ring.
+            for (int left = 2 * entries; left > 0; left -= P::kSlots) advance(base, base_lap, min(left, P::kSlots));
+        }
+      }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+        // ---------------- softmax: thread = query row of tile t ----------------
+        const int t = warp >> 2;
+        const int row = (warp & 3) * 32 + lane;         // row inside the tile = TMEM lane
+        const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+        const uint32_t s_addr = tmem + lane_addr + (t ? 128 : 0);
+        const uint32_t p_addr = tmem + lane_addr + P::kP + t * P::kPStep;
+        const uint32_t o_addr = tmem + lane_addr + P::kO + t * DP;
+        int blk = 0;        // key blocks of this tile so far: parity of its barriers
+        int shared = 0;     // dual: items in which B had a part
+        bool ok = true;
+        auto wait_for = [&](int b, int parity, int code) {
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_inline(bar(b), parity, abort_flag, code, tp.status));
+        };
+        const float sc = p.scale_log2;
+
+        for (int n = 0; ok; ++n) {
+            const int w = take_item(n, ok);
+            if (w == -1) break;
+            if (w == -2) continue;
+            Item k = decode_item(tp, w);
+            if (!(t ? k.valid[1] : k.valid[0])) continue;
+            if constexpr (kMask == 2) apply_plan(tp, k);
+            // (Selected once: an index that is not a constant would put the item into memory.)
+            const int nb = t ? k.n[1] : k.n[0], h = t ? k.h[1] : k.h[0], q0 = t ? k.q0[1] : k.q0[0], kend = t ? k.kend[1] : k.kend[0];
+            const int qi = q0 + row;                    // row inside the sequence
+            const bool real = qi < k.si.lq;
+            if (nb == 0) {
+                // No key is visible to this tile: zeros, lse = -inf, and no barrier is involved.
+                // (Dual: tile A answers for both; B has no part of a tile with one key block.)
+                if (real && !(dual && t == 1)) {
+                    __nv_bfloat16* og = p.out + k.b * p.os[0] + h * p.os[1] + static_cast<int64_t>(k.si.q_off + qi) * p.os[2];
+                    for (int c = 0; c < p.dv; c += 8) *reinterpret_cast<uint4*>(og + c) = make_uint4(0u, 0u, 0u, 0u);
+                    if (p.lse) p.lse[k.b * p.ls[0] + h * p.ls[1] + (k.si.q_off + qi) * p.ls[2]] = -INFINITY;
+                }
+                continue;
+            }
+            // Keys this row may see: [0, row_limit). The smallest limit of the warp is its first
+            // row's, the largest its last row's.
+            auto limit_of = [&](int i) { return p.causal ? min(kend, i + k.si.shift + 1) : kend; };
+            const int row_limit = limit_of(qi), limit_lo = limit_of(q0 + (warp & 3) * 32), limit_hi = limit_of(q0 + (warp & 3) * 32 + 31);
+            float m_ref = -INFINITY;   // reference maximum (base-2 logits), moved lazily
+            float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            Iter it;
+            it.start(tp, k, (dual && t == 1) ? k.n[0] : 0);
+            const uint8_t* kinds = nullptr;
+            int64_t piece0 = 0;        // plan: index of this warp's first piece
+            if constexpr (kMask == 2) {
+                const MaskPlan& m = tp.plan;
+                const int g = min((q0 >> 5) + (warp & 3), m.groups - 1);
+                const int plane = (m.batched ? k.b * m.heads : 0) + (m.heads > 1 ? h : 0);
+                piece0 = (static_cast<int64_t>(plane) * m.groups + g) * m.blocks;
+                kinds = m.kind + piece0;
+            }
+
+            for (int j = 0; ok && j < nb; ++j) {
+                const int gb = blk + j;
+                const int block = it.next();
+                const int limit = row_limit - block * kBN;        // my columns [0, limit) are visible
+                const int lo = limit_lo - block * kBN;
+                int chunks = min(max(limit_hi - block * kBN + 31, 0) >> 5, 4);   // 32-column chunks with a visible key
+                const int stored = min((kend - block * kBN + 31) >> 5, 4);  // chunks that P V reads
+                int kind = kNoEffect;
+                const float* mrow = nullptr;
+                if constexpr (kMask == 1) {
+                    // One thread per column fetches the block's mask term, the tile's threads share
+                    // the row through shared memory. (A bounded mbarrier, not bar.sync: a warp that
+                    // gave up elsewhere must not strand the others. Two rows alternate: a row is
+                    // written again only after everybody has arrived for the block between.)
+                    float* rows = reinterpret_cast<float*>(smem + P::kMaskRow) + (t * 2 + (gb & 1)) * 128;
+                    const int key = max(min(block * kBN + row, k.si.klen - 1), 0);
+                    rows[row] = mask_value(p, k.b, h, 0, static_cast<int64_t>(k.si.k_off) + key) * kLog2e;
+                    mbar_arrive_warp(bar(P::bMask + t));
+                    wait_for(P::bMask + t, gb & 1, 340 + t);
+                    if (!ok) break;
+                    mrow = rows;
+                }
+                uint4 bits = make_uint4(0u, 0u, 0u, 0u);
+                if constexpr (kMask == 2) {
+                    kind = kinds[block];
+                    if (kind == kHidden) chunks = 0;
+                    if (kind == kYesNo) bits = tp.plan.bits[(piece0 + block) * 32 + lane];
+                }
+                wait_for(P::bSFull + t, gb & 1, 300 + t);
+                if (!ok) break;
+                tc_fence_after();
+
+                // A block every key of which every row of this warp sees, without a mask term: the
+                // scores go into registers once, in straight-line code. Any other block (the diagonal,
+                // the last keys, masks) takes a loop over 32-column chunks that reads them twice.
+                const bool fast = kMask != 1 && lo >= kBN && (kMask == 0 || kind == kNoEffect);
+                float s[128];
+                float mx[2] = {-INFINITY, -INFINITY};
+                auto chunk_max = [&](const float* x) {
+#pragma unroll
+                    for (int e = 0; e < 32; e += 4) {
+                        mx[0] = max3(mx[0], x[e], x[e + 1]);
+                        mx[1] = max3(mx[1], x[e + 2], x[e + 3]);
+                    }
+                };
+                // Chunk c of the scores as base-2 logits with their mask terms, hidden columns -inf.
+                auto logits = [&](float (&x)[32], int c) {
+                    tmem_ld32(s_addr + c * 32, x);
+                    tmem_wait_ld();
+                    if constexpr (kMask == 1) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const float4 m4 = reinterpret_cast<const float4*>(mrow + c * 32)[e];
+                            x[e * 4] = fmaf(x[e * 4], sc, m4.x);
+                            x[e * 4 + 1] = fmaf(x[e * 4 + 1], sc, m4.y);
+                            x[e * 4 + 2] = fmaf(x[e * 4 + 2], sc, m4.z);
+                            x[e * 4 + 3] = fmaf(x[e * 4 + 3], sc, m4.w);
+                        }
+                    } else if (kMask == 2 && kind == kValues && !tp.plan.wide) {
+                        const uint4* v = tp.plan.values + ((piece0 + block) * 16 + c * 4) * 32 + lane;
+                        uint4 q[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) q[e] = v[e * 32];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const uint32_t u[4] = {q[e].x, q[e].y, q[e].z, q[e].w};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const float m0 = fmaxf(__uint_as_float(u[i] << 16), kMaskedLogit), m1 = fmaxf(__uint_as_float(u[i] & 0xffff0000u), kMaskedLogit);
+                                x[e * 8 + i * 2] = fmaf(x[e * 8 + i * 2], sc, m0 * kLog2e);
+                                x[e * 8 + i * 2 + 1] = fmaf(x[e * 8 + i * 2 + 1], sc, m1 * kLog2e);
+                            }
+                        }
+                    } else if (kMask == 2 && kind == kValues) {
+                        const float4* v = reinterpret_cast<const float4*>(tp.plan.values) + ((piece0 + block) * 32 + c * 8) * 32 + lane;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const float4 m4 = v[e * 32];
+                            x[e * 4] = fmaf(x[e * 4], sc, fmaxf(m4.x, kMaskedLogit) * kLog2e);
+                            x[e * 4 + 1] = fmaf(x[e * 4 + 1], sc, fmaxf(m4.y, kMaskedLogit) * kLog2e);
+                            x[e * 4 + 2] = fmaf(x[e * 4 + 2], sc, fmaxf(m4.z, kMaskedLogit) * kLog2e);
+                            x[e * 4 + 3] = fmaf(x[e * 4 + 3], sc, fmaxf(m4.w, kMaskedLogit) * kLog2e);
+                        }
+                    } else if (kMask == 2 && kind != kNoEffect) {
+                        const uint32_t word = c == 0 ? bits.x : c == 1 ? bits.y : c == 2 ? bits.z : bits.w;
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) x[e] = fmaf(x[e], sc, (word >> e) & 1u ? 0.f : kMaskedLogit * kLog2e);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) x[e] *= sc;
+                    }
+                    if (lo < (c + 1) * 32) {
+                        const int left = limit - c * 32;
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) x[e] = e < left ? x[e] : -INFINITY;
+                    }
+                };
+                float top;
+                if (fast) {
+                    tmem_ld32(s_addr, s);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        tmem_wait_ld();
+                        if (c < 3) {
+                            tmem_ld32(s_addr + (c + 1) * 32, s + (c < 3 ? c + 1 : 3) * 32);
+                        } else if (!P::kPOverS) {
+                            // The scores are in registers: the next Q K^T may have their columns.
+                            tc_fence_before();
+                            mbar_arrive_warp(bar(P::bSFree + t));
+                        }
+                        chunk_max(s + c * 32);
+                    }
+                    top = fmaxf(mx[0], mx[1]) * sc;
+                } else {
+#pragma unroll 1
+                    for (int c = 0; c < chunks; ++c) {
+                        float x[32];
+                        logits(x, c);
+                        chunk_max(x);
+                    }
+                    top = fmaxf(mx[0], mx[1]);
+                }
+
+                // Lazy rescale: move the reference only when this block exceeds it by 2^8.
+                const bool move = top > m_ref + kRescaleGap;
+                if (__any_sync(0xffffffffu, move)) {
+                    float f = 1.f;
+                    if (move) {
+                        f = fast_exp2(m_ref - top);   // 0 on the first block
+                        m_ref = top;
+                        l2[0] = __fmul2_rn(l2[0], make_float2(f, f));
+                        l2[1] = __fmul2_rn(l2[1], make_float2(f, f));
+                    }
+                    if (j > 0) {
+                        // O holds blocks [0, j): wait for block j - 1's P V.
+                        wait_for(P::bPVDone + t, (gb - 1) & 1, 310 + t);
+                        if (!ok) break;
+                        tc_fence_after();
+#pragma unroll 1
+                        for (int c = 0; c < DP / 16; ++c) {   // small chunks: this rare path claims no registers
+                            float o[16];
+                            tmem_ld16(o_addr + c * 16, o);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) o[e] *= f;
+                            tmem_st16(o_addr + c * 16, reinterpret_cast<const uint32_t*>(o));
+                        }
+                        tmem_wait_st();
+                    }
+                }
+                const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+
+                // ---- P = 2^(logit - m) as packed bf16 pairs ----
+                const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(-m_use, -m_use);
+                // P's columns are free once the previous block's P V has read them.
+                auto wait_p_free = [&]() {
+                    if (j > 0) {
+                        wait_for(P::bPVDone + t, (gb - 1) & 1, 320 + t);
+                        tc_fence_after();
+                    }
+                };
+                if (fast) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t wv[16];
+                        const float* x = s + c * 32;
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            const float2 y = __ffma2_rn(make_float2(x[2 * e], x[2 * e + 1]), sc2, nm2);
+                            float2 pr;
+                            // The polynomial pairs are spread evenly: MUFU and FMA work alternate.
+                            if ((e * P::kPolyPairs) % 8 < P::kPolyPairs) {
+                                pr = exp2_poly2(y);
+                            } else {
+                                pr.x = fast_exp2(y.x);
+                                pr.y = fast_exp2(y.y);
+                            }
+                            l2[e & 1] = __fadd2_rn(l2[e & 1], pr);
+                            wv[e] = pack_bf16(pr.x, pr.y);
+                        }
+                        if (!P::kPOverS && c == 0) wait_p_free();
+                        tmem_st16(p_addr + c * 16, wv);
+                        if (P::kPOverS && c == 1) {
+                            // P V may start on the first half of the keys.
+                            tmem_wait_st();
+                            tc_fence_before();
+                            mbar_arrive_warp(bar(P::bPFull + 2 * t));
+                        }
+                    }
+                } else {
+                    if (!P::kPOverS) wait_p_free();
+#pragma unroll 1
+                    for (int c = 0; c < stored; ++c) {
+                        uint32_t wv[16];
+                        if (c < chunks) {
+                            // Hidden columns take MUFU, whose 2^-inf is exactly 0.
+                            float x[32];
+                            logits(x, c);
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) {
+                                const float2 y = __fadd2_rn(make_float2(x[2 * e], x[2 * e + 1]), nm2);
+                                const float2 pr = make_float2(fast_exp2(y.x), fast_exp2(y.y));
+                                l2[e & 1] = __fadd2_rn(l2[e & 1], pr);
+                                wv[e] = pack_bf16(pr.x, pr.y);
+                            }
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) wv[e] = 0u;
+                        }
+                        tmem_st16(p_addr + c * 16, wv);
+                    }
+                    tmem_wait_st();
+                    tc_fence_before();
+                    mbar_arrive_warp(bar(P::kPOverS ? P::bPFull + 2 * t : P::bSFree + t));
+                }
+                if (!ok) break;
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive_warp(bar(P::bPFull + 2 * t + (P::kPOverS ? 1 : 0)));
+            }
+            if (!ok) break;
+
+            // ---- the item's end: O / l to memory ----
+            const int last = blk + nb - 1;
+            blk += nb;
+            wait_for(P::bPVDone + t, last & 1, 330 + t);
+            if (!ok) break;
+            tc_fence_after();
+            float l_row = (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y), m_row = m_ref;
+            float f_mine = 1.f, f_other = 0.f;
+            const bool merge = dual && k.n[1] > 0;
+            if (merge) {
+                float2* part = reinterpret_cast<float2*>(smem + P::kPartial);
+                if (t == 1) {
+                    // Tile A's threads take this half out of tensor memory and free it.
+                    part[row] = make_float2(m_row, l_row);
+                    tc_fence_before();
+                    mbar_arrive_warp(bar(P::bPartial));
+                    continue;
+                }
+                wait_for(P::bPartial, shared & 1, 380);
+                ++shared;
+                if (!ok) break;
+                tc_fence_after();
+                const float2 other = part[row];
+                const float m_all = fmaxf(m_row, other.x);
+                const float base_m = (m_all == -INFINITY) ? 0.f : m_all;
+                f_mine = fast_exp2(m_row - base_m);
+                f_other = fast_exp2(other.x - base_m);
+                l_row = fmaf(other.y, f_other, l_row * f_mine);
+                m_row = m_all;
+            }
+            const float inv = l_row > 0.f ? 1.f / l_row : 0.f;
+            __nv_bfloat16* og = p.out + k.b * p.os[0] + h * p.os[1] + static_cast<int64_t>(k.si.q_off + qi) * p.os[2];
+#pragma unroll
+            for (int c = 0; c < DP / 32; ++c) {
+                if (c * 32 < p.dv) {
+                    float o[32];
+                    tmem_ld32(o_addr + c * 32, o);
+                    if (merge) {
+                        float o1[32];
+                        tmem_ld32(tmem + lane_addr + P::kO + DP + c * 32, o1);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) o[e] = fmaf(o1[e], f_other, o[e] * f_mine);
+                    } else {
+                        tmem_wait_ld();
+                    }
+                    if (c * 32 + 32 >= p.dv) {
+                        // O is in registers: the next item's P V may overwrite it.
+                        tc_fence_before();
+                        mbar_arrive_warp(bar(P::bOFree + t));
+                        if (merge) mbar_arrive_warp(bar(P::bOFree + 1));
+                    }
+                    if (real) {
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            uint32_t q[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) q[i] = pack_bf16(o[e * 16 + 2 * i] * inv, o[e * 16 + 2 * i + 1] * inv);
+                            const int left = p.dv - c * 32 - e * 16;   // columns still to write (Dv is a multiple of 8)
+                            if (left >= 16) {
+                                store_32_bytes(og + c * 32 + e * 16, q);
+                            } else if (left >= 8) {
+                                *reinterpret_cast<uint4*>(og + c * 32 + e * 16) = make_uint4(q[0], q[1], q[2], q[3]);
+                            }
+                        }
+                    }
+                }
+            }
+            if (real && p.lse) {
+                p.lse[k.b * p.ls[0] + h * p.ls[1] + (k.si.q_off + qi) * p.ls[2]] =
+                    l_row > 0.f ? kLn2 * (m_row + log2f(l_row)) : -INFINITY;
+            }
+        }
+    }
+
+    // Teardown: everyone arrives (all waits above are bounded), then the allocating warp frees
+    // tensor memory.
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        if (*abort_flag) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < 2000000) {
+            }
+        }
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+// ---- masks with a row per query ----------------------------------------------------------
+//
+// One CTA per 32 query rows of a plane walks the keys once: eight warps of four rows each, four
+// blocks of 128 keys at a time (sixteen loads in flight per lane: with one block at a time the
+// walk was a chain of trips to memory). It is bound by reading the mask once; pieces without
+// values to apply cost nothing further, and what the attention kernel reads back is the bits or
+// values of the pieces that have any.
+//
+// A block is hidden from a group when every term of it is at the floor (-5e5): its weights are
+// exactly 0 as long as each row of the group keeps a key well above the floor. A group with a
+// row that does not (a row that sees nothing) has none of its blocks left out.
+constexpr float kSafeTerm = 0.5f * kMaskedLogit;
+constexpr int kPlanUnroll = 4;
+
+__device__ __forceinline__ float mask_raw(const AttnParams& p, int64_t idx) {
+    switch (p.mask_dtype) {
+        case KTT_B200_MASK_BOOL: return reinterpret_cast<const uint8_t*>(p.mask)[idx] ? 0.f : kMaskedLogit;
+        case KTT_B200_MASK_BF16: return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.mask)[idx]);
+        case KTT_B200_MASK_F16: return __half2float(reinterpret_cast<const __half*>(p.mask)[idx]);
+        default: return reinterpret_cast<const float*>(p.mask)[idx];
+    }
+}
+
+// kVec: the keys are contiguous and every row of the mask starts on an 8-byte (16-bit types),
+// 4-byte (bool) or 16-byte (fp32) boundary, so that a lane reads its four keys in one load.
+template <bool kVec>
+__global__ void __launch_bounds__(256) mask_plan_kernel(const AttnParams p, const MaskPlan m, int32_t* header) {
+    __shared__ uint32_t seen[kMaxPlanBlocks];   // per block: 1 floor, 2 zero, 4 anything else
+    __shared__ int unsafe;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int g = blockIdx.x, plane = blockIdx.y;
+    const int pb = plane / m.heads, ph = plane - pb * m.heads;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < m.blocks; i += 256) seen[i] = 0;
+    if (threadIdx.x == 0) unsafe = 0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The attention kernel's work counters: this launch comes first in the stream.
+    if (g == 0 && plane == 0 && threadIdx.x < 2) header[threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t piece0 = (static_cast<int64_t>(plane) * m.groups + g) * m.blocks;
+    float best[4];   // per row: the largest term so far
+#pragma unroll
+    for (int r = 0; r < 4; ++r) best[r] = -INFINITY;
+    for (int b0 = 0; b0 < m.blocks; b0 += kPlanUnroll) {
+        float v[kPlanUnroll][4][4];
+        uint32_t flags[kPlanUnroll];
+#pragma unroll
+        for (int u = 0; u < kPlanUnroll; ++u) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int row = g * 32 + warp * 4 + r, col = (b0 + u) * 128 + lane * 4;
+                const int64_t at = pb * p.ms[0] + ph * p.ms[1] + static_cast<int64_t>(min(row, p.sq - 1)) * p.ms[2];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[u][r][e] = kMaskedLogit;
+                if (kVec && col + 3 < p.sk) {
+                    const int64_t idx = at + col;
+                    if (p.mask_dtype == KTT_B200_MASK_F32) {
+                        const float4 x = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(p.mask) + idx));
+                        v[u][r][0] = x.x; v[u][r][1] = x.y; v[u][r][2] = x.z; v[u][r][3] = x.w;
+                    } else if (p.mask_dtype == KTT_B200_MASK_BOOL) {
+                        const uint32_t x = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(p.mask) + idx));
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v[u][r][e] = (x >> (8 * e)) & 0xffu ? 0.f : kMaskedLogit;
+                    } else {
+                        const uint2 x = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.mask) + idx));
+                        if (p.mask_dtype == KTT_B200_MASK_BF16) {
+                            v[u][r][0] = __uint_as_float(x.x << 16); v[u][r][1] = __uint_as_float(x.x & 0xffff0000u);
+                            v[u][r][2] = __uint_as_float(x.y << 16); v[u][r][3] = __uint_as_float(x.y & 0xffff0000u);
+                        } else {
+                            const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&x.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&x.y));
+                            v[u][r][0] = lo.x; v[u][r][1] = lo.y; v[u][r][2] = hi.x; v[u][r][3] = hi.y;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (col + e < p.sk) v[u][r][e] = mask_raw(p, at + (col + e) * p.ms[3]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kPlanUnroll; ++u) {
+            flags[u] = 0;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (g * 32 + warp * 4 + r < p.sq) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        // Columns past the last key count as hidden; they decide nothing.
+                        const bool floor_ = !(v[u][r][e] > kMaskedLogit);
+                        const bool inside = (b0 + u) * 128 + lane * 4 + e < p.sk;
+                        if (inside) flags[u] |= floor_ ? 1u : v[u][r][e] == 0.f ? 2u : 4u;
+                        if (inside && !floor_) best[r] = fmaxf(best[r], v[u][r][e]);
+                    }
+                }
+            }
+            flags[u] = __reduce_or_sync(0xffffffffu, flags[u]);
+            if (lane == 0 && b0 + u < m.blocks && flags[u]) atomicOr(&seen[b0 + u], flags[u]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kPlanUnroll; ++u) {
+            if (b0 + u >= m.blocks) break;
+            const uint32_t f = seen[b0 + u];
+            const int64_t piece = piece0 + b0 + u;
+            if (f & 4u) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int rr = warp * 4 + r;
+                    if (m.wide) {
+                        reinterpret_cast<float4*>(m.values)[(piece * 32 + lane) * 32 + rr] = make_float4(v[u][r][0], v[u][r][1], v[u][r][2], v[u][r][3]);
+                    } else {
+                        // bf16 in, bf16 out: the upper halves, two lanes to a 16-byte chunk
+                        uint2 w;
+                        w.x = __byte_perm(__float_as_uint(v[u][r][0]), __float_as_uint(v[u][r][1]), 0x7632);
+                        w.y = __byte_perm(__float_as_uint(v[u][r][2]), __float_as_uint(v[u][r][3]), 0x7632);
+                        reinterpret_cast<uint2*>(m.values + (piece * 16 + (lane >> 1)) * 32 + rr)[lane & 1] = w;
+                    }
+                }
+            } else if (f == 3u) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    // Four bits per lane; eight lanes make a word, four words a row.
+                    uint32_t x = 0;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) x |= (v[u][r][e] > kMaskedLogit ? 1u : 0u) << (4 * (lane & 7) + e);
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) x |= __shfl_xor_sync(0xffffffffu, x, o);
+                    if ((lane & 7) == 0) reinterpret_cast<uint32_t*>(m.bits + piece * 32 + warp * 4 + r)[lane >> 3] = x;
+                }
+            }
+        }
+    }
+    bool bad = false;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        float x = best[r];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+        bad = bad || (g * 32 + warp * 4 + r < p.sq && !(x > kSafeTerm));
+    }
+    if (bad && lane == 0) unsafe = 1;
+    __syncthreads();
+    for (int i = threadIdx.x; i < m.blocks; i += 256) {
+        const uint32_t f = seen[i];
+        m.kind[piece0 + i] = (f & 4u) ? kValues : f == 3u ? kYesNo : f == 2u ? kNoEffect : unsafe ? kAllFloor : kHidden;
+    }
+    for (int w = threadIdx.x; w < m.words; w += 256) {
+        uint32_t bits = 0;
+        for (int i = 0; i < 32 && w * 32 + i < m.blocks; ++i) bits |= (unsafe || seen[w * 32 + i] != 1u ? 1u : 0u) << i;
+        m.active[(static_cast<int64_t>(plane) * m.groups + g) * m.words + w] = bits;
+    }
+}
+
+// ---- host side ---------------------------------------------------------------------------
+
+bool mask_needs_plan(const AttnParams& p) { return p.mask_dtype != KTT_B200_MASK_NONE && p.ms[2] != 0 && p.sq > 1; }
+
+int64_t up256(int64_t x) { return (x + 255) / 256 * 256; }
+
+// Sizes of a plan and its place in `base` (null: sizes only); returns its bytes.
+int64_t plan_layout(const AttnParams& p, unsigned char* base, MaskPlan* m) {
+    m->groups = (p.sq + 31) / 32;
+    m->blocks = (p.sk + kBN - 1) / kBN;
+    m->words = (m->blocks + 31) / 32;
+    m->heads = p.ms[1] != 0 ? p.heads : 1;
+    m->batched = p.ms[0] != 0 ? 1 : 0;
+    m->wide = (p.mask_dtype == KTT_B200_MASK_F32 || p.mask_dtype == KTT_B200_MASK_F16) ? 1 : 0;
+    const int64_t planes = static_cast<int64_t>(m->heads) * (m->batched ? p.batch : 1);
+    const int64_t pieces = planes * m->groups * m->blocks;
+    const int64_t active = up256(planes * m->groups * m->words * 4), kind = up256(pieces), bits = up256(pieces * 32 * 16);
+    const int64_t values = p.mask_dtype == KTT_B200_MASK_BOOL ? 0 : pieces * 32 * 128 * (m->wide ? 4 : 2);
+    m->active = reinterpret_cast<uint32_t*>(base);
+    m->kind = base + active;
+    m->bits = reinterpret_cast<uint4*>(base + active + kind);
+    m->values = reinterpret_cast<uint4*>(base + active + kind + bits);
+    return active + kind + bits + values;
+}
+
+constexpr int64_t kHeaderBytes = 256;   // {int32 next item, int32 producers finished}
+
+int sm_count() {
+    static int sms[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (!sms[dev]) {
+        int n = 148;
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        sms[dev] = n;
+    }
+    return sms[dev];
+}
+
+template <typename Kernel, typename... Args>
+int launch_dependent(Kernel kernel, dim3 grid, int threads, int smem, cudaStream_t stream, const char* what, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, args...), what);
+}
+
+template <int DP>
+int launch_pair(const AttnParams& p, const CUtensorMap (&maps)[3], PairParams& tp, int grid, cudaStream_t stream) {
+    using P = PairPlan<DP>;
+    auto kernel = p.mask_dtype == KTT_B200_MASK_NONE ? fwd_pair_kernel<DP, 0> : mask_needs_plan(p) ? fwd_pair_kernel<DP, 2> : fwd_pair_kernel<DP, 1>;
+    if (int rc = ensure_smem(kernel, P::kBytes, "cudaFuncSetAttribute(fwd_pair)")) return rc;
+    return launch_dependent(kernel, dim3(grid), kPairThreads, P::kBytes, stream, "fwd_pair launch", maps[0], maps[1], maps[2], tp);
+}
+
+}  // namespace
+
+bool forward_pair_takes(const AttnParams& p) {
+    if (p.d > 128 || p.dv > 128 || p.d % 8 || p.dv % 8) return false;
+    // A plan covers the keys whatever a sequence's length, and 131,072 of them.
+    if (mask_needs_plan(p) && (p.cu_q || p.key_lengths || p.sk > kMaxPlanBlocks * kBN)) return false;
+    if (reinterpret_cast<uintptr_t>(p.out) & 15 || p.os[0] % 8 || p.os[1] % 8 || p.os[2] % 8) return false;
+    const int64_t tq = p.cu_q ? p.total_q : p.sq, tk = p.cu_q ? p.total_k : p.sk;
+    const int64_t bq = p.cu_q ? 1 : p.batch;
+    int64_t s[3];
+    const char* why;
+    return operand_layout(p.q, tq, p.heads, bq, p.qs, s, &why) && operand_layout(p.k, tk, p.kv_heads, bq, p.ks, s, &why) &&
+           operand_layout(p.v, tk, p.kv_heads, bq, p.vs, s, &why);
+}
+
+int64_t forward_pair_workspace(const AttnParams& p) {
+    MaskPlan m;
+    return kHeaderBytes + (mask_needs_plan(p) ? plan_layout(p, nullptr, &m) : 0);
+}
+
+int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
+    const char* why = "";
+    const int64_t tq = p.cu_q ? p.total_q : p.sq, tk = p.cu_q ? p.total_k : p.sk;
+    const int64_t bq = p.cu_q ? 1 : p.batch;
+    const void* base[3] = {p.q, p.k, p.v};
+    const int64_t rows[3] = {tq, tk, tk}, heads[3] = {p.heads, p.kv_heads, p.kv_heads};
+    const int64_t* strides[3] = {p.qs, p.ks, p.vs};
+    const int width[3] = {p.d, p.d, p.dv};
+    PairParams tp;
+    CUtensorMap maps[3];
+    for (int o = 0; o < 3; ++o) {
+        int64_t s[3];
+        if (!operand_layout(base[o], rows[o], heads[o], bq, strides[o], s, &why)) return fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 forward: %s", why);
+        const DimOrder order = order_of(s);
+        if (!encode_map(&maps[o], base[o], width[o], rows[o], heads[o], bq, s, order, kBM, &why)) return fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 forward: %s", why);
+        for (int i = 0; i < 3; ++i) tp.dim_of[o][i] = order.slot_of[i];
+    }
+    tp.a = p;
+    int* host_status = status_word(&tp.status);
+    if (!host_status || !tp.status) return fail(KTT_B200_ERR_LAUNCH, "tcgen05 forward: no status word");
+    if (*host_status != 0) {
+        const int code = *host_status;
+        *host_status = 0;
+        note_call(5);
+        return fail(KTT_B200_ERR_DEVICE_WAIT, "an earlier tcgen05 launch gave up waiting (code %d)", code);
+    }
+
+    const int group = p.heads / p.kv_heads;
+    const int q_tiles = (p.sq + kBM - 1) / kBM;
+    const int64_t units = static_cast<int64_t>(q_tiles) * group * p.kv_heads * p.batch;   // (query tile, head)
+    if (units > 0x3fffffff) return fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 forward: too many query tiles");
+    const int sms = sm_count();
+    tp.dual = p.sk > kBN && units <= 6 * static_cast<int64_t>(sms) ? 1 : 0;
+    const int levels = tp.dual ? q_tiles * group : (q_tiles * group + 1) / 2;
+    tp.work = levels * p.kv_heads * p.batch;
+    tp.by_batch = divisor_of(p.batch);
+    tp.by_kv_heads = divisor_of(p.kv_heads);
+    tp.by_group = divisor_of(group);
+    tp.by_levels = divisor_of(levels);
+
+    const bool planned = mask_needs_plan(p);
+    const bool usable = workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
+    if (planned) {
+        if (!usable || workspace_bytes < forward_pair_workspace(p)) {
+            return fail(KTT_B200_ERR_BAD_ARGUMENT, "tcgen05 forward: a mask with a row per query needs %lld bytes of workspace",
+                        static_cast<long long>(forward_pair_workspace(p)));
+        }
+        plan_layout(p, static_cast<unsigned char*>(workspace) + kHeaderBytes, &tp.plan);
+        const MaskPlan& m = tp.plan;
+        const int64_t planes = static_cast<int64_t>(m.heads) * (m.batched ? p.batch : 1);
+        const int size = p.mask_dtype == KTT_B200_MASK_BOOL ? 1 : p.mask_dtype == KTT_B200_MASK_F32 ? 4 : 2;
+        const bool vec = p.ms[3] == 1 && (reinterpret_cast<uintptr_t>(p.mask) % (4 * size)) == 0 && p.ms[0] % 4 == 0 && p.ms[1] % 4 == 0 && p.ms[2] % 4 == 0;
+        if (int rc = launch_dependent(vec ? mask_plan_kernel<true> : mask_plan_kernel<false>, dim3(m.groups, static_cast<unsigned>(planes)), 256, 0, stream,
+                                      "mask_plan launch", p, tp.plan, static_cast<int32_t*>(workspace))) return rc;
+    }
+    // K / V beyond what L2 keeps (126 MB on B200): the grouped order, which needs the counter.
+    const int64_t kv_bytes = (p.cu_q ? p.total_k : static_cast<int64_t>(p.batch) * p.sk) * p.kv_heads * (p.d + p.dv) * 2;
+    const bool large = kv_bytes > (96ll << 20);
+    // The counter pays when a CTA gets several items; with one or two the fixed deal (longest
+    // first, snake order) is as even and saves the trip to the counter before each item's first
+    // load. A workspace of 4 to 255 bytes is one int32 the caller zeroes before every call.
+    const bool header = usable && workspace_bytes >= kHeaderBytes;
+    const bool drawn = header ? tp.work > 2 * static_cast<int64_t>(sms) : workspace && (reinterpret_cast<uintptr_t>(workspace) & 3) == 0 && workspace_bytes >= 4;
+    tp.work_counter = drawn ? static_cast<int*>(workspace) : nullptr;
+    tp.done_counter = drawn && header ? static_cast<int*>(workspace) + 1 : nullptr;
+    tp.grouped = drawn && large ? 1 : 0;
+    const int grid = tp.work < sms ? tp.work : sms;
+    if (p.d <= 64 && p.dv <= 64) return launch_pair<64>(p, maps, tp, grid, stream);
+    return launch_pair<128>(p, maps, tp, grid, stream);
+}
+
+}  // namespace ktt

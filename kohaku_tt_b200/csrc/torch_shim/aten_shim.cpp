@@ -124,20 +124,20 @@ void mask_operand(ktt_b200_attn_args& a, const c10::optional<Tensor>& mask, int6
     keep = m;
 }
 
-// The head-dim-64 forward's workspace: one zero-filled buffer per (device, stream); the kernel
-// leaves it zero.
+// The tcgen05 forward's workspace. Without a mask that has a row per query it is the counter the
+// CTAs draw their tiles from: one zero-filled buffer per (device, stream), which the kernel
+// leaves zero. A plan of such a mask is as large as the mask and belongs to the call.
+constexpr int64_t kHeaderBytes = 256;
 Tensor forward_workspace(const ktt_b200_attn_args& a, const Tensor& like, cudaStream_t stream) {
     const int64_t need = ktt_b200_sdpa_forward_workspace(&a);
     if (need <= 0) return Tensor();
+    if (need > kHeaderBytes) return at::empty({need}, like.options().dtype(at::kByte));
     static std::mutex mu;
     static std::unordered_map<uint64_t, Tensor> cache;
     const uint64_t key = (static_cast<uint64_t>(like.get_device()) << 56) ^ reinterpret_cast<uint64_t>(stream);
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
-    if (it == cache.end() || it->second.numel() < need) {
-        Tensor buf = at::zeros({need}, like.options().dtype(at::kByte));
-        it = cache.insert_or_assign(key, buf).first;
-    }
+    if (it == cache.end()) it = cache.emplace(key, at::zeros({kHeaderBytes}, like.options().dtype(at::kByte))).first;
     return it->second;
 }
 

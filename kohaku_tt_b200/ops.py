@@ -140,18 +140,26 @@ def dynamic_work(on=True, min_items_per_sm=6):
 _FORWARD_WORKSPACE = {}
 
 
+_COUNTER_BYTES = 256
+
+
 def forward_workspace(args, device):
-    """The head-dim-64 forward kernel's workspace (the counter its CTAs draw their tiles
-    from): one zero-filled buffer per (device, stream); the kernel leaves it zero, so it is
-    filled once. Returns the buffer or None when the kernel that will run uses none."""
+    """The tcgen05 forward's workspace, or None when the kernel that will run uses none. Without
+    a mask that has a row per query that is the counter its CTAs draw their tiles from: one
+    zero-filled buffer per (device, stream), which the kernel leaves zero, so it is filled
+    once. With such a mask the plan of the mask follows, as large as the mask; it belongs to
+    the call, which clears the counter in front of it itself."""
     need = _lib.lib().ktt_b200_sdpa_forward_workspace(ctypes.byref(args))
     if need <= 0:
         return None
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
-    buf = _FORWARD_WORKSPACE.get(key)
-    if buf is None or buf.numel() < need:
-        buf = torch.zeros((need,), dtype=torch.uint8, device=device)
-        _FORWARD_WORKSPACE[key] = buf
+    if need > _COUNTER_BYTES:
+        buf = torch.empty((need,), dtype=torch.uint8, device=device)
+    else:
+        key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+        buf = _FORWARD_WORKSPACE.get(key)
+        if buf is None:
+            buf = torch.zeros((_COUNTER_BYTES,), dtype=torch.uint8, device=device)
+            _FORWARD_WORKSPACE[key] = buf
     args.workspace, args.workspace_bytes = buf.data_ptr(), buf.numel()
     return buf
 
@@ -167,7 +175,8 @@ def _work_counter(args, device, dynamic=None):
     zeroed counter when dynamic work distribution applies (`dynamic`: this call's own
     choice, None = the module setting; False also keeps the head-dim-64 kernel on its fixed
     deal of whole tiles)."""
-    if dynamic is not False:
+    planned = args.mask_dtype != _lib.MASK_NONE and args.mask_strides[2] != 0
+    if dynamic is not False or planned:
         buf = forward_workspace(args, device)
         if buf is not None:
             return buf

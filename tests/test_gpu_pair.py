@@ -1,0 +1,88 @@
+"""The forward kernel of two query tiles per CTA (csrc/fwd_pair.cu): head dims it zero-fills and
+masks with a row per query, at the edges of its tiles, against the float64 ruler."""
+
+import math
+
+import pytest
+import torch
+
+import kohaku_tt_b200 as ktt
+from kohaku_tt_b200 import _lib, ops
+from oracle import attention_oracle as ao
+from tests.gpu_util import FWD_BOUND, LSE_RMS, qkv, rel, rms
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(cuda, q, k, v, mask=None, causal=False, lengths=None):
+    before = ktt.counters()["attention_flash"]
+    ln = None if lengths is None else torch.tensor(lengths, dtype=torch.int32, device=cuda)
+    out, lse = ops.sdpa_forward(q.to(cuda), k.to(cuda), v.to(cuda), causal=causal, key_lengths=ln,
+                                mask=None if mask is None else mask.to(cuda))
+    torch.cuda.synchronize()
+    _lib.device_status()
+    assert ktt.counters()["attention_flash"] == before + 1   # the tcgen05 kernel took it
+    if lengths is not None:
+        ruler = ao.ruler_lengths(q, k, v, lengths)
+    else:
+        ruler = ao.ruler_dense(q, k, v, mask=mask, causal=causal)
+        assert rms(lse, ao.ruler_lse(q, k, v, mask=mask, causal=causal)) <= LSE_RMS
+    assert rel(out, ruler) <= FWD_BOUND
+
+
+# One key or row past a tile, a tile exactly, one short of it; a block with 1, 16, 17 and 128 keys;
+# one tile (its keys in two halves), an odd number of tiles, more tiles than CTAs.
+@pytest.mark.parametrize("b,h,hk,sq,sk,d,dv,causal", [
+    (1, 1, 1, 1, 1, 8, 8, False), (1, 2, 1, 128, 144, 80, 80, False), (2, 3, 3, 129, 257, 80, 80, False),
+    (1, 6, 2, 127, 145, 96, 96, True), (2, 2, 2, 300, 128, 40, 40, True), (1, 5, 1, 400, 400, 72, 72, True),
+    (1, 4, 2, 130, 200, 64, 128, False), (1, 2, 2, 200, 130, 120, 16, False), (40, 8, 8, 257, 257, 88, 88, False),
+])
+def test_head_dims(cuda, b, h, hk, sq, sk, d, dv, causal):
+    _check(cuda, *qkv(b, h, hk, sq, sk, d, sq + sk + d, dv=dv), causal=causal)
+
+
+def test_head_dim_80_with_key_lengths_and_a_key_mask(cuda):
+    q, k, v = qkv(3, 4, 2, 200, 300, 80, 5)
+    _check(cuda, q, k, v, lengths=[300, 1, 130])
+    keep = torch.rand(3, 1, 1, 300, generator=torch.Generator().manual_seed(6)) > 0.3
+    keep[..., 0] = True
+    _check(cuda, q, k, v, mask=keep)
+
+
+def _mask(kind, b, h, sq, sk):
+    g = torch.Generator().manual_seed(sq + sk)
+    if kind == "values":                       # every piece has values
+        return torch.randn(b, h, sq, sk, generator=g)
+    if kind == "bf16":
+        return torch.randn(b, 1, sq, sk, generator=g).to(torch.bfloat16)
+    if kind == "fp16":
+        return torch.randn(1, h, sq, sk, generator=g).to(torch.float16)
+    if kind == "random":                       # yes / no everywhere
+        keep = torch.rand(b, 1, sq, sk, generator=g) > 0.5
+        keep[..., 0] = True
+        return keep
+    keep = torch.ones(sq, sk, dtype=torch.bool).tril(max(sk - sq, 0))   # blocks hidden, free and mixed
+    if kind == "causal":
+        return keep
+    add = torch.zeros(1, 1, sq, sk).masked_fill(~keep, -math.inf)
+    if kind == "mixed":                        # a value in one piece, and a row that sees nothing
+        add[..., 5, 3] = -1.5
+        add[..., sq // 2, :] = -5e5
+    return add
+
+
+@pytest.mark.parametrize("kind", ["values", "bf16", "fp16", "random", "causal", "additive", "mixed"])
+@pytest.mark.parametrize("b,h,hk,sq,sk,d", [
+    (2, 4, 4, 257, 300, 64), (1, 6, 2, 128, 129, 128), (2, 2, 2, 33, 520, 96), (2, 16, 16, 700, 700, 64),
+])
+def test_masks_with_a_row_per_query(cuda, kind, b, h, hk, sq, sk, d):
+    q, k, v = qkv(b, h, hk, sq, sk, d, sq + sk + d)
+    _check(cuda, q, k, v, mask=_mask(kind, b, h, sq, sk))
+
+
+def test_mask_strides(cuda):
+    # A slice of a wider mask (rows start anywhere), a mask broadcast over the keys, an odd width.
+    q, k, v = qkv(2, 4, 4, 150, 203, 64, 9)
+    wide = torch.randn(2, 1, 150, 211, generator=torch.Generator().manual_seed(7)).to(torch.bfloat16)
+    _check(cuda, q, k, v, mask=wide[..., 5:208])
+    _check(cuda, q, k, v, mask=wide[..., :1])
