@@ -201,6 +201,8 @@ SHIM_PATH = os.path.join(LIB_DIR, "libktt_b200_aten.so")
 def build_shim(force=False):
     """Compiles the C++ registration of the aten overloads (csrc/torch_shim/aten_shim.cpp)
     against the installed torch and libktt_b200.so. Returns its path."""
+    import sysconfig
+
     import torch
     from torch.utils import cpp_extension
 
@@ -215,8 +217,8 @@ def build_shim(force=False):
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     for inc in cpp_extension.include_paths():
         cmd += ["-I", inc]
-    cmd += ["-I", os.path.join(cuda_home, "include"), SHIM_SRC, "-o", tmp,
-            "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+    cmd += ["-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda_home, "include"), SHIM_SRC, "-o", tmp,
+            "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
             "-L", LIB_DIR, "-lktt_b200", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
@@ -241,6 +243,26 @@ def shim():
         handle.ktt_b200_aten_set_scope.restype = None
         _SHIM = handle
     return _SHIM
+
+
+_NATIVE = None
+
+
+def native():
+    """The shim as a Python module (the eager fast paths), or None when it has not been built or
+    KTT_B200_PYTHON_ATEN=1 asks for the Python registration."""
+    global _NATIVE
+    if _NATIVE is None:
+        _NATIVE = False
+        if os.environ.get("KTT_B200_PYTHON_ATEN", "0") != "1" and shim() is not None:
+            import importlib.machinery
+            import importlib.util
+
+            loader = importlib.machinery.ExtensionFileLoader("ktt_b200_native", SHIM_PATH)
+            spec = importlib.util.spec_from_file_location("ktt_b200_native", SHIM_PATH, loader=loader)
+            _NATIVE = importlib.util.module_from_spec(spec)
+            loader.exec_module(_NATIVE)
+    return _NATIVE or None
 
 
 _LIB = None

@@ -5,7 +5,7 @@ kohakutt.sdpa_varlen (src/kohakutt/attention.py:10-76)."""
 import torch
 import torch.nn.functional as F
 
-from . import aten, ops
+from . import _lib, aten, ops
 
 # The logit of a key a bool mask leaves out, and the floor of an additive mask
 # (kohakutt/torch_backend/varlen.py:163-165).
@@ -76,8 +76,19 @@ def sdpa(q, k, v, key_lengths=None, is_causal=False, scale=None):
     if key_lengths is None:
         return F.scaled_dot_product_attention(q, k, v, is_causal=is_causal, scale=scale,
                                               enable_gqa=q.size(1) != k.size(1))
-    lengths = device_lengths(key_lengths, q.size(0), k.size(-2), q.device)
     causal = bool(is_causal)
+    # Eager calls on plain CUDA tensors are served by C++ in one step (None: not such a call). A
+    # compiled graph sees the operators below.
+    eager = not torch.compiler.is_compiling() and _lib.native()
+    if eager:
+        out = eager.sdpa_lengths(q, k, v, key_lengths, causal, scale)
+        if out is not None:
+            return out
+    lengths = device_lengths(key_lengths, q.size(0), k.size(-2), q.device)
+    if eager:
+        out = eager.sdpa_lengths(q, k, v, lengths, causal, scale)
+        if out is not None:
+            return out
     wants_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
     if wants_grad:
         return _Lengths.apply(q, k, v, lengths, causal, scale)
@@ -93,8 +104,11 @@ def decode_step(q, k_new, v_new, k_cache, v_cache, lengths, cos, sin, scale=None
     [B, D] rows for this step, or a [positions, D] table looked up at lengths[b]. No
     gradients. Returns out [B, H, 1, D]; k_cache / v_cache are updated in place and
     lengths_out (optional, another buffer) receives lengths + 1."""
-    from . import ops
-
+    eager = not torch.compiler.is_compiling() and _lib.native()
+    if eager:
+        out = eager.decode_step(q, k_new, v_new, k_cache, v_cache, lengths, cos, sin, scale, lengths_out)
+        if out is not None:
+            return out
     with torch.no_grad():
         return ops.decode_append(q, k_new, v_new, k_cache, v_cache, lengths, cos, sin,
                                  scale=scale, lengths_out=lengths_out)
@@ -179,6 +193,11 @@ def sdpa_varlen(q, k, v, cu_seq_q, cu_seq_k=None, max_q=None, max_k=None, is_cau
     validated on the host before anything is launched; the kernels then read their
     device copy."""
     causal = bool(is_causal)
+    eager = attn_mask is None and not torch.compiler.is_compiling() and _lib.native()
+    if eager:
+        out = eager.sdpa_varlen(q, k, v, cu_seq_q, cu_seq_k, max_q, max_k, causal, scale)
+        if out is not None:
+            return out
     cu_q = offsets(cu_seq_q)
     cu_k = offsets(cu_seq_k) if cu_seq_k is not None else cu_q
     check_offsets(cu_q, cu_k, q.size(0), k.size(0), causal)
@@ -188,6 +207,11 @@ def sdpa_varlen(q, k, v, cu_seq_q, cu_seq_k=None, max_q=None, max_k=None, is_cau
 
     max_q = longest(cu_q) if max_q is None else max_q
     max_k = longest(cu_k) if max_k is None else max_k
+    if eager:   # offsets from a list or the device: the same, now that they are on the host
+        out = eager.sdpa_varlen(q, k, v, torch.tensor(cu_q, dtype=torch.int32), torch.tensor(cu_k, dtype=torch.int32),
+                                max_q, max_k, causal, scale)
+        if out is not None:
+            return out
     dev_q = torch.tensor(cu_q, dtype=torch.int32, device=q.device)
     dev_k = dev_q if cu_k == cu_q else torch.tensor(cu_k, dtype=torch.int32, device=q.device)
     if attn_mask is None:

@@ -168,6 +168,9 @@ def drop_forward_workspaces():
     """Forgets the cached forward workspaces (after a device-wait error their counters may
     be left non-zero)."""
     _FORWARD_WORKSPACE.clear()
+    native = _lib.native()
+    if native is not None:
+        native.drop_workspaces()
 
 
 def _work_counter(args, device, dynamic=None):
