@@ -58,50 +58,65 @@ struct BwdParams {
 };
 
 
-// Shared-memory plan: a resident pair of tiles (A0, A1), a ring of streamed pairs (B0, B1),
-// two double-buffered vectors of 128 floats, barriers.
+// Shared-memory plan: a resident pair of tiles (A0, A1), a ring of streamed tiles (dK/dV body: Q,
+// dO, Q, dO, ...; dQ body: K, V, K, V, ...), the row terms of the query blocks in flight, barriers.
+// The ring holds single tiles, not pairs: dO (V) is done with well before Q (K) of the same item,
+// and at D 128, where five tiles fit, that is the difference between a next item whose loads are
+// under way and one that waits for them (measured, dQ body: 3,004 clk an item with two pairs).
 template <int D>
 struct BwdPlan {
     static constexpr int kSub = D / 64;
     static constexpr int kTile = 128 * 128;              // one [128][64] bf16 sub-tile
-    static constexpr int kStages = D == 64 ? 4 : 2;
+    static constexpr int kOperand = kSub * kTile;
+    static constexpr int kSlots = D == 64 ? 8 : 5;
+    // Row terms in flight. An item's buffer is written again kTerms items later, when the load of
+    // that item's dO goes out: it waits for the slot's previous tile, dO of four items before
+    // (D 64; released behind P of that item, so the threads have left the item before it) or Q of
+    // two items before (D 128; released behind that item's dS).
+    static constexpr int kTerms = D == 64 ? 5 : 2;
     static constexpr int kA0 = 0;
-    static constexpr int kA1 = kA0 + kSub * kTile;
-    static constexpr int kB0 = kA1 + kSub * kTile;
-    static constexpr int kB1 = kB0 + kStages * kSub * kTile;
-    static constexpr int kVec = kB1 + kStages * kSub * kTile;  // float [3 buffers][2 vectors][128] (dK/dV), [2][128] mask terms (dQ)
-    static constexpr int kBars = kVec + 2 * 3 * 128 * 4;
-    static constexpr int kBytes = kBars + 256;
+    static constexpr int kA1 = kA0 + kOperand;
+    static constexpr int kRing = kA1 + kOperand;
+    static constexpr int kVec = kRing + kSlots * kOperand;   // float [kTerms][-lse, delta][128]; dQ body: [2][128] mask terms
+    static constexpr int kBars = kVec + kTerms * 1024;
+    static constexpr int kBarBytes = 384;
+    static constexpr int kBytes = kBars + kBarBytes;
+    static_assert(kBytes <= 232448, "shared memory per CTA");
     static constexpr int bAFull = 0;
-    static constexpr int bBFull = 1;                  // + stage
-    static constexpr int bBEmpty = bBFull + kStages;  // + stage
-    static constexpr int bSReady = bBEmpty + kStages; // + score buffer
-    static constexpr int bDPReady = bSReady + 2;
-    static constexpr int bPFull = bDPReady + 1;       // + half
-    static constexpr int bDone = bPFull + 2;
+    static constexpr int bFull = 1;                   // + slot
+    static constexpr int bEmpty = bFull + kSlots;     // + slot
+    static constexpr int bTerms = bEmpty + kSlots;    // + buffer
+    static constexpr int bSReady = bTerms + kTerms;   // + score buffer
+    static constexpr int bDPReady = bSReady + 2;      // + dP buffer (the dK/dV body has one)
+    // P of 32 queries is stored (dK/dV body: + 4 score buffer + 2 half + quarter); dS is stored (dQ
+    // body: + 2 (block & 1) + half; dK/dV body: + half). A half may be an item ahead of the other
+    // while the MMA warp waits for that one, and a parity wait tells phases apart only one step
+    // deep: where the next item's scores and dP go out before this item's P or dS has been waited
+    // for, consecutive items have barriers of their own.
+    static constexpr int bPFull = bDPReady + 2;
+    static constexpr int bDSFull = bPFull + 8;
+    static constexpr int bSFree = bDSFull + 4;        // dQ body: the scores are in registers
+    static constexpr int bDone = bSFree + 1;
     static constexpr int bMeet = bDone + 1;           // the eight score warps meet (bounded, unlike bar.sync)
     static constexpr int bCount = bMeet + 1;
-    static_assert(bCount * 8 + 16 <= 256, "barrier area");
+    static_assert(bCount * 8 + 16 <= kBarBytes, "barrier area");
 };
 
+// By the whole producer warp, a barrier or two per lane (one lane after the other's barriers took
+// 40 dependent stores of every CTA's set-up).
 template <int D>
-__device__ __forceinline__ void init_barriers(uint32_t bars, volatile int* abort_flag) {
+__device__ __forceinline__ void init_barriers(uint32_t bars, volatile int* abort_flag, int lane) {
     using P = BwdPlan<D>;
-    mbar_init(bars + 8 * P::bAFull, 1);
-    for (int s = 0; s < P::kStages; ++s) {
-        mbar_init(bars + 8 * (P::bBFull + s), 1);
-        mbar_init(bars + 8 * (P::bBEmpty + s), 1);
+    for (int i = lane; i < P::bCount; i += 32) {
+        uint32_t count = 1;
+        if (i >= P::bPFull && i < P::bSFree) count = 4;   // one arrival per warp of the group
+        if (i == P::bSFree || i == P::bMeet) count = 8;
+        mbar_init(bars + 8 * i, count);
     }
-    mbar_init(bars + 8 * (P::bSReady + 0), 1);
-    mbar_init(bars + 8 * (P::bSReady + 1), 1);
-    mbar_init(bars + 8 * P::bDPReady, 1);
-    mbar_init(bars + 8 * (P::bPFull + 0), 4);   // one arrival per warp of the group
-    mbar_init(bars + 8 * (P::bPFull + 1), 4);
-    mbar_init(bars + 8 * P::bDone, 1);
-    mbar_init(bars + 8 * P::bMeet, 8);
-    *abort_flag = 0;
+    if (lane == 0) *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
+    __syncwarp();
 }
 
 // Phase stamp of a CTA's first thread (slots 4..7 of its trace row), while a buffer is set.
@@ -164,26 +179,35 @@ __device__ __forceinline__ void dkv_body(
         c[tp.dim_of[operand][2]] = batch;
     };
     const int batch_c = p.cu_q ? 0 : b;
-    // Q and dO tiles of item `it` into their ring stage (producer warp, converged; called for
-    // it = 0, 1, 2, ... in turn, so head and query block are counted, not divided out).
+    // Ring tile x (item x / 2: Q, then dO) into its slot (producer warp, converged; called for x = 0,
+    // 1, 2, ... in turn, so head and query block are counted, not divided out).
     int ld_head = 0, ld_qb = 0;
-    auto load_item = [&](int it) {
-        int c[4], c2[4];
-        c[0] = c2[0] = 0;
-        const int st = it % P::kStages;
-        const int h = hk * full_group + g0 + ld_head;
-        const int q0 = (qstart + ld_qb) * kBN;
-        if (++ld_qb == per_head) {
+    auto load_tile = [&](int x) {
+        const int st = x % P::kSlots, op = (x & 1) ? 3 : 0;
+        const int h = hk * full_group + g0 + ld_head, q0 = (qstart + ld_qb) * kBN;
+        if ((x & 1) && ++ld_qb == per_head) {
             ld_qb = 0;
             ++ld_head;
         }
-        coords(0, si.q_off + q0, h, batch_c, c);
-        coords(3, si.q_off + q0, h, batch_c, c2);
-        mbar_expect_tx(bar(P::bBFull + st), 2 * P::kSub * P::kTile);
+        int c[4];
+        c[0] = 0;
+        coords(op, si.q_off + q0, h, batch_c, c);
+        mbar_expect_tx(bar(P::bFull + st), P::kOperand);
         for (int s = 0; s < P::kSub; ++s) {
-            tma_load_4d(sbase + P::kB0 + (st * P::kSub + s) * P::kTile, &map_q, bar(P::bBFull + st), s * 64, c[1], c[2], c[3]);
-            tma_load_4d(sbase + P::kB1 + (st * P::kSub + s) * P::kTile, &map_do, bar(P::bBFull + st), s * 64, c2[1], c2[2], c2[3]);
+            tma_load_4d(sbase + P::kRing + st * P::kOperand + s * P::kTile, op ? &map_do : &map_q, bar(P::bFull + st), s * 64, c[1], c[2], c[3]);
         }
+    };
+    // Row terms of item `it`, in turn as well.
+    int tm_head = 0, tm_qb = 0;
+    auto load_terms = [&](int it) {
+        const int buf = it % P::kTerms;
+        const float* src = p.row_terms + (first_row_block(p, si, b, hk * full_group + g0 + tm_head) + qstart + tm_qb) * 256;
+        if (++tm_qb == per_head) {
+            tm_qb = 0;
+            ++tm_head;
+        }
+        mbar_expect_tx(bar(P::bTerms + buf), 1024);
+        bulk_load(sbase + P::kVec + buf * 1024, src, 1024, bar(P::bTerms + buf));
     };
 
     // Set-up. The producer warp initialises the barriers itself and sends the CTA's first
@@ -191,8 +215,7 @@ __device__ __forceinline__ void dkv_body(
     // launch may overlap) while warp 8 allocates tensor memory and the rest wait.
     int issued = 0;
     if (warp == 9) {
-        if (lane == 0) init_barriers<D>(bars, abort_flag);
-        __syncwarp();
+        init_barriers<D>(bars, abort_flag, lane);
         if (nitems > 0) {
             int c[4], c2[4];
             c[0] = c2[0] = 0;
@@ -203,7 +226,7 @@ __device__ __forceinline__ void dkv_body(
                 tma_load_4d(sbase + P::kA0 + s * P::kTile, &map_k, bar(P::bAFull), s * 64, c[1], c[2], c[3]);
                 tma_load_4d(sbase + P::kA1 + s * P::kTile, &map_v, bar(P::bAFull), s * 64, c2[1], c2[2], c2[3]);
             }
-            for (; issued < nitems && issued < P::kStages; ++issued) load_item(issued);
+            for (; issued < 2 * nitems && issued < P::kSlots; ++issued) load_tile(issued);
         }
     }
     if (warp == 8) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
@@ -217,23 +240,28 @@ __device__ __forceinline__ void dkv_body(
     mark(tp, 4);   // set-up done
     // S^T buffers at columns 0 and (D 64 only) 384; dP^T 128; dV 256; dK 256 + D.
     constexpr int kSBufs = 256 + 2 * D + 128 <= kTmemCols ? 2 : 1;
+    // P is handed over 32 queries of a half at a time where the next scores wait for its columns, a
+    // half at a time where they have a buffer of their own (each wait is 100 clk of the MMA warp's
+    // item).
+    constexpr int kQuarters = kSBufs == 1 ? 2 : 1;
     const uint32_t tmem_dp = tmem + 128, tmem_dv = tmem + 256, tmem_dk = tmem + 256 + D;
     auto tmem_s_of = [&](int it) { return tmem + ((kSBufs == 2 && (it & 1)) ? 384u : 0u); };
 
     if (warp == 9) {
         // ---------------- producer ----------------
         if (nitems > 0) {
-            for (int it = issued; it < nitems; ++it) {
-                const int st = it % P::kStages;
-                if (!__all_sync(0xffffffffu, mbar_wait(bar(P::bBEmpty + st), ((it / P::kStages) - 1) & 1, abort_flag, 400 + st, tp.status))) break;
-                load_item(it);
+            for (int it = 0; it < issued / 2; ++it) load_terms(it);   // not before the previous kernel is done: it wrote them
+            for (int x = issued; x < 2 * nitems; ++x) {
+                const int st = x % P::kSlots;
+                if (!__all_sync(0xffffffffu, mbar_wait(bar(P::bEmpty + st), ((x / P::kSlots) - 1) & 1, abort_flag, 400 + st, tp.status))) break;
+                load_tile(x);
+                if (x & 1) load_terms(x >> 1);
                 ++issued;
             }
             if (*abort_flag) {
-                for (int it = max(0, issued - P::kStages); it < issued; ++it) {
-                    const int st = it % P::kStages;
+                for (int x = max(0, issued - P::kSlots); x < issued; ++x) {
                     const long long t0 = clock64();
-                    while (!mbar_try_wait(bar(P::bBFull + st), (it / P::kStages) & 1) && clock64() - t0 < kWaitCycles / 8) {
+                    while (!mbar_try_wait(bar(P::bFull + x % P::kSlots), (x / P::kSlots) & 1) && clock64() - t0 < kWaitCycles / 8) {
                     }
                 }
             }
@@ -245,10 +273,11 @@ __device__ __forceinline__ void dkv_body(
             constexpr uint32_t idesc_g = instr_desc(D, true);     // 128 x D, B MN-major
             const uint64_t k_desc = smem_desc(sbase + P::kA0, 16, 1024);
             const uint64_t v_desc = smem_desc(sbase + P::kA1, 16, 1024);
-            const uint64_t q_desc = smem_desc(sbase + P::kB0, 16, 1024);
-            const uint64_t do_desc = smem_desc(sbase + P::kB1, 16, 1024);
-            const uint64_t q_mn = smem_desc(sbase + P::kB0, P::kTile, 1024);
-            const uint64_t do_mn = smem_desc(sbase + P::kB1, P::kTile, 1024);
+            // Ring tiles as the K-major B operand (Q of S, dO of dP) and as the MN-major one (dO of dV, Q
+            // of dK).
+            const uint64_t b_desc = smem_desc(sbase + P::kRing, 16, 1024);
+            const uint64_t b_mn = smem_desc(sbase + P::kRing, P::kTile, 1024);
+            auto slot_off = [](int x) { return static_cast<uint32_t>((x % P::kSlots) * (P::kOperand >> 4)); };
             bool ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bAFull), 0, abort_flag, 500, tp.status));
             if (ok && p.key_lengths && si.klen - k0 < kBM) {
                 // Cache rows past the length may hold anything (0 x inf would poison dK and dV):
@@ -265,53 +294,80 @@ __device__ __forceinline__ void dkv_body(
             }
             // S^T = K Q^T of item `it` into its score buffer (the previous reader of that
             // buffer, dV of an earlier item, was issued before: MMAs run in issue order).
+            auto wait_tile = [&](int x, int code) -> bool {
+                return __all_sync(0xffffffffu, mbar_wait(bar(P::bFull + x % P::kSlots), (x / P::kSlots) & 1, abort_flag, code, tp.status));
+            };
             auto issue_s = [&](int it) -> bool {
-                const int st = it % P::kStages;
-                const uint32_t soff = (st * P::kSub * P::kTile) >> 4;
-                if (!__all_sync(0xffffffffu, mbar_wait(bar(P::bBFull + st), (it / P::kStages) & 1, abort_flag, 510 + st, tp.status))) return false;
+                if (!wait_tile(2 * it, 510)) return false;
                 tc_fence_after();
+                const uint64_t q_desc = b_desc + slot_off(2 * it);
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
                     const uint32_t off = ((ks / 4) * P::kTile + (ks % 4) * 32) >> 4;
-                    tc_mma(tmem_s_of(it), k_desc + off, q_desc + soff + off, idesc_s, ks > 0);
+                    tc_mma(tmem_s_of(it), k_desc + off, q_desc + off, idesc_s, ks > 0);
                 }
                 tc_commit(bar(P::bSReady + it % kSBufs));
                 return true;
             };
-            if (ok) ok = issue_s(0);
-            for (int it = 0; ok && it < nitems; ++it) {
-                const int st = it % P::kStages;
-                const uint32_t soff = (st * P::kSub * P::kTile) >> 4;
-                // dP^T = V dO^T, behind the previous item's dK (which read dS^T from there).
+            // dP^T = V dO^T of item `it` (behind dK of the item before, which read dS^T from there).
+            auto issue_dp = [&](int it) -> bool {
+                if (!wait_tile(2 * it + 1, 511)) return false;
+                tc_fence_after();
+                const uint64_t do_desc = b_desc + slot_off(2 * it + 1);
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
                     const uint32_t off = ((ks / 4) * P::kTile + (ks % 4) * 32) >> 4;
-                    tc_mma(tmem_dp, v_desc + off, do_desc + soff + off, idesc_s, ks > 0);
+                    tc_mma(tmem_dp, v_desc + off, do_desc + off, idesc_s, ks > 0);
                 }
                 tc_commit(bar(P::bDPReady));
-                if (kSBufs == 2 && it + 1 < nitems) {
-                    ok = issue_s(it + 1);
-                    if (!ok) break;
+                return true;
+            };
+            for (int it = 0; ok && it < kSBufs && it < nitems; ++it) {
+                ok = issue_s(it);
+                if (ok && it == 0) ok = issue_dp(0);
+            }
+            // P and dS of an item are handed over separately: dV runs as P is stored, 32 queries of each
+            // half at a time, behind it the scores of the next item that share P's columns, both
+            // while the threads are in their second phase; dK and the next item's dP follow when dS
+            // is stored. (With one hand-over for both an item was one serial chain: scores, P, dS,
+            // dV, dK; at D 128 that was 3,900 clk for 2,080 of tensor pipe.)
+            for (int it = 0; ok && it < nitems; ++it) {
+                const uint64_t do_mn = b_mn + slot_off(2 * it + 1), q_mn = b_mn + slot_off(2 * it);
+#pragma unroll
+                for (int c = 0; c < kQuarters; ++c) {
+#pragma unroll
+                    for (int g = 0; g < 2; ++g) {
+                        ok = ok && __all_sync(0xffffffffu, mbar_wait(bar(P::bPFull + 4 * (it % kSBufs) + 2 * g + c), (it / kSBufs) & 1, abort_flag, 520 + g, tp.status));
+                        if (!ok) break;
+                        tc_fence_after();
+#pragma unroll
+                        for (int ks = c * (4 / kQuarters); ks < (c + 1) * (4 / kQuarters); ++ks) {
+                            // 16 query rows of this half per step: A = P^T (8 TMEM columns), B = dO rows as
+                            // the MN-major operand (16 rows of 128 bytes).
+                            tc_mma_ts(tmem_dv, tmem_s_of(it) + g * 64 + ks * 8, do_mn + (((g * 4 + ks) * 2048) >> 4), idesc_g,
+                                      (it > 0 || g > 0 || ks > 0) ? 1u : 0u);
+                        }
+                    }
                 }
+                if (!ok) break;
+                tc_commit(bar(P::bEmpty + (2 * it + 1) % P::kSlots));
+                if (it + kSBufs < nitems) ok = issue_s(it + kSBufs);
+                if (!ok) break;
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bPFull + g), it & 1, abort_flag, 520 + g, tp.status));
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bDSFull + g), it & 1, abort_flag, 530 + g, tp.status));
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
-                        // 16 query rows of this half per step: A = P^T / dS^T (8 TMEM columns),
-                        // B = dO / Q rows as the MN-major operand (16 rows of 128 bytes).
-                        const uint32_t boff = soff + (((g * 4 + ks) * 2048) >> 4);
-                        const uint32_t acc = (it > 0 || g > 0 || ks > 0) ? 1u : 0u;
-                        tc_mma_ts(tmem_dv, tmem_s_of(it) + g * 64 + ks * 8, do_mn + boff, idesc_g, acc);
-                        tc_mma_ts(tmem_dk, tmem_dp + g * 64 + ks * 8, q_mn + boff, idesc_g, acc);
+                        tc_mma_ts(tmem_dk, tmem_dp + g * 64 + ks * 8, q_mn + (((g * 4 + ks) * 2048) >> 4), idesc_g,
+                                  (it > 0 || g > 0 || ks > 0) ? 1u : 0u);
                     }
                 }
                 if (!ok) break;
-                tc_commit(bar(P::bBEmpty + st));
+                tc_commit(bar(P::bEmpty + (2 * it) % P::kSlots));
                 if (it + 1 == nitems) tc_commit(bar(P::bDone));
-                if (kSBufs == 1 && it + 1 < nitems) ok = issue_s(it + 1);
+                if (it + 1 < nitems) ok = issue_dp(it + 1);
             }
         }
     } else {
@@ -343,63 +399,6 @@ __device__ __forceinline__ void dkv_body(
             }
         };
 
-        // Row terms of one item: group 0 threads fetch lse, group 1 threads fetch delta. The
-        // load is issued one item ahead and nothing looks at the loaded value until the next
-        // item starts (a select or a multiply right behind the load would make the warp sit
-        // out a trip to L2 in every item: measured, ~900 clk of a 3,300-clk item).
-        // (Head and query block of the item to fetch are kept as running counters and the row's
-        // address as a running pointer: the divisions and 64-bit products they replace were a
-        // fifth of an item, one dependent chain per warp with nothing to overlap it.)
-        int nxt_head = 0, nxt_qb = 0;   // item to fetch next: head inside this CTA's part, query block from qstart
-        const float* src_row = g == 0
-            ? p.lse + b * p.ls[0] + (hk * full_group + g0) * p.ls[1] + static_cast<int64_t>(si.q_off) * p.ls[2]
-            : p.delta + b * p.delta_bs + (hk * full_group + g0) * p.delta_hs + si.q_off;
-        const int64_t src_head = g == 0 ? p.ls[1] : p.delta_hs, src_step = g == 0 ? p.ls[2] : 1;
-        auto fetch = [&](bool& exists) -> float {
-            const int qi = (qstart + nxt_qb) * kBN + row;
-            exists = qi < si.lq;
-            const int qc = exists ? qi : 0;   // a row of this sequence, read and discarded
-            const float raw = src_row[nxt_head * src_head + qc * src_step];
-            if (++nxt_qb == per_head) {
-                nxt_qb = 0;
-                ++nxt_head;
-            }
-            return raw;
-        };
-        // What goes into the vectors: minus lse as base-2, ready to be added to the scaled
-        // score (-inf for rows that do not exist or saw no key: P exactly 0), and delta (0 for
-        // rows that do not exist).
-        auto row_term = [&](float raw, bool exists) -> float {
-            if (g == 0) {
-                const float l = raw * kLog2e;
-                return (!exists || l == -INFINITY) ? -INFINITY : -l;
-            }
-            return exists ? raw : 0.f;
-        };
-        // The vectors have three buffers (item mod 3) so that a warp can publish the terms of
-        // item i + 1 and sign in at that item's meeting while it starts on item i: the buffer
-        // it overwrites was read in item i - 2, which every warp has left (all have signed
-        // in at meeting i, which they do at the top of item i - 1). By the time a warp
-        // waits for meeting i + 1 the others have usually long signed in; met right after
-        // the write, the warps waited for the slowest of them in every item (560 clk of a
-        // 2,750-clk item).
-        auto publish = [&](int it, float raw, bool exists) {
-            float* buf = vec + (it % 3) * 256;
-            (g == 0 ? buf : buf + 128)[row] = row_term(raw, exists);
-            mbar_arrive_warp(bar(P::bMeet));
-        };
-        auto met_for = [&](int code) -> bool {
-            const bool met = __all_sync(0xffffffffu, mbar_wait(bar(P::bMeet), meets & 1, abort_flag, code, tp.status));
-            ++meets;
-            return met;
-        };
-        bool pre_exists = false;
-        float pre = 0.f;
-        if (nitems > 0) {
-            pre = fetch(pre_exists);
-            publish(0, pre, pre_exists);
-            if (nitems > 1) pre = fetch(pre_exists);
-        }
         // While a trace buffer is set the CTA's first thread adds up where its item loop
         // waits (row 64 + 512 + CTA: meeting, wait for S, phase 1, wait for dP, phase 2).
         const bool timing = tp.trace && (threadIdx.x & 31) == 0 && blockIdx.x < 56;   // one row of 8 slots per warp
@@ -413,13 +412,15 @@ __device__ __forceinline__ void dkv_body(
         };
 
         for (int it = 0; it < nitems; ++it) {
-            float* lse2 = vec + (it % 3) * 256;
-            float* delta = lse2 + 128;
-            ok = met_for(630);   // everybody's terms of item `it` are in
-            if (!ok) break;
-            if (it + 1 < nitems) publish(it + 1, pre, pre_exists);
+            // Row terms of the item's queries: minus lse in base 2, ready to be added to the scaled score
+            // (-inf for rows that do not exist or saw no key: P exactly 0), and delta. (Fetched by the
+            // threads themselves and shared at a meeting of the eight warps they cost 450 clk of an
+            // item.)
+            const float* lse2 = vec + (it % P::kTerms) * 256;
+            const float* delta = lse2 + 128;
             mask_term(it);
-            if (it + 2 < nitems) pre = fetch(pre_exists);
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bTerms + it % P::kTerms), (it / P::kTerms) & 1, abort_flag, 630, tp.status));
+            if (!ok) break;
             lap(0);
             const int q0 = (qstart + cur_qb) * kBN;
             const uint32_t tmem_s = tmem_s_of(it);
@@ -438,11 +439,13 @@ __device__ __forceinline__ void dkv_body(
             const bool whole_w = __all_sync(0xffffffffu, whole);
             const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
             float2 pv[32];
+            float sc_all[64];
+            tmem_ld32(tmem_s + lane_addr + g * 64, sc_all);
+            tmem_ld32(tmem_s + lane_addr + g * 64 + 32, sc_all + 32);
+            tmem_wait_ld();
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                float sc[32];
-                tmem_ld32(tmem_s + lane_addr + g * 64 + c * 32, sc);
-                tmem_wait_ld();
+                const float* sc = sc_all + c * 32;
                 const float4* l4 = reinterpret_cast<const float4*>(lse2 + g * 64 + c * 32);
                 if (whole_w) {
                     // Every thread of the warp sees all its columns: no tests, and some pairs
@@ -474,14 +477,16 @@ __device__ __forceinline__ void dkv_body(
                         pv[c * 16 + e4 * 2 + 1] = make_float2(fast_exp2(x1.x), fast_exp2(x1.y));
                     }
                 }
-            }
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
+                // P (bf16) goes over columns this thread has already consumed.
                 uint32_t wp[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) wp[e] = pack_bf16(pv[c * 16 + e].x, pv[c * 16 + e].y);
-                // Packed results go over columns this thread has already consumed.
                 tmem_st16(tmem_s + lane_addr + g * 64 + c * 16, wp);
+                if (kQuarters == 2 || c == 1) {
+                    tmem_wait_st();
+                    tc_fence_before();
+                    mbar_arrive_warp(bar(P::bPFull + 4 * (it % kSBufs) + 2 * g + (kQuarters == 2 ? c : 0)));
+                }
             }
             // Phase 2: dS^T = P^T o (dP^T - delta) over dP^T.
             lap(2);
@@ -508,7 +513,7 @@ __device__ __forceinline__ void dkv_body(
             }
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive_warp(bar(P::bPFull + g));
+            mbar_arrive_warp(bar(P::bDSFull + g));
             if (++cur_qb == per_head) {
                 cur_qb = 0;
                 ++cur_head;
@@ -691,17 +696,15 @@ __device__ __forceinline__ void dq_body(
         c[tp.dim_of[operand][2]] = batch;
     };
     const int batch_c = p.cu_q ? 0 : b;
-    // K and V tiles of key block j into their ring stage (producer warp, converged).
-    auto load_block = [&](int j) {
-        int c[4], c2[4];
-        c[0] = c2[0] = 0;
-        const int st = j % P::kStages;
-        coords(1, si.k_off + j * kBN, hk, batch_c, c);
-        coords(2, si.k_off + j * kBN, hk, batch_c, c2);
-        mbar_expect_tx(bar(P::bBFull + st), 2 * P::kSub * P::kTile);
+    // Ring tile x (key block x / 2: K, then V) into its slot (producer warp, converged).
+    auto load_tile = [&](int x) {
+        const int st = x % P::kSlots, op = (x & 1) ? 2 : 1;
+        int c[4];
+        c[0] = 0;
+        coords(op, si.k_off + (x >> 1) * kBN, hk, batch_c, c);
+        mbar_expect_tx(bar(P::bFull + st), P::kOperand);
         for (int s = 0; s < P::kSub; ++s) {
-            tma_load_4d(sbase + P::kB0 + (st * P::kSub + s) * P::kTile, &map_k, bar(P::bBFull + st), s * 64, c[1], c[2], c[3]);
-            tma_load_4d(sbase + P::kB1 + (st * P::kSub + s) * P::kTile, &map_v, bar(P::bBFull + st), s * 64, c2[1], c2[2], c2[3]);
+            tma_load_4d(sbase + P::kRing + st * P::kOperand + s * P::kTile, op == 2 ? &map_v : &map_k, bar(P::bFull + st), s * 64, c[1], c[2], c[3]);
         }
     };
 
@@ -709,8 +712,7 @@ __device__ __forceinline__ void dq_body(
     // first loads while tensor memory is being allocated.
     int issued = 0;
     if (warp == 9) {
-        if (lane == 0) init_barriers<D>(bars, abort_flag);
-        __syncwarp();
+        init_barriers<D>(bars, abort_flag, lane);
         if (nblocks > 0) {
             int c[4], c2[4];
             c[0] = c2[0] = 0;
@@ -721,7 +723,7 @@ __device__ __forceinline__ void dq_body(
                 tma_load_4d(sbase + P::kA0 + s * P::kTile, &map_q, bar(P::bAFull), s * 64, c[1], c[2], c[3]);
                 tma_load_4d(sbase + P::kA1 + s * P::kTile, &map_do, bar(P::bAFull), s * 64, c2[1], c2[2], c2[3]);
             }
-            for (; issued < nblocks && issued < P::kStages; ++issued) load_block(issued);
+            for (; issued < 2 * nblocks && issued < P::kSlots; ++issued) load_tile(issued);
         }
     }
     if (warp == 8) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
@@ -731,23 +733,25 @@ __device__ __forceinline__ void dq_body(
     asm volatile("griddepcontrol.wait;" ::: "memory");   // delta comes from the previous kernel in the stream
     const uint32_t tmem = *tmem_slot;
     mark(tp, 4);
-    // S buffers at columns 0 and 384, dP 128, dQ 256 (D <= 128 columns).
-    const uint32_t tmem_dp = tmem + 128, tmem_dq = tmem + 256;
-    auto tmem_s_of = [&](int j) { return tmem + ((j & 1) ? 384u : 0u); };
+    // S at column 0, dP buffers at 128 and 384, dQ 256 (D <= 128 columns). The scores leave for
+    // registers as soon as they land, so one buffer serves; dP waits there for its dS and then for
+    // dQ, so it has two. (The other way round dP of a block stood behind dQ of the block before,
+    // which stood behind that block's dS.)
+    const uint32_t tmem_dq = tmem + 256;
+    auto tmem_dp_of = [&](int j) { return tmem + ((j & 1) ? 384u : 128u); };
 
     if (warp == 9) {
         if (nblocks > 0) {
-            for (int j = issued; j < nblocks; ++j) {
-                const int st = j % P::kStages;
-                if (!__all_sync(0xffffffffu, mbar_wait(bar(P::bBEmpty + st), ((j / P::kStages) - 1) & 1, abort_flag, 700 + st, tp.status))) break;
-                load_block(j);
+            for (int x = issued; x < 2 * nblocks; ++x) {
+                const int st = x % P::kSlots;
+                if (!__all_sync(0xffffffffu, mbar_wait(bar(P::bEmpty + st), ((x / P::kSlots) - 1) & 1, abort_flag, 700 + st, tp.status))) break;
+                load_tile(x);
                 ++issued;
             }
             if (*abort_flag) {
-                for (int j = max(0, issued - P::kStages); j < issued; ++j) {
-                    const int st = j % P::kStages;
+                for (int x = max(0, issued - P::kSlots); x < issued; ++x) {
                     const long long t0 = clock64();
-                    while (!mbar_try_wait(bar(P::bBFull + st), (j / P::kStages) & 1) && clock64() - t0 < kWaitCycles / 8) {
+                    while (!mbar_try_wait(bar(P::bFull + x % P::kSlots), (x / P::kSlots) & 1) && clock64() - t0 < kWaitCycles / 8) {
                     }
                 }
             }
@@ -758,65 +762,70 @@ __device__ __forceinline__ void dq_body(
             constexpr uint32_t idesc_g = instr_desc(D, true);
             const uint64_t q_desc = smem_desc(sbase + P::kA0, 16, 1024);
             const uint64_t do_desc = smem_desc(sbase + P::kA1, 16, 1024);
-            const uint64_t k_desc = smem_desc(sbase + P::kB0, 16, 1024);
-            const uint64_t v_desc = smem_desc(sbase + P::kB1, 16, 1024);
-            const uint64_t k_mn = smem_desc(sbase + P::kB0, P::kTile, 1024);
+            const uint64_t b_desc = smem_desc(sbase + P::kRing, 16, 1024);    // K of S, V of dP
+            const uint64_t b_mn = smem_desc(sbase + P::kRing, P::kTile, 1024);   // K of dQ
+            auto slot_off = [](int x) { return static_cast<uint32_t>((x % P::kSlots) * (P::kOperand >> 4)); };
             bool ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bAFull), 0, abort_flag, 800, tp.status));
-            // S = Q K^T of block j into its buffer: free since the threads published dS of
-            // block j - 2 (they only read the scores).
-            auto issue_s = [&](int j) -> bool {
-                const int st = j % P::kStages;
-                const uint32_t soff = (st * P::kSub * P::kTile) >> 4;
-                if (!__all_sync(0xffffffffu, mbar_wait(bar(P::bBFull + st), (j / P::kStages) & 1, abort_flag, 810 + st, tp.status))) return false;
-                if (p.key_lengths && si.klen - j * kBN < kBN) {
-                    // Blank the key and value rows past the length (see the dK/dV body).
-                    const int first = si.klen - j * kBN;   // > 0: the block has a visible key
+            // S = Q K^T of block j, once the threads hold the block before in registers, and dP = dO V^T
+            // (its buffer was read by dQ of block j - 2, issued before).
+            // Waits for ring tile x and, in the block that straddles the length, blanks its rows past it
+            // (cache rows there may hold anything: see the dK/dV body).
+            auto wait_tile = [&](int x) -> bool {
+                if (!__all_sync(0xffffffffu, mbar_wait(bar(P::bFull + x % P::kSlots), (x / P::kSlots) & 1, abort_flag, 810, tp.status))) return false;
+                const int first = si.klen - (x >> 1) * kBN;   // > 0: the block has a visible key
+                if (p.key_lengths && first < kBN) {
                     for (int idx = lane; idx < P::kSub * (kBN - first) * 8; idx += 32) {
                         const int sub = idx / ((kBN - first) * 8), rem = idx % ((kBN - first) * 8);
-                        const int off = (st * P::kSub + sub) * P::kTile + (first + rem / 8) * 128 + (rem % 8) * 16;
-                        *reinterpret_cast<uint4*>(smem + P::kB0 + off) = make_uint4(0u, 0u, 0u, 0u);
-                        *reinterpret_cast<uint4*>(smem + P::kB1 + off) = make_uint4(0u, 0u, 0u, 0u);
+                        const int off = (x % P::kSlots) * P::kOperand + sub * P::kTile + (first + rem / 8) * 128 + (rem % 8) * 16;
+                        *reinterpret_cast<uint4*>(smem + P::kRing + off) = make_uint4(0u, 0u, 0u, 0u);
                     }
                     fence_async_smem();
                     __syncwarp();
                 }
+                return true;
+            };
+            auto issue_scores = [&](int j) -> bool {
+                if (!wait_tile(2 * j)) return false;
+                if (j > 0 && !__all_sync(0xffffffffu, mbar_wait(bar(P::bSFree), (j - 1) & 1, abort_flag, 815, tp.status))) return false;
+                tc_fence_after();
+                const uint64_t k_desc = b_desc + slot_off(2 * j), v_desc = b_desc + slot_off(2 * j + 1);
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    const uint32_t off = ((ks / 4) * P::kTile + (ks % 4) * 32) >> 4;
+                    tc_mma(tmem, q_desc + off, k_desc + off, idesc_s, ks > 0);
+                }
+                tc_commit(bar(P::bSReady));
+                if (!wait_tile(2 * j + 1)) return false;
                 tc_fence_after();
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
                     const uint32_t off = ((ks / 4) * P::kTile + (ks % 4) * 32) >> 4;
-                    tc_mma(tmem_s_of(j), q_desc + off, k_desc + soff + off, idesc_s, ks > 0);
+                    tc_mma(tmem_dp_of(j), do_desc + off, v_desc + off, idesc_s, ks > 0);
                 }
-                tc_commit(bar(P::bSReady + (j & 1)));
+                tc_commit(bar(P::bDPReady + (j & 1)));
+                tc_commit(bar(P::bEmpty + (2 * j + 1) % P::kSlots));
                 return true;
             };
-            if (ok) ok = issue_s(0);
+            if (ok) ok = issue_scores(0);
             for (int j = 0; ok && j < nblocks; ++j) {
-                const int st = j % P::kStages;
-                const uint32_t soff = (st * P::kSub * P::kTile) >> 4;
-                // dP = dO V^T, behind the previous block's dQ MMA (which read dS from there).
-#pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks) {
-                    const uint32_t off = ((ks / 4) * P::kTile + (ks % 4) * 32) >> 4;
-                    tc_mma(tmem_dp, do_desc + off, v_desc + soff + off, idesc_s, ks > 0);
-                }
-                tc_commit(bar(P::bDPReady));
+                const uint64_t k_mn = b_mn + slot_off(2 * j);
                 if (j + 1 < nblocks) {
-                    ok = issue_s(j + 1);
+                    ok = issue_scores(j + 1);
                     if (!ok) break;
                 }
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bPFull + g), j & 1, abort_flag, 820 + g, tp.status));
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bDSFull + 2 * (j & 1) + g), (j >> 1) & 1, abort_flag, 820 + g, tp.status));
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
-                        tc_mma_ts(tmem_dq, tmem_dp + g * 64 + ks * 8,
-                                  k_mn + soff + (((g * 4 + ks) * 2048) >> 4), idesc_g, (j > 0 || g > 0 || ks > 0) ? 1u : 0u);
+                        tc_mma_ts(tmem_dq, tmem_dp_of(j) + g * 64 + ks * 8,
+                                  k_mn + (((g * 4 + ks) * 2048) >> 4), idesc_g, (j > 0 || g > 0 || ks > 0) ? 1u : 0u);
                     }
                 }
                 if (!ok) break;
-                tc_commit(bar(P::bBEmpty + st));
+                tc_commit(bar(P::bEmpty + (2 * j) % P::kSlots));
                 if (j + 1 == nblocks) tc_commit(bar(P::bDone));
             }
         }
@@ -827,12 +836,8 @@ __device__ __forceinline__ void dq_body(
         const int qi = q0 + row;
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
         bool ok = true;
-        float lse2 = INFINITY, delta = 0.f;
-        if (qi < si.lq) {
-            lse2 = p.lse[b * p.ls[0] + h * p.ls[1] + (si.q_off + qi) * p.ls[2]] * kLog2e;
-            if (lse2 == -INFINITY) lse2 = INFINITY;  // a row without keys: P exactly 0
-            delta = p.delta[b * p.delta_bs + h * p.delta_hs + si.q_off + qi];
-        }
+        const float* terms = p.row_terms + (first_row_block(p, si, b, h) + qb) * 256 + row;
+        const float neg_lse = terms[0], delta = terms[128];   // -inf (P exactly 0) where the row does not exist or saw no key
         int row_limit = si.klen;
         if (p.causal) row_limit = min(row_limit, qi + si.shift + 1);
         float* vec = reinterpret_cast<float*>(smem + P::kVec);   // [block parity][128]: a block's mask terms
@@ -862,7 +867,7 @@ __device__ __forceinline__ void dq_body(
                 if (!ok) break;
             }
             lap(0);
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bSReady + (j & 1)), (j >> 1) & 1, abort_flag, 900 + g, tp.status));
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bSReady), j & 1, abort_flag, 900 + g, tp.status));
             if (!ok) break;
             tc_fence_after();
             lap(1);
@@ -873,14 +878,18 @@ __device__ __forceinline__ void dq_body(
             // tests.
             const bool whole = limit >= 64;
             const bool whole_w = __all_sync(0xffffffffu, whole);
-            const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(-lse2, -lse2);
+            const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(neg_lse, neg_lse);
             const float2 nd2 = make_float2(-delta, -delta);
             float2 pv[32];
+            float sc_all[64];
+            tmem_ld32(tmem + lane_addr + g * 64, sc_all);
+            tmem_ld32(tmem + lane_addr + g * 64 + 32, sc_all + 32);
+            tmem_wait_ld();
+            tc_fence_before();
+            mbar_arrive_warp(bar(P::bSFree));
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                float sc[32];
-                tmem_ld32(tmem_s_of(j) + lane_addr + g * 64 + c * 32, sc);
-                tmem_wait_ld();
+                const float* sc = sc_all + c * 32;
                 if (whole_w) {
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
@@ -909,7 +918,8 @@ __device__ __forceinline__ void dq_body(
             }
             // Phase 2: dS = P o (dP - delta) over dP.
             lap(2);
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bDPReady), j & 1, abort_flag, 920 + g, tp.status));
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(P::bDPReady + (j & 1)), (j >> 1) & 1, abort_flag, 920 + g, tp.status));
+            const uint32_t tmem_dp = tmem_dp_of(j);
             if (!ok) break;
             tc_fence_after();
             lap(3);
@@ -932,7 +942,7 @@ __device__ __forceinline__ void dq_body(
             }
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive_warp(bar(P::bPFull + g));
+            mbar_arrive_warp(bar(P::bDSFull + 2 * (j & 1) + g));
             lap(4);
         }
         if (timing) {
@@ -981,6 +991,68 @@ __device__ __forceinline__ void dq_body(
         }
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
+    }
+}
+
+// ---- row terms ----------------------------------------------------------------------------
+
+// The first kernel of the backward: per query row -lse in base 2 and delta = sum_d dO O (see
+// AttnParams::row_terms), one row per D / 8 lanes with 16-byte loads. Large problems give a thread
+// four rows, so that eight loads are in flight (one row each: 4.3 TB/s on a packed 65,536-token
+// batch); where that leaves SMs without a CTA it has one. Bound by reading dO and O once. It also clears the tickets of the dK/dV CTAs that share a key block and the
+// gradient rows that no packed sequence covers.
+template <int D, int kPer, bool kPacked>
+__global__ void __launch_bounds__(256, kPer == 1 && !kPacked ? 8 : 4) bwd_rows_kernel(const AttnParams p, int64_t ncounters) {
+    // The backward kernel behind this one may start its set-up and input loads now; it waits
+    // (griddepcontrol.wait) for this kernel to finish before it reads the row terms or the tickets.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    constexpr int kLanes = D / 8, kRows = 256 / kLanes;   // rows per pass of the CTA, kPer passes
+    const int b = blockIdx.z, h = blockIdx.y;
+    if (kPacked || ncounters) {
+        const int64_t cta = (static_cast<int64_t>(b) * gridDim.y + h) * gridDim.x + blockIdx.x;
+        const int64_t thread = cta * 256 + threadIdx.x, threads = static_cast<int64_t>(gridDim.x) * gridDim.y * gridDim.z * 256;
+        for (int64_t i = thread; i < ncounters; i += threads) p.dkv_counters[i] = 0;
+        if (kPacked) zero_uncovered_rows(p, thread, threads);
+    }
+    const SeqInfo si = seq_info(p, b);
+    const int row0 = blockIdx.x * (kRows * kPer) + threadIdx.x / kLanes;
+    if (static_cast<int>(blockIdx.x) * (kRows * kPer) >= (si.lq + 127) / 128 * 128) return;
+    const int c = (threadIdx.x % kLanes) * 8;
+    const __nv_bfloat16* og = p.out + b * p.os[0] + h * p.os[1] + static_cast<int64_t>(si.q_off) * p.os[2] + c;
+    const __nv_bfloat16* dg = p.dout + b * p.dos[0] + h * p.dos[1] + static_cast<int64_t>(si.q_off) * p.dos[2] + c;
+    const float* lg = p.lse + b * p.ls[0] + h * p.ls[1] + static_cast<int64_t>(si.q_off) * p.ls[2];
+    uint4 o[kPer], d[kPer];
+    float lse[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int row = row0 + u * kRows;
+        o[u] = d[u] = make_uint4(0u, 0u, 0u, 0u);
+        lse[u] = -INFINITY;
+        if (row < si.lq) {
+            o[u] = __ldg(reinterpret_cast<const uint4*>(og + row * p.os[2]));
+            d[u] = __ldg(reinterpret_cast<const uint4*>(dg + row * p.dos[2]));
+            if (c == 0) lse[u] = __ldg(lg + row * p.ls[2]);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&o[u]);
+        const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&d[u]);
+        float acc = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 x = __bfloat1622float2(o2[e]), y = __bfloat1622float2(d2[e]);
+            acc = fmaf(x.x, y.x, acc);
+            acc = fmaf(x.y, y.y, acc);
+        }
+#pragma unroll
+        for (int off = kLanes / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        const int row = row0 + u * kRows;
+        if (c == 0 && row < (si.lq + 127) / 128 * 128) {
+            float* t = p.row_terms + (first_row_block(p, si, b, h) + (row >> 7)) * 256 + (row & 127);
+            t[0] = lse[u] == -INFINITY ? -INFINITY : -lse[u] * kLog2e;
+            t[128] = acc;
+        }
     }
 }
 
@@ -1141,8 +1213,20 @@ int64_t backward_partial_bytes(const AttnParams& p, int gsplit) {
     return backward_counter_offset(p, gsplit) + (backward_counter_count(p, gsplit) * 4 + 255) / 256 * 256;
 }
 
+template <int D>
+int launch_bwd_rows(const AttnParams& p, cudaStream_t stream) {
+    const int64_t ncounters = p.dkv_counters ? backward_counter_count(p, p.gsplit) : 0;
+    const int padded = (p.sq + 127) / 128 * 128, rows = 256 / (D / 8);
+    const int64_t ctas = static_cast<int64_t>(padded / rows) * p.heads * p.batch;
+    const int per = ctas >= 4 * 8 * 148 ? 4 : 1;   // eight CTAs of 256 threads fit an SM
+    auto kernel = p.cu_q ? (per == 4 ? bwd_rows_kernel<D, 4, true> : bwd_rows_kernel<D, 1, true>)
+                         : (per == 4 ? bwd_rows_kernel<D, 4, false> : bwd_rows_kernel<D, 1, false>);
+    kernel<<<dim3(padded / (per * rows), p.heads, p.batch), 256, 0, stream>>>(p, ncounters);
+    return check_cuda(cudaGetLastError(), "bwd_rows launch");
+}
+
 int launch_backward_tc5(const AttnParams& p, cudaStream_t stream) {
-    if (int rc = launch_backward_delta(p, stream)) return rc;
+    if (int rc = p.d == 64 ? launch_bwd_rows<64>(p, stream) : launch_bwd_rows<128>(p, stream)) return rc;
     if (p.d == 64) return launch_bwd<64>(p, stream);
     return launch_bwd<128>(p, stream);
 }

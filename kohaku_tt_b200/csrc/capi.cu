@@ -118,6 +118,13 @@ void delta_layout(const ktt_b200_attn_args* a, int64_t& bs, int64_t& hs, int64_t
     }
 }
 
+// Bytes of it, or of the row terms that stand there in the tcgen05 backward.
+int64_t row_term_bytes(const ktt_b200_attn_args* a, int64_t total) {
+    const int64_t blocks = row_blocks(a->cu_seqlens_q != nullptr, a->total_q, a->batch, a->sq) * a->heads;
+    const int64_t need = total * 4 > blocks * 1024 ? total * 4 : blocks * 1024;
+    return (need + 255) / 256 * 256;
+}
+
 __global__ void merge_partials_kernel(
     void* out, float* lse, const void* out2, const float* lse2, int64_t rows, int dv, int f32, int vec) {
     const int64_t row = blockIdx.x * static_cast<int64_t>(blockDim.y) + threadIdx.y;
@@ -358,31 +365,11 @@ extern "C" int64_t ktt_b200_sdpa_backward_workspace(const ktt_b200_attn_args* a)
     delta_layout(a, bs, hs, total);
     AttnParams p;
     to_params(a, p);
-    return (total * 4 + 255) / 256 * 256 + backward_partial_bytes(p, backward_group_split(p));
+    return row_term_bytes(a, total) + backward_partial_bytes(p, backward_group_split(p));
 }
 
-// Packed calls: rows of dq, dk and dv that no sequence of the offsets covers (before the
-// first offset, after the last) get zeros here; every row inside a sequence is written by the
-// CTA that owns it, so callers need not clear the gradients first.
 __global__ void zero_uncovered_rows_kernel(const AttnParams p) {
-    const int64_t q_lo = p.cu_q[0], q_hi = p.cu_q[p.batch], k_lo = p.cu_k[0], k_hi = p.cu_k[p.batch];
-    const int64_t q_rows = q_lo + (p.total_q - q_hi), k_rows = k_lo + (p.total_k - k_hi);
-    if (q_rows <= 0 && k_rows <= 0) return;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x, t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const __nv_bfloat16 zero = __float2bfloat16(0.f);
-    auto clear = [&](__nv_bfloat16* base, const int64_t (&st)[3], int heads, int d, int64_t lo, int64_t hi, int64_t total) {
-        const int64_t rows = lo + (total - hi);
-        for (int64_t i = t0; i < rows * heads * d; i += stride) {
-            const int e = static_cast<int>(i % d);
-            const int h = static_cast<int>((i / d) % heads);
-            const int64_t r = i / (static_cast<int64_t>(d) * heads);
-            const int64_t row = r < lo ? r : hi + (r - lo);
-            base[h * st[1] + row * st[2] + e] = zero;
-        }
-    };
-    clear(p.dq, p.dqs, p.heads, p.d, q_lo, q_hi, p.total_q);
-    clear(p.dk, p.dks, p.kv_heads, p.d, k_lo, k_hi, p.total_k);
-    clear(p.dv_out, p.dvs, p.kv_heads, p.dv, k_lo, k_hi, p.total_k);
+    zero_uncovered_rows(p, static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x, static_cast<int64_t>(gridDim.x) * blockDim.x);
 }
 
 extern "C" int ktt_b200_sdpa_backward(const ktt_b200_attn_args* a, void* stream) {
@@ -397,14 +384,14 @@ extern "C" int ktt_b200_sdpa_backward(const ktt_b200_attn_args* a, void* stream)
     delta_layout(a, bs, hs, total);
     AttnParams p;
     to_params(a, p);
-    const int64_t delta_bytes = (total * 4 + 255) / 256 * 256;
+    const int64_t delta_bytes = row_term_bytes(a, total);
     p.gsplit = backward_group_split(p);
     const int64_t need = delta_bytes + backward_partial_bytes(p, p.gsplit);
     if (!a->workspace || a->workspace_bytes < need) {
         return fail(KTT_B200_ERR_BAD_ARGUMENT, "sdpa_backward: workspace holds %lld bytes, %lld needed",
                     static_cast<long long>(a->workspace_bytes), static_cast<long long>(need));
     }
-    p.delta = static_cast<float*>(a->workspace);
+    p.delta = p.row_terms = static_cast<float*>(a->workspace);
     p.delta_bs = bs;
     p.delta_hs = hs;
     p.dkv_partial = reinterpret_cast<float*>(static_cast<unsigned char*>(a->workspace) + delta_bytes);
@@ -412,10 +399,6 @@ extern "C" int ktt_b200_sdpa_backward(const ktt_b200_attn_args* a, void* stream)
         ? reinterpret_cast<int32_t*>(static_cast<unsigned char*>(a->workspace) + delta_bytes + backward_counter_offset(p, p.gsplit))
         : nullptr;
     note_call(2);
-    if (p.cu_q) {
-        zero_uncovered_rows_kernel<<<64, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
-        if (int rc = check_cuda(cudaGetLastError(), "zero_uncovered_rows launch")) return rc;
-    }
     const char* why = nullptr;
     const bool tc5 = backward_tc5_takes(p, &why);
     if (a->kernel == KTT_B200_KERNEL_TC5 && !tc5) {
@@ -425,6 +408,10 @@ extern "C" int ktt_b200_sdpa_backward(const ktt_b200_attn_args* a, void* stream)
     if (tc5 && a->kernel != KTT_B200_KERNEL_MMA) {
         note_call(6);
         return launch_backward_tc5(p, static_cast<cudaStream_t>(stream));
+    }
+    if (p.cu_q) {   // (the first kernel of the tcgen05 backward does this itself)
+        zero_uncovered_rows_kernel<<<64, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+        if (int rc = check_cuda(cudaGetLastError(), "zero_uncovered_rows launch")) return rc;
     }
     return launch_backward_mma(p, static_cast<cudaStream_t>(stream));
 }

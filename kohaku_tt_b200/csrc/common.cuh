@@ -41,6 +41,9 @@ struct AttnParams {
     int64_t dos[3], dqs[3], dks[3], dvs[3];
     float* delta;  // [batch, heads, sq_pad] (packed: [heads, total_q_pad])
     int64_t delta_bs, delta_hs;
+    // tcgen05 backward, in place of delta: per 128-row query block of a (batch, head), 128 values of
+    // -lse in base 2 and then 128 of delta, rows past the sequence -inf and 0 (row_block below).
+    float* row_terms;
     // tcgen05 backward with grouped heads: the query heads of a group are split over
     // `gsplit` CTAs per key block, which leave fp32 partial dV / dK here for a reduction.
     int gsplit;
@@ -81,6 +84,17 @@ __device__ __forceinline__ SeqInfo seq_info(const AttnParams& p, int b) {
     return s;
 }
 
+// Query blocks (of 128 rows) per head that row_terms has room for, and the first of a batch
+// entry's. Packed: sequence b starts at block cu_q[b] / 128 + b, which leaves every sequence the
+// blocks its length needs.
+__host__ __device__ inline int64_t row_blocks(int packed, int64_t total_q, int batch, int sq) {
+    return packed ? total_q / 128 + batch : static_cast<int64_t>(batch) * ((sq + 127) / 128);
+}
+__device__ __forceinline__ int64_t first_row_block(const AttnParams& p, const SeqInfo& si, int b, int h) {
+    const int64_t per_head = row_blocks(p.cu_q != nullptr, p.total_q, p.batch, p.sq);
+    return h * per_head + (p.cu_q ? (si.q_off >> 7) + b : b * static_cast<int64_t>((p.sq + 127) >> 7));
+}
+
 // Additive mask value (already clamped) for (b, h, query i, key j); j is the packed key
 // index for packed calls.
 __device__ __forceinline__ float mask_value(
@@ -102,6 +116,29 @@ __device__ __forceinline__ float mask_value(
     }
     // NaN-safe clamp: -inf and anything below the floor become the masked logit.
     return m > kMaskedLogit ? m : kMaskedLogit;
+}
+
+// Packed backward: rows of dq, dk and dv that no sequence of the offsets covers (before the first
+// offset, after the last) get zeros here; every row inside a sequence is written by the CTA that
+// owns it, so callers need not clear the gradients first. `thread` of `threads`.
+__device__ __forceinline__ void zero_uncovered_rows(const AttnParams& p, int64_t thread, int64_t threads) {
+    const int64_t q_lo = p.cu_q[0], q_hi = p.cu_q[p.batch], k_lo = p.cu_k[0], k_hi = p.cu_k[p.batch];
+    const int64_t q_rows = q_lo + (p.total_q - q_hi), k_rows = k_lo + (p.total_k - k_hi);
+    if (q_rows <= 0 && k_rows <= 0) return;
+    const __nv_bfloat16 zero = __float2bfloat16(0.f);
+    auto clear = [&](__nv_bfloat16* base, const int64_t (&st)[3], int heads, int d, int64_t lo, int64_t hi, int64_t total) {
+        const int64_t rows = lo + (total - hi);
+        for (int64_t i = thread; i < rows * heads * d; i += threads) {
+            const int e = static_cast<int>(i % d);
+            const int h = static_cast<int>((i / d) % heads);
+            const int64_t r = i / (static_cast<int64_t>(d) * heads);
+            const int64_t row = r < lo ? r : hi + (r - lo);
+            base[h * st[1] + row * st[2] + e] = zero;
+        }
+    };
+    clear(p.dq, p.dqs, p.heads, p.d, q_lo, q_hi, p.total_q);
+    clear(p.dk, p.dks, p.kv_heads, p.d, k_lo, k_hi, p.total_k);
+    clear(p.dv_out, p.dvs, p.kv_heads, p.dv, k_lo, k_hi, p.total_k);
 }
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -185,7 +222,6 @@ int ensure_smem(K kernel, int bytes, const char* what) {
 // Launchers (one per kernel family).
 int launch_forward_mma(const AttnParams& p, cudaStream_t stream);
 int launch_backward_mma(const AttnParams& p, cudaStream_t stream);
-int launch_backward_delta(const AttnParams& p, cudaStream_t stream);  // delta = rowsum(dO o O)
 int launch_backward_tc5(const AttnParams& p, cudaStream_t stream);
 bool backward_tc5_takes(const AttnParams& p, const char** why);
 // Number of CTAs the query heads of a GQA group are split over in the tcgen05 dK/dV kernel

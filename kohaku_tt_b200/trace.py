@@ -126,7 +126,7 @@ def backward(dev):
                   f"results stored {med[3]:.0f} | ticket, sum of the parts, teardown {med[4]:.0f}")
     del group
     # Where the item loop of a dK/dV CTA spends its clocks, per score warp (first 56 CTAs).
-    names = ["meeting + next fetch", "wait for S", "phase 1 (P)", "wait for dP", "phase 2 (dS)"]
+    names = ["row terms", "wait for S", "phase 1 (P)", "wait for dP", "phase 2 (dS)"]
     per_warp = []
     for w in range(8):
         rws = torch.stack([table[64 + 512 + c * 8 + w] for c in range(56)])
