@@ -16,7 +16,7 @@
 //
 // These calls ran on the warp-MMA kernel before (mma.sync, 64-row CTAs). Measured on B200: 16 x
 // 16 heads x 257 rows, D 80: 220 -> 55 us; 2 x 16 heads x 2048, D 64, a causal mask with padding
-// as a bf16 tensor: 577 -> 104 us, of which the plan of the mask is 5.
+// as a bf16 tensor: 577 -> 75 us.
 //
 // Tensor memory (512 columns): S_A, S_B (128 each); head dims up to 64: P_A, P_B (64 each) and
 // O_A, O_B (64 each), so that the next scores can be computed while P V still reads P; up to 128:
@@ -971,103 +971,104 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
 
 // ---- masks with a row per query ----------------------------------------------------------
 //
-// One CTA per 32 query rows of a plane walks the keys once: eight warps of four rows each, four
-// blocks of 128 keys at a time (sixteen loads in flight per lane: with one block at a time the
-// walk was a chain of trips to memory). It is bound by reading the mask once; pieces without
-// values to apply cost nothing further, and what the attention kernel reads back is the bits or
-// values of the pieces that have any.
+// One CTA per 32 query rows of a plane walks the keys once, a warp per row, four blocks of 128
+// keys at a time. It is bound by reading the mask once; pieces without values to apply cost
+// nothing further, and what the attention kernel reads back is the bits or values of the pieces
+// that have any. The code is kept small (a type per instance, one row per warp): with four rows
+// per warp and the type looked up per load it was 85 to 106 KB of straight-line instructions that
+// every pass fetched again. A call with 2 x 2048 x 2048 bf16 terms (2 x 16 heads, D 64): 103 -> 75 us.
 //
 // A block is hidden from a group when every term of it is at the floor (-5e5): its weights are
 // exactly 0 as long as each row of the group keeps a key well above the floor. A group with a
 // row that does not (a row that sees nothing) has none of its blocks left out.
 constexpr float kSafeTerm = 0.5f * kMaskedLogit;
-constexpr int kPlanUnroll = 4;
+constexpr int kPlanUnroll = 4, kPlanThreads = 1024;
 
-__device__ __forceinline__ float mask_raw(const AttnParams& p, int64_t idx) {
-    switch (p.mask_dtype) {
-        case KTT_B200_MASK_BOOL: return reinterpret_cast<const uint8_t*>(p.mask)[idx] ? 0.f : kMaskedLogit;
-        case KTT_B200_MASK_BF16: return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.mask)[idx]);
-        case KTT_B200_MASK_F16: return __half2float(reinterpret_cast<const __half*>(p.mask)[idx]);
-        default: return reinterpret_cast<const float*>(p.mask)[idx];
+// The term at `idx`.
+template <int kType>
+__device__ __forceinline__ float mask_term(const void* mask, int64_t idx) {
+    if constexpr (kType == KTT_B200_MASK_BOOL) return __ldg(static_cast<const uint8_t*>(mask) + idx) ? 0.f : kMaskedLogit;
+    if constexpr (kType == KTT_B200_MASK_BF16) return __uint_as_float(static_cast<uint32_t>(__ldg(static_cast<const uint16_t*>(mask) + idx)) << 16);
+    if constexpr (kType == KTT_B200_MASK_F16) return __half2float(__ldg(static_cast<const __half*>(mask) + idx));
+    return __ldg(static_cast<const float*>(mask) + idx);
+}
+// The four terms from `idx`, in one load.
+template <int kType>
+__device__ __forceinline__ void mask_terms(const void* mask, int64_t idx, float (&v)[4]) {
+    if constexpr (kType == KTT_B200_MASK_BOOL) {
+        const uint32_t x = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(mask) + idx));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = (x >> (8 * e)) & 0xffu ? 0.f : kMaskedLogit;
+    } else if constexpr (kType == KTT_B200_MASK_F32) {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(mask) + idx));
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else {
+        const uint2 x = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(mask) + idx));
+        if constexpr (kType == KTT_B200_MASK_BF16) {
+            v[0] = __uint_as_float(x.x << 16); v[1] = __uint_as_float(x.x & 0xffff0000u);
+            v[2] = __uint_as_float(x.y << 16); v[3] = __uint_as_float(x.y & 0xffff0000u);
+        } else {
+            const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&x.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&x.y));
+            v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+        }
     }
 }
 
-// kVec: the keys are contiguous and every row of the mask starts on an 8-byte (16-bit types),
-// 4-byte (bool) or 16-byte (fp32) boundary, so that a lane reads its four keys in one load.
-template <bool kVec>
-__global__ void __launch_bounds__(256) mask_plan_kernel(const AttnParams p, const MaskPlan m, int32_t* header) {
+// `vec`: the keys are contiguous and every row of the mask starts on a multiple of four terms, so
+// that a lane reads its four keys in one load.
+template <int kType>
+__global__ void __launch_bounds__(kPlanThreads) mask_plan_kernel(const AttnParams p, const MaskPlan m, int32_t* header, const bool vec) {
     __shared__ uint32_t seen[kMaxPlanBlocks];   // per block: 1 floor, 2 zero, 4 anything else
     __shared__ int unsafe;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int g = blockIdx.x, plane = blockIdx.y;
     const int pb = plane / m.heads, ph = plane - pb * m.heads;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < m.blocks; i += 256) seen[i] = 0;
+    const int rr = threadIdx.x >> 5, lane = threadIdx.x & 31;   // row of the group, position in the row
+    for (int i = threadIdx.x; i < m.blocks; i += kPlanThreads) seen[i] = 0;
     if (threadIdx.x == 0) unsafe = 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // The attention kernel's work counters: this launch comes first in the stream.
     if (g == 0 && plane == 0 && threadIdx.x < 2) header[threadIdx.x] = 0;
     __syncthreads();
     const int64_t piece0 = (static_cast<int64_t>(plane) * m.groups + g) * m.blocks;
-    float best[4];   // per row: the largest term so far
-#pragma unroll
-    for (int r = 0; r < 4; ++r) best[r] = -INFINITY;
+    const int row = g * 32 + rr;
+    const bool real = row < p.sq;
+    const int64_t at = pb * p.ms[0] + ph * p.ms[1] + static_cast<int64_t>(min(row, p.sq - 1)) * p.ms[2];
+    float best = -INFINITY;   // the row's largest term so far
+#pragma unroll 1
     for (int b0 = 0; b0 < m.blocks; b0 += kPlanUnroll) {
-        float v[kPlanUnroll][4][4];
-        uint32_t flags[kPlanUnroll];
+        float v[kPlanUnroll][4];
 #pragma unroll
         for (int u = 0; u < kPlanUnroll; ++u) {
+            const int col = (b0 + u) * 128 + lane * 4;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int row = g * 32 + warp * 4 + r, col = (b0 + u) * 128 + lane * 4;
-                const int64_t at = pb * p.ms[0] + ph * p.ms[1] + static_cast<int64_t>(min(row, p.sq - 1)) * p.ms[2];
+            for (int e = 0; e < 4; ++e) v[u][e] = kMaskedLogit;
+            if (vec && col + 3 < p.sk) mask_terms<kType>(p.mask, at + col, v[u]);
+        }
+        if (!vec || (b0 + kPlanUnroll) * 128 > p.sk) {   // terms apart, and the last ones of a row
 #pragma unroll
-                for (int e = 0; e < 4; ++e) v[u][r][e] = kMaskedLogit;
-                if (kVec && col + 3 < p.sk) {
-                    const int64_t idx = at + col;
-                    if (p.mask_dtype == KTT_B200_MASK_F32) {
-                        const float4 x = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(p.mask) + idx));
-                        v[u][r][0] = x.x; v[u][r][1] = x.y; v[u][r][2] = x.z; v[u][r][3] = x.w;
-                    } else if (p.mask_dtype == KTT_B200_MASK_BOOL) {
-                        const uint32_t x = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(p.mask) + idx));
+            for (int u = 0; u < kPlanUnroll; ++u) {
+                const int col = (b0 + u) * 128 + lane * 4;
+                if (vec && col + 3 < p.sk) continue;
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) v[u][r][e] = (x >> (8 * e)) & 0xffu ? 0.f : kMaskedLogit;
-                    } else {
-                        const uint2 x = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.mask) + idx));
-                        if (p.mask_dtype == KTT_B200_MASK_BF16) {
-                            v[u][r][0] = __uint_as_float(x.x << 16); v[u][r][1] = __uint_as_float(x.x & 0xffff0000u);
-                            v[u][r][2] = __uint_as_float(x.y << 16); v[u][r][3] = __uint_as_float(x.y & 0xffff0000u);
-                        } else {
-                            const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&x.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&x.y));
-                            v[u][r][0] = lo.x; v[u][r][1] = lo.y; v[u][r][2] = hi.x; v[u][r][3] = hi.y;
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        if (col + e < p.sk) v[u][r][e] = mask_raw(p, at + (col + e) * p.ms[3]);
-                    }
+                for (int e = 0; e < 4; ++e) {
+                    if (col + e < p.sk) v[u][e] = mask_term<kType>(p.mask, at + (col + e) * p.ms[3]);
                 }
             }
         }
 #pragma unroll
         for (int u = 0; u < kPlanUnroll; ++u) {
-            flags[u] = 0;
+            uint32_t flags = 0;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                if (g * 32 + warp * 4 + r < p.sq) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        // Columns past the last key count as hidden; they decide nothing.
-                        const bool floor_ = !(v[u][r][e] > kMaskedLogit);
-                        const bool inside = (b0 + u) * 128 + lane * 4 + e < p.sk;
-                        if (inside) flags[u] |= floor_ ? 1u : v[u][r][e] == 0.f ? 2u : 4u;
-                        if (inside && !floor_) best[r] = fmaxf(best[r], v[u][r][e]);
-                    }
-                }
+            for (int e = 0; e < 4; ++e) {
+                // Columns past the last key count as hidden; they decide nothing.
+                const float x = v[u][e];
+                const uint32_t f = !(x > kMaskedLogit) ? 1u : x == 0.f ? 2u : 4u;
+                if ((b0 + u) * 128 + lane * 4 + e < p.sk) flags |= f;
+                if (f != 1u) best = fmaxf(best, x);
             }
-            flags[u] = __reduce_or_sync(0xffffffffu, flags[u]);
-            if (lane == 0 && b0 + u < m.blocks && flags[u]) atomicOr(&seen[b0 + u], flags[u]);
+            flags = __reduce_or_sync(0xffffffffu, flags);
+            if (lane == 0 && b0 + u < m.blocks && real) atomicOr(&seen[b0 + u], flags);
         }
         __syncthreads();
 #pragma unroll
@@ -1076,51 +1077,38 @@ __global__ void __launch_bounds__(256) mask_plan_kernel(const AttnParams p, cons
             const uint32_t f = seen[b0 + u];
             const int64_t piece = piece0 + b0 + u;
             if (f & 4u) {
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int rr = warp * 4 + r;
-                    if (m.wide) {
-                        reinterpret_cast<float4*>(m.values)[(piece * 32 + lane) * 32 + rr] = make_float4(v[u][r][0], v[u][r][1], v[u][r][2], v[u][r][3]);
-                    } else {
-                        // bf16 in, bf16 out: the upper halves, two lanes to a 16-byte chunk
-                        uint2 w;
-                        w.x = __byte_perm(__float_as_uint(v[u][r][0]), __float_as_uint(v[u][r][1]), 0x7632);
-                        w.y = __byte_perm(__float_as_uint(v[u][r][2]), __float_as_uint(v[u][r][3]), 0x7632);
-                        reinterpret_cast<uint2*>(m.values + (piece * 16 + (lane >> 1)) * 32 + rr)[lane & 1] = w;
-                    }
+                if (m.wide) {
+                    reinterpret_cast<float4*>(m.values)[(piece * 32 + lane) * 32 + rr] = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+                } else {
+                    // bf16 in, bf16 out: the upper halves, two lanes to a 16-byte chunk
+                    uint2 w;
+                    w.x = __byte_perm(__float_as_uint(v[u][0]), __float_as_uint(v[u][1]), 0x7632);
+                    w.y = __byte_perm(__float_as_uint(v[u][2]), __float_as_uint(v[u][3]), 0x7632);
+                    reinterpret_cast<uint2*>(m.values + (piece * 16 + (lane >> 1)) * 32 + rr)[lane & 1] = w;
                 }
             } else if (f == 3u) {
+                // Four bits per lane; eight lanes make a word, four words a row.
+                uint32_t x = 0;
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    // Four bits per lane; eight lanes make a word, four words a row.
-                    uint32_t x = 0;
+                for (int e = 0; e < 4; ++e) x |= (v[u][e] > kMaskedLogit ? 1u : 0u) << (4 * (lane & 7) + e);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) x |= (v[u][r][e] > kMaskedLogit ? 1u : 0u) << (4 * (lane & 7) + e);
-#pragma unroll
-                    for (int o = 1; o < 8; o <<= 1) x |= __shfl_xor_sync(0xffffffffu, x, o);
-                    if ((lane & 7) == 0) reinterpret_cast<uint32_t*>(m.bits + piece * 32 + warp * 4 + r)[lane >> 3] = x;
-                }
+                for (int o = 1; o < 8; o <<= 1) x |= __shfl_xor_sync(0xffffffffu, x, o);
+                if ((lane & 7) == 0) reinterpret_cast<uint32_t*>(m.bits + piece * 32 + rr)[lane >> 3] = x;
             }
         }
     }
-    bool bad = false;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        float x = best[r];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
-        bad = bad || (g * 32 + warp * 4 + r < p.sq && !(x > kSafeTerm));
-    }
-    if (bad && lane == 0) unsafe = 1;
+    for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (lane == 0 && real && !(best > kSafeTerm)) unsafe = 1;
     __syncthreads();
-    for (int i = threadIdx.x; i < m.blocks; i += 256) {
+    for (int i = threadIdx.x; i < m.blocks; i += kPlanThreads) {
         const uint32_t f = seen[i];
         m.kind[piece0 + i] = (f & 4u) ? kValues : f == 3u ? kYesNo : f == 2u ? kNoEffect : unsafe ? kAllFloor : kHidden;
     }
-    for (int w = threadIdx.x; w < m.words; w += 256) {
-        uint32_t bits = 0;
-        for (int i = 0; i < 32 && w * 32 + i < m.blocks; ++i) bits |= (unsafe || seen[w * 32 + i] != 1u ? 1u : 0u) << i;
-        m.active[(static_cast<int64_t>(plane) * m.groups + g) * m.words + w] = bits;
+    if (rr < m.words) {   // (at most 1,024 blocks: 32 words, a warp each)
+        const int i = rr * 32 + lane;
+        const uint32_t bits = __ballot_sync(0xffffffffu, i < m.blocks && (unsafe || seen[i] != 1u));
+        if (lane == 0) m.active[(static_cast<int64_t>(plane) * m.groups + g) * m.words + rr] = bits;
     }
 }
 
@@ -1258,8 +1246,10 @@ int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_
         const int64_t planes = static_cast<int64_t>(m.heads) * (m.batched ? p.batch : 1);
         const int size = p.mask_dtype == KTT_B200_MASK_BOOL ? 1 : p.mask_dtype == KTT_B200_MASK_F32 ? 4 : 2;
         const bool vec = p.ms[3] == 1 && (reinterpret_cast<uintptr_t>(p.mask) % (4 * size)) == 0 && p.ms[0] % 4 == 0 && p.ms[1] % 4 == 0 && p.ms[2] % 4 == 0;
-        if (int rc = launch_dependent(vec ? mask_plan_kernel<true> : mask_plan_kernel<false>, dim3(m.groups, static_cast<unsigned>(planes)), 256, 0, stream,
-                                      "mask_plan launch", p, tp.plan, static_cast<int32_t*>(workspace))) return rc;
+        auto plan = p.mask_dtype == KTT_B200_MASK_BOOL ? mask_plan_kernel<KTT_B200_MASK_BOOL> : p.mask_dtype == KTT_B200_MASK_BF16 ? mask_plan_kernel<KTT_B200_MASK_BF16>
+                  : p.mask_dtype == KTT_B200_MASK_F16  ? mask_plan_kernel<KTT_B200_MASK_F16>  : mask_plan_kernel<KTT_B200_MASK_F32>;
+        if (int rc = launch_dependent(plan, dim3(m.groups, static_cast<unsigned>(planes)), kPlanThreads, 0, stream, "mask_plan launch", p, tp.plan,
+                                      static_cast<int32_t*>(workspace), vec)) return rc;
     }
     // K / V beyond what L2 keeps (126 MB on B200): the grouped order, which needs the counter.
     const int64_t kv_bytes = (p.cu_q ? p.total_k : static_cast<int64_t>(p.batch) * p.sk) * p.kv_heads * (p.d + p.dv) * 2;
