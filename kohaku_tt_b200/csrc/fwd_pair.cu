@@ -12,11 +12,18 @@
 //                      No two threads ever exchange anything inside the loop.
 //   warps 8, 9         issue S = Q K^T and O += P V (P read from tensor memory) of A and of B: while
 //                      one tile is in its exponentials the tensor core serves the other
-//   warp 10            TMA loads of Q and of a ring of K and V tiles, and the draw of the work
+//   warp 10            draws the work and hands the items round, TMA loads of Q and of a ring of K
+//                      and V tiles
+//
+// An item of few blocks runs every role's code once or twice, so the code itself is what such
+// calls are bound by: a third of the instruction fetches miss the cache. Hence one copy of the item
+// arithmetic (the producer's), short waits, and loops where a block is not the common one: 94 to
+// 150 KB of instructions became 79 to 105 (16 x 16 heads x 257 rows, D 80: 49 -> 42 us; 2 x 16
+// heads x 2048 x 2048, D 128, a mask of random values: 343 -> 278 us).
 //
 // These calls ran on the warp-MMA kernel before (mma.sync, 64-row CTAs). Measured on B200: 16 x
-// 16 heads x 257 rows, D 80: 220 -> 55 us; 2 x 16 heads x 2048, D 64, a causal mask with padding
-// as a bf16 tensor: 577 -> 75 us.
+// 16 heads x 257 rows, D 80: 220 -> 42 us; 2 x 16 heads x 2048, D 64, a causal mask with padding
+// as a bf16 tensor: 577 -> 71 us.
 //
 // Tensor memory (512 columns): S_A, S_B (128 each); head dims up to 64: P_A, P_B (64 each) and
 // O_A, O_B (64 each), so that the next scores can be computed while P V still reads P; up to 128:
@@ -72,7 +79,9 @@ struct PairPlan {
     static constexpr int kMaskRow = kRing + kSlots * kOperand;   // float [tile][parity][128]: a block's mask terms
     static constexpr int kBars = kMaskRow + 2 * 2 * 128 * 4;
     static constexpr int kBarBytes = 512;
-    static constexpr int kBytes = kBars + kBarBytes;
+    static constexpr int kQueue = 4;
+    static constexpr int kItems = kBars + kBarBytes;  // Item [kQueue]: what the producer hands to the other roles
+    static constexpr int kBytes = kItems + kQueue * 96;
     static_assert(kBytes <= 232448, "shared memory per CTA");
     // dual: float2 [128] of B's (m, l); Q_B is idle then
     static constexpr int kPartial = kQ + kOperand;
@@ -92,11 +101,11 @@ struct PairPlan {
     static constexpr int bPFull = 8;                   // + 2 t + half of the keys (64 each; one phase for all where P has columns of its own)
     static constexpr int bPVDone = 12;                 // + t
     static constexpr int bOFree = 14;                  // + t
-    static constexpr int bWorkFull = 16;               // + slot
-    static constexpr int bWorkFree = 18;               // + slot
-    static constexpr int bMask = 20;                   // + t: the block's mask terms are written
-    static constexpr int bPartial = 22;                // dual: B's half is final
-    static constexpr int bKVFull = 23;                 // + ring slot
+    static constexpr int bWorkFull = 16;               // + queue slot
+    static constexpr int bWorkFree = bWorkFull + kQueue;   // + queue slot
+    static constexpr int bMask = bWorkFree + kQueue;   // + t: the block's mask terms are written
+    static constexpr int bPartial = bMask + 2;         // dual: B's half is final
+    static constexpr int bKVFull = bPartial + 1;       // + ring slot
     static constexpr int bKVEmpty = bKVFull + kSlots;  // + ring slot
     static constexpr int bCount = bKVEmpty + kSlots;
     static_assert(bCount * 8 + 32 <= kBarBytes, "barrier area");
@@ -132,13 +141,14 @@ struct PairParams {
     MaskPlan plan;
 };
 
-struct Item {
-    int b, hk;
+struct alignas(16) Item {
+    int b, hk;                  // b < 0: no more items
     int h[2], q0[2], kend[2];   // per tile; kend: keys any of its rows sees
     int n[2];                   // key blocks per tile (dual: its share); n[0] >= n[1]
-    bool valid[2];
+    int valid[2];
     SeqInfo si;
 };
+static_assert(sizeof(Item) <= 96, "the queue's slots");
 
 // Items of one (batch, K / V head) are neighbours in its list of (query tile, head), longest
 // causal tiles first, heads fastest. Two orders of the items: with the level slowest every deal
@@ -251,6 +261,32 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
+// Bounded waits of a converged warp, for one barrier or two at once (their polls overlap). Kept
+// short: there are two dozen of them in this kernel, and what does not fit the instruction cache
+// is fetched again for every item.
+__device__ __forceinline__ bool wait_both(uint32_t b0, uint32_t par0, uint32_t b1, uint32_t par1, volatile int* abort_flag, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(b0, par0) & mbar_try_wait(b1, par1))) return true;
+    const long long t0 = clock64();
+#pragma unroll 1
+    while (!__all_sync(0xffffffffu, mbar_try_wait(b0, par0) & mbar_try_wait(b1, par1))) {
+        const bool late = clock64() - t0 > kWaitCycles;
+        if (late) *abort_flag = code;   // reported when the CTA ends
+        if (__any_sync(0xffffffffu, late || *abort_flag)) return false;
+    }
+    return true;
+}
+__device__ __forceinline__ bool wait_one(uint32_t b, uint32_t par, volatile int* abort_flag, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(b, par))) return true;
+    const long long t0 = clock64();
+#pragma unroll 1
+    while (!__all_sync(0xffffffffu, mbar_try_wait(b, par))) {
+        const bool late = clock64() - t0 > kWaitCycles;
+        if (late) *abort_flag = code;   // reported when the CTA ends
+        if (__any_sync(0xffffffffu, late || *abort_flag)) return false;
+    }
+    return true;
+}
+
 // ---- the kernel ------------------------------------------------------------------------
 
 // kMask: 0 none, 1 a row per (batch, head), 2 a plan (a row per query).
@@ -271,7 +307,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
     auto bar = [&](int i) { return bars + 8u * i; };
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + P::kBars + P::bCount * 8);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + P::kBars + P::bCount * 8 + 8);
-    volatile int* work_slot = reinterpret_cast<volatile int*>(smem + P::kBars + P::bCount * 8 + 16);   // [2]
+    Item* queue = reinterpret_cast<Item*>(smem + P::kItems);   // [kQueue]
     const AttnParams& p = tp.a;
 
     if (warp == kProducerWarp) {
@@ -280,7 +316,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             // Softmax threads arrive once per warp (mbar_arrive_warp).
             if ((i >= P::bSFree && i < P::bSFree + 2) || (i >= P::bPFull && i < P::bPFull + 4) ||
                 (i >= P::bOFree && i < P::bOFree + 2) || (i >= P::bMask && i < P::bMask + 2) || i == P::bPartial) count = 4;
-            if (i >= P::bWorkFree && i < P::bWorkFree + 2) count = 10;   // the softmax and the MMA warps
+            if (i >= P::bWorkFree && i < P::bWorkFree + P::kQueue) count = 10;   // the softmax and the MMA warps
             // Pair: both tiles release every ring tile. Dual: each has one user, but they share Q.
             if (i >= P::bKVEmpty && !tp.dual) count = 2;
             if (i == P::bQFree && tp.dual) count = 2;
@@ -308,49 +344,18 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
     const uint32_t tmem = *tmem_slot;
     const bool dual = tp.dual != 0;
 
-    // The n-th item of this CTA: -1 = no more, -2 = nothing at this position. Without a counter
-    // every role computes the same snake order by itself; with one, the producer warp draws the
-    // items and hands them to the other roles through a two-slot queue in shared memory.
-    const bool dynamic = tp.work_counter != nullptr;
-    auto static_item = [&](int n) -> int {
-        if (static_cast<int64_t>(n) * gridDim.x >= tp.work) return -1;
-        const int w = snake(n, blockIdx.x, gridDim.x);
-        return w < tp.work ? w : -2;
+    // The producer warp draws the items (from a counter, or the fixed deal of a snake order), works
+    // out what they are and hands them to the other roles through a queue in shared memory: one
+    // role's divisions and one copy of that code. Positions past the end of a short sequence are
+    // left out. A role gives an item back when it no longer reads the queue's copy.
+    auto take_item = [&](int n, Item& k, bool& ok) {   // the other roles
+        const int slot = n % P::kQueue;
+        ok = ok && wait_one(bar(P::bWorkFull + slot), (n / P::kQueue) & 1, abort_flag, 130 + slot);
+        k.b = -1;
+        if (ok) k = queue[slot];
+        return k.b >= 0;
     };
-    auto draw_item = [&](int n, bool& ok) -> int {   // producer warp, converged
-        if (!dynamic) return static_item(n);
-        const int slot = n & 1;
-        if (n >= 2) {
-            ok = __all_sync(0xffffffffu, mbar_wait_inline(bar(P::bWorkFree + slot), ((n >> 1) - 1) & 1, abort_flag, 120 + slot, tp.status));
-            if (!ok) return -1;
-        }
-        int w;
-        while (true) {   // positions past the end of a short sequence are skipped here
-            w = 0;
-            if (lane == 0) w = atomicAdd(tp.work_counter, 1);
-            w = __shfl_sync(0xffffffffu, w, 0);
-            if (w >= tp.work) {
-                w = -1;
-                break;
-            }
-            if (decode_item(tp, w).valid[0]) break;
-        }
-        if (lane == 0) {
-            work_slot[slot] = w;
-            __threadfence_block();
-            mbar_arrive(bar(P::bWorkFull + slot));
-        }
-        return w;
-    };
-    auto take_item = [&](int n, bool& ok) -> int {   // the other roles
-        if (!dynamic) return static_item(n);
-        const int slot = n & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait_inline(bar(P::bWorkFull + slot), (n >> 1) & 1, abort_flag, 130 + slot, tp.status));
-        if (!ok) return -1;
-        const int w = work_slot[slot];
-        mbar_arrive_warp(bar(P::bWorkFree + slot));
-        return w;
-    };
+    auto give_item = [&](int n) { mbar_arrive_warp(bar(P::bWorkFree + n % P::kQueue)); };
     // Tensor-map coordinate of slot `slot` (1..3): row, head and batch sit where the host sorted
     // them by stride.
     auto coord = [&](int operand, int slot, int row, int head, int batch) {
@@ -367,7 +372,21 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
         int slot = 0, lap = 0;      // next ring slot, times round the ring
         bool ok = true;
         auto wait_for = [&](int b, int parity, int code) {
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_inline(bar(b), parity, abort_flag, code, tp.status));
+            ok = ok && wait_one(bar(b), parity, abort_flag, code);
+        };
+        const bool dynamic = tp.work_counter != nullptr;
+        int round = 0;
+        auto draw = [&]() -> int {   // the next position in the list of items; -1 = no more
+            if (!dynamic) {
+                const int64_t first = static_cast<int64_t>(round) * gridDim.x;
+                const int w = first < tp.work ? snake(round, blockIdx.x, gridDim.x) : -1;
+                ++round;
+                return w;
+            }
+            int w = 0;
+            if (lane == 0) w = atomicAdd(tp.work_counter, 1);
+            w = __shfl_sync(0xffffffffu, w, 0);
+            return w < tp.work ? w : -1;
         };
         auto load_q = [&](const Item& k, int t) {
             if (items_of[t] > 0) wait_for(P::bQFree + t, (items_of[t] - 1) & 1, 110 + t);
@@ -394,19 +413,32 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 ++lap;
             }
         };
-        // In the grouped order items are fetched one ahead: the trip to the counter, and the
-        // positions a draw skips, hide behind an item's loads. Otherwise an item is drawn when
-        // its loads start: committing earlier evens the CTAs out less well at the end.
+        // In the grouped order positions are fetched one ahead: the trip to the counter hides behind
+        // an item's loads. Otherwise an item is drawn when its loads start: committing earlier evens
+        // the CTAs out less well at the end.
         const bool ahead = tp.grouped != 0;
-        int w_next = ahead ? draw_item(0, ok) : 0;
-        for (int n = 0; ok; ++n) {
-            const int w = ahead ? w_next : draw_item(n, ok);
-            if (w == -1) break;
-            if (ahead) w_next = draw_item(n + 1, ok);
+        int w_next = ahead ? draw() : 0;
+        for (int n = 0; ok;) {
+            const int w = ahead ? w_next : draw();
+            Item k;
+            k.b = -1;
+            if (w >= 0) {
+                if (ahead) w_next = draw();
+                if (w >= tp.work) continue;   // the fixed deal's last round
+                k = decode_item(tp, w);
+                if (!k.valid[0]) continue;
+                if constexpr (kMask == 2) apply_plan(tp, k);
+            }
+            const int q_slot = n % P::kQueue;
+            if (n >= P::kQueue) wait_for(P::bWorkFree + q_slot, (n / P::kQueue - 1) & 1, 120 + q_slot);
             if (!ok) break;
-            if (w == -2) continue;
-            Item k = decode_item(tp, w);
-            if constexpr (kMask == 2) apply_plan(tp, k);
+            if (lane == 0) {
+                queue[q_slot] = k;
+                mbar_arrive(bar(P::bWorkFull + q_slot));   // release: the item before the arrival
+            }
+            __syncwarp();
+            ++n;
+            if (w < 0) break;
             if (k.n[0] == 0) continue;
             Iter it[2];
             it[0].start(tp, k, 0);
@@ -450,13 +482,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
         int q_items = 0;                    // Q tiles so far
         int base = 0, base_lap = 0;         // ring position of the item's first tile
         bool ok = true;
-        // Waits for two barriers at once (their polls overlap).
         auto wait_two = [&](uint32_t b0, uint32_t par0, uint32_t b1, uint32_t par1, int code) {
-            const bool got = mbar_try_wait(b0, par0) & mbar_try_wait(b1, par1);
-            if (!__all_sync(0xffffffffu, got)) {
-                ok = ok && __all_sync(0xffffffffu, mbar_wait_inline(b0, par0, abort_flag, code, tp.status) && mbar_wait_inline(b1, par1, abort_flag, code + 1, tp.status));
-            }
+            ok = ok && wait_both(b0, par0, b1, par1, abort_flag, code);
         };
+        auto wait_bar = [&](uint32_t b, uint32_t par, int code) { ok = ok && wait_one(b, par, abort_flag, code); };
         auto advance = [](int& slot, int& lap, int by) {
             slot += by;
             if (slot >= P::kSlots) {
@@ -465,11 +494,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             }
         };
         for (int n = 0; ok; ++n) {
-            const int w = take_item(n, ok);
-            if (w == -1) break;
-            if (w == -2) continue;
-            Item k = decode_item(tp, w);
-            if constexpr (kMask == 2) apply_plan(tp, k);
+            Item k;
+            if (!take_item(n, k, ok)) break;
+            give_item(n);
             if (k.n[0] == 0) continue;
             const int nb = t ? k.n[1] : k.n[0], kend = t ? k.kend[1] : k.kend[0], klen = k.si.klen;
             const int entries = dual ? k.n[0] + k.n[1] : k.n[0];
@@ -490,9 +517,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     const int gb = blk + j + 1;     // this tile's score products so far
                     if (j < 0) {
                         wait_two(bar(P::bQFull + q_bar), q_items & 1, bar(P::bKVFull + s_slot), s_lap, 200 + 2 * t);
-                        if (!P::kPOverS && gb > 0) wait_two(bar(P::bSFree + t), (gb - 1) & 1, bar(P::bSFree + t), (gb - 1) & 1, 210);
+                        if (!P::kPOverS && gb > 0) wait_bar(bar(P::bSFree + t), (gb - 1) & 1, 210 + t);
                     } else if (P::kPOverS) {
-                        wait_two(bar(P::bKVFull + s_slot), s_lap, bar(P::bKVFull + s_slot), s_lap, 220 + t);
+                        wait_bar(bar(P::bKVFull + s_slot), s_lap, 220 + t);
                     } else {
                         wait_two(bar(P::bKVFull + s_slot), s_lap, bar(P::bSFree + t), (gb - 1) & 1, 222 + 2 * t);
                     }
@@ -500,6 +527,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     tc_fence_after();
                     const int keys = min(kBN, (kend - s_block * kBN + 15) & ~15);   // in the MMA's steps of 16
                     const uint64_t kd = k_desc + static_cast<uint32_t>(s_slot * (P::kOperand >> 4));
+                    const uint32_t idesc = instr_desc(keys, false);
                     if (d_steps == DP / 16 && keys == kBN) {
 #pragma unroll
                         for (int ks = 0; ks < DP / 16; ++ks) {
@@ -507,7 +535,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                             tc_mma(d_s, q_desc + off, kd + off, instr_desc(kBN, false), ks > 0);
                         }
                     } else {
-                        const uint32_t idesc = instr_desc(keys, false);
 #pragma unroll 1
                         for (int ks = 0; ks < d_steps; ++ks) {
                             const uint32_t off = ((ks / 4) * P::kTile + (ks % 4) * 32) >> 4;
@@ -522,7 +549,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 auto values = [&]() {
                     const int gb = blk + j, keys = min(kBN, (kend - block * kBN + 15) & ~15), seen = klen - block * kBN;
                     wait_two(bar(P::bKVFull + v_slot), v_lap, bar(P::bPFull + 2 * t), gb & 1, 230 + 2 * t);
-                    if (j == 0 && items > 0) wait_two(bar(P::bOFree + t), (items - 1) & 1, bar(P::bOFree + t), (items - 1) & 1, 250 + t);
+                    if (j == 0 && items > 0) wait_bar(bar(P::bOFree + t), (items - 1) & 1, 250 + t);
                     if (!ok) return;
                     if (seen < keys) {
                         // Rows past the sequence's keys may hold anything (a cache past its length, a
@@ -545,26 +572,20 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     const bool whole = keys == kBN && p.dv == DP;
                     if (whole) {
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), instr_desc(DP, true), (j > 0 || ks > 0) ? 1u : 0u);
-                        }
+                        for (int ks = 0; ks < 4; ++ks) tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), instr_desc(DP, true), (j > 0 || ks > 0) ? 1u : 0u);
                     }
                     if constexpr (P::kPOverS) {
-                        wait_two(bar(P::bPFull + 2 * t + 1), gb & 1, bar(P::bPFull + 2 * t + 1), gb & 1, 240 + t);
+                        wait_bar(bar(P::bPFull + 2 * t + 1), gb & 1, 240 + t);
                         if (!ok) return;
                         tc_fence_after();
                     }
                     if (whole) {
 #pragma unroll
-                        for (int ks = 4; ks < 8; ++ks) {
-                            tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), instr_desc(DP, true), 1u);
-                        }
+                        for (int ks = 4; ks < 8; ++ks) tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), instr_desc(DP, true), 1u);
                     } else {
                         const uint32_t idesc = instr_desc((p.dv + 15) & ~15, true);
 #pragma unroll 1
-                        for (int ks = 0; ks < keys >> 4; ++ks) {
-                            tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), idesc, (j > 0 || ks > 0) ? 1u : 0u);
-                        }
+                        for (int ks = 0; ks < keys >> 4; ++ks) tc_mma_ts(d_o, a_p + ks * 8, vd + ((ks * 2048) >> 4), idesc, (j > 0 || ks > 0) ? 1u : 0u);
                     }
                     tc_commit(bar(P::bPVDone + t));
                     tc_commit(bar(P::bKVEmpty + v_slot));
@@ -583,14 +604,14 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 // Blocks that only tile A sees: this warp's release of their ring tiles. (Not before
                 // they have been loaded: the arrival must not fall into the slot's previous use.)
                 for (int e = 0; ok && e < 2 * (entries - nb); ++e) {
-                    wait_two(bar(P::bKVFull + s_slot), s_lap, bar(P::bKVFull + s_slot), s_lap, 260);
+                    wait_bar(bar(P::bKVFull + s_slot), s_lap, 260 + t);
                     if (lane == 0) mbar_arrive(bar(P::bKVEmpty + s_slot));
                     __syncwarp();
                     advance(s_slot, s_lap, 1);
                 }
             }
             if (dual && nb == 0) {   // Q is released by both
-                wait_two(bar(P::bQFull), q_items & 1, bar(P::bQFull), q_items & 1, 204);
+                wait_bar(bar(P::bQFull), q_items & 1, 204);
                 if (lane == 0) mbar_arrive(bar(P::bQFree));
                 __syncwarp();
             }
@@ -613,18 +634,16 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
         int blk = 0;        // key blocks of this tile so far: parity of its barriers
         int shared = 0;     // dual: items in which B had a part
         bool ok = true;
-        auto wait_for = [&](int b, int parity, int code) {
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait_inline(bar(b), parity, abort_flag, code, tp.status));
-        };
+        auto wait_for = [&](int b, int parity, int code) { ok = ok && wait_one(bar(b), parity, abort_flag, code); };
         const float sc = p.scale_log2;
 
         for (int n = 0; ok; ++n) {
-            const int w = take_item(n, ok);
-            if (w == -1) break;
-            if (w == -2) continue;
-            Item k = decode_item(tp, w);
-            if (!(t ? k.valid[1] : k.valid[0])) continue;
-            if constexpr (kMask == 2) apply_plan(tp, k);
+            Item k;
+            if (!take_item(n, k, ok)) break;
+            if (!(t ? k.valid[1] : k.valid[0])) {
+                give_item(n);
+                continue;
+            }
             // (Selected once: an index that is not a constant would put the item into memory.)
             const int nb = t ? k.n[1] : k.n[0], h = t ? k.h[1] : k.h[0], q0 = t ? k.q0[1] : k.q0[0], kend = t ? k.kend[1] : k.kend[0];
             const int qi = q0 + row;                    // row inside the sequence
@@ -637,10 +656,13 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     for (int c = 0; c < p.dv; c += 8) *reinterpret_cast<uint4*>(og + c) = make_uint4(0u, 0u, 0u, 0u);
                     if (p.lse) p.lse[k.b * p.ls[0] + h * p.ls[1] + (k.si.q_off + qi) * p.ls[2]] = -INFINITY;
                 }
+                give_item(n);
                 continue;
             }
             // Keys this row may see: [0, row_limit). The smallest limit of the warp is its first
-            // row's, the largest its last row's.
+            // row's, the largest its last row's. A warp without a row of the sequence does no
+            // arithmetic; what its rows of P hold reaches only rows of O that nobody reads.
+            const bool idle = q0 + (warp & 3) * 32 >= k.si.lq;
             auto limit_of = [&](int i) { return p.causal ? min(kend, i + k.si.shift + 1) : kend; };
             const int row_limit = limit_of(qi), limit_lo = limit_of(q0 + (warp & 3) * 32), limit_hi = limit_of(q0 + (warp & 3) * 32 + 31);
             float m_ref = -INFINITY;   // reference maximum (base-2 logits), moved lazily
@@ -663,7 +685,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 const int limit = row_limit - block * kBN;        // my columns [0, limit) are visible
                 const int lo = limit_lo - block * kBN;
                 int chunks = min(max(limit_hi - block * kBN + 31, 0) >> 5, 4);   // 32-column chunks with a visible key
-                const int stored = min((kend - block * kBN + 31) >> 5, 4);  // chunks that P V reads
+                int stored = min((kend - block * kBN + 31) >> 5, 4);             // chunks that P V reads
                 int kind = kNoEffect;
                 const float* mrow = nullptr;
                 if constexpr (kMask == 1) {
@@ -672,27 +694,31 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     // gave up elsewhere must not strand the others. Two rows alternate: a row is
                     // written again only after everybody has arrived for the block between.)
                     float* rows = reinterpret_cast<float*>(smem + P::kMaskRow) + (t * 2 + (gb & 1)) * 128;
-                    const int key = max(min(block * kBN + row, k.si.klen - 1), 0);
-                    rows[row] = mask_value(p, k.b, h, 0, static_cast<int64_t>(k.si.k_off) + key) * kLog2e;
+                    // (-inf past the last key of the tile: such a block needs no other test.)
+                    const int key = block * kBN + row;
+                    rows[row] = key < kend ? mask_value(p, k.b, h, 0, static_cast<int64_t>(k.si.k_off) + key) * kLog2e : -INFINITY;
                     mbar_arrive_warp(bar(P::bMask + t));
                     wait_for(P::bMask + t, gb & 1, 340 + t);
                     if (!ok) break;
                     mrow = rows;
                 }
-                uint4 bits = make_uint4(0u, 0u, 0u, 0u);
                 if constexpr (kMask == 2) {
                     kind = kinds[block];
                     if (kind == kHidden) chunks = 0;
-                    if (kind == kYesNo) bits = tp.plan.bits[(piece0 + block) * 32 + lane];
                 }
+                if (idle) chunks = stored = 0;
+                // A block every key of which every row of this warp sees, without a mask term or with one
+                // that is the same for all rows: the scores go into registers once, in straight-line code.
+                // Any other block (the diagonal, the last keys, a mask with a row per query) takes two
+                // loops over 32-column chunks: the first puts the finished logits back in their place.
+                // (Keys past the end of K are zeros from TMA; past a length they are anything.)
+                const bool fast = kMask == 1 ? !p.causal && (lo >= kBN || (!p.cu_k && kend == p.sk)) && !idle : lo >= kBN && (kMask == 0 || kind == kNoEffect) && !idle;
+                uint4 held = make_uint4(0u, 0u, 0u, 0u);   // plan: this row's visibility bits
+                if (kMask == 2 && kind == kYesNo) held = tp.plan.bits[(piece0 + block) * 32 + lane];
                 wait_for(P::bSFull + t, gb & 1, 300 + t);
                 if (!ok) break;
                 tc_fence_after();
 
-                // A block every key of which every row of this warp sees, without a mask term: the
-                // scores go into registers once, in straight-line code. Any other block (the diagonal,
-                // the last keys, masks) takes a loop over 32-column chunks that reads them twice.
-                const bool fast = kMask != 1 && lo >= kBN && (kMask == 0 || kind == kNoEffect);
                 float s[128];
                 float mx[2] = {-INFINITY, -INFINITY};
                 auto chunk_max = [&](const float* x) {
@@ -702,83 +728,93 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                         mx[1] = max3(mx[1], x[e + 2], x[e + 3]);
                     }
                 };
-                // Chunk c of the scores as base-2 logits with their mask terms, hidden columns -inf.
-                auto logits = [&](float (&x)[32], int c) {
-                    tmem_ld32(s_addr + c * 32, x);
-                    tmem_wait_ld();
-                    if constexpr (kMask == 1) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const float4 m4 = reinterpret_cast<const float4*>(mrow + c * 32)[e];
-                            x[e * 4] = fmaf(x[e * 4], sc, m4.x);
-                            x[e * 4 + 1] = fmaf(x[e * 4 + 1], sc, m4.y);
-                            x[e * 4 + 2] = fmaf(x[e * 4 + 2], sc, m4.z);
-                            x[e * 4 + 3] = fmaf(x[e * 4 + 3], sc, m4.w);
-                        }
-                    } else if (kMask == 2 && kind == kValues && !tp.plan.wide) {
-                        const uint4* v = tp.plan.values + ((piece0 + block) * 16 + c * 4) * 32 + lane;
-                        uint4 q[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) q[e] = v[e * 32];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const uint32_t u[4] = {q[e].x, q[e].y, q[e].z, q[e].w};
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const float m0 = fmaxf(__uint_as_float(u[i] << 16), kMaskedLogit), m1 = fmaxf(__uint_as_float(u[i] & 0xffff0000u), kMaskedLogit);
-                                x[e * 8 + i * 2] = fmaf(x[e * 8 + i * 2], sc, m0 * kLog2e);
-                                x[e * 8 + i * 2 + 1] = fmaf(x[e * 8 + i * 2 + 1], sc, m1 * kLog2e);
-                            }
-                        }
-                    } else if (kMask == 2 && kind == kValues) {
-                        const float4* v = reinterpret_cast<const float4*>(tp.plan.values) + ((piece0 + block) * 32 + c * 8) * 32 + lane;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const float4 m4 = v[e * 32];
-                            x[e * 4] = fmaf(x[e * 4], sc, fmaxf(m4.x, kMaskedLogit) * kLog2e);
-                            x[e * 4 + 1] = fmaf(x[e * 4 + 1], sc, fmaxf(m4.y, kMaskedLogit) * kLog2e);
-                            x[e * 4 + 2] = fmaf(x[e * 4 + 2], sc, fmaxf(m4.z, kMaskedLogit) * kLog2e);
-                            x[e * 4 + 3] = fmaf(x[e * 4 + 3], sc, fmaxf(m4.w, kMaskedLogit) * kLog2e);
-                        }
-                    } else if (kMask == 2 && kind != kNoEffect) {
-                        const uint32_t word = c == 0 ? bits.x : c == 1 ? bits.y : c == 2 ? bits.z : bits.w;
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) x[e] = fmaf(x[e], sc, (word >> e) & 1u ? 0.f : kMaskedLogit * kLog2e);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) x[e] *= sc;
-                    }
-                    if (lo < (c + 1) * 32) {
-                        const int left = limit - c * 32;
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) x[e] = e < left ? x[e] : -INFINITY;
-                    }
-                };
-                float top;
+                float fs = kMask == 1 ? 1.f : sc;   // what is left to scale the registers' values by
                 if (fast) {
                     tmem_ld32(s_addr, s);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
+                        if (kMask == 1 && c >= stored) continue;
+                        float* x = s + c * 32;
                         tmem_wait_ld();
-                        if (c < 3) {
-                            tmem_ld32(s_addr + (c + 1) * 32, s + (c < 3 ? c + 1 : 3) * 32);
-                        } else if (!P::kPOverS) {
+                        if (c < 3 && !(kMask == 1 && c + 1 >= stored)) tmem_ld32(s_addr + (c + 1) * 32, s + (c < 3 ? c + 1 : 3) * 32);
+                        else if (!P::kPOverS) {
                             // The scores are in registers: the next Q K^T may have their columns.
                             tc_fence_before();
                             mbar_arrive_warp(bar(P::bSFree + t));
                         }
-                        chunk_max(s + c * 32);
+                        if constexpr (kMask == 1) {
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                const float4 m4 = reinterpret_cast<const float4*>(mrow + c * 32)[e];
+                                x[e * 4] = fmaf(x[e * 4], sc, m4.x);
+                                x[e * 4 + 1] = fmaf(x[e * 4 + 1], sc, m4.y);
+                                x[e * 4 + 2] = fmaf(x[e * 4 + 2], sc, m4.z);
+                                x[e * 4 + 3] = fmaf(x[e * 4 + 3], sc, m4.w);
+                            }
+                        }
+                        chunk_max(x);
                     }
-                    top = fmaxf(mx[0], mx[1]) * sc;
                 } else {
+                    fs = 1.f;
 #pragma unroll 1
                     for (int c = 0; c < chunks; ++c) {
                         float x[32];
-                        logits(x, c);
+                        tmem_ld32(s_addr + c * 32, x);
+                        if constexpr (kMask == 2) {
+                            if (kind == kValues && !tp.plan.wide) {
+                                const uint4* v = tp.plan.values + ((piece0 + block) * 16 + c * 4) * 32 + lane;
+                                uint4 q[4];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) q[e] = v[e * 32];
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const uint32_t u[4] = {q[e].x, q[e].y, q[e].z, q[e].w};
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) {
+                                        const float m0 = fmaxf(__uint_as_float(u[i] << 16), kMaskedLogit), m1 = fmaxf(__uint_as_float(u[i] & 0xffff0000u), kMaskedLogit);
+                                        x[e * 8 + i * 2] = fmaf(x[e * 8 + i * 2], sc, m0 * kLog2e);
+                                        x[e * 8 + i * 2 + 1] = fmaf(x[e * 8 + i * 2 + 1], sc, m1 * kLog2e);
+                                    }
+                                }
+                            } else if (kind == kValues) {
+                                const float4* v = reinterpret_cast<const float4*>(tp.plan.values) + ((piece0 + block) * 32 + c * 8) * 32 + lane;
+                                float4 q[8];
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) q[e] = v[e * 32];
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) {
+                                    x[e * 4] = fmaf(x[e * 4], sc, fmaxf(q[e].x, kMaskedLogit) * kLog2e);
+                                    x[e * 4 + 1] = fmaf(x[e * 4 + 1], sc, fmaxf(q[e].y, kMaskedLogit) * kLog2e);
+                                    x[e * 4 + 2] = fmaf(x[e * 4 + 2], sc, fmaxf(q[e].z, kMaskedLogit) * kLog2e);
+                                    x[e * 4 + 3] = fmaf(x[e * 4 + 3], sc, fmaxf(q[e].w, kMaskedLogit) * kLog2e);
+                                }
+                            } else if (kind != kNoEffect) {
+                                const uint32_t word = c == 0 ? held.x : c == 1 ? held.y : c == 2 ? held.z : held.w;
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int e = 0; e < 32; ++e) x[e] = fmaf(x[e], sc, (word >> e) & 1u ? 0.f : kMaskedLogit * kLog2e);
+                            } else {
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int e = 0; e < 32; ++e) x[e] *= sc;
+                            }
+                        } else {
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) x[e] = kMask == 1 ? fmaf(x[e], sc, mrow[c * 32 + e]) : x[e] * sc;
+                        }
+                        if (lo < c * 32 + 32) {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) x[e] = c * 32 + e < limit ? x[e] : -INFINITY;
+                        }
+                        tmem_st32(s_addr + c * 32, x);
                         chunk_max(x);
                     }
-                    top = fmaxf(mx[0], mx[1]);
+                    tmem_wait_st();
                 }
+                const float top = fmaxf(mx[0], mx[1]) * fs;
 
                 // Lazy rescale: move the reference only when this block exceeds it by 2^8.
                 const bool move = top > m_ref + kRescaleGap;
@@ -810,10 +846,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
 
                 // ---- P = 2^(logit - m) as packed bf16 pairs ----
-                const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(-m_use, -m_use);
+                const float2 sc2 = make_float2(fs, fs), nm2 = make_float2(-m_use, -m_use);
                 // P's columns are free once the previous block's P V has read them.
                 auto wait_p_free = [&]() {
-                    if (j > 0) {
+                    if (!P::kPOverS && j > 0) {
                         wait_for(P::bPVDone + t, (gb - 1) & 1, 320 + t);
                         tc_fence_after();
                     }
@@ -821,6 +857,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 if (fast) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
+                        if (kMask == 1 && c >= stored) continue;
                         uint32_t wv[16];
                         const float* x = s + c * 32;
 #pragma unroll
@@ -828,7 +865,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                             const float2 y = __ffma2_rn(make_float2(x[2 * e], x[2 * e + 1]), sc2, nm2);
                             float2 pr;
                             // The polynomial pairs are spread evenly: MUFU and FMA work alternate.
-                            if ((e * P::kPolyPairs) % 8 < P::kPolyPairs) {
+                            // (Terms may hide a key; those take MUFU, whose 2^-inf is exactly 0.)
+                            if (kMask != 1 && (e * P::kPolyPairs) % 8 < P::kPolyPairs) {
                                 pr = exp2_poly2(y);
                             } else {
                                 pr.x = fast_exp2(y.x);
@@ -837,9 +875,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                             l2[e & 1] = __fadd2_rn(l2[e & 1], pr);
                             wv[e] = pack_bf16(pr.x, pr.y);
                         }
-                        if (!P::kPOverS && c == 0) wait_p_free();
+                        if (c == 0) wait_p_free();
                         tmem_st16(p_addr + c * 16, wv);
-                        if (P::kPOverS && c == 1) {
+                        if (P::kPOverS && (c == 1 || (kMask == 1 && c == 0 && stored == 1))) {
                             // P V may start on the first half of the keys.
                             tmem_wait_st();
                             tc_fence_before();
@@ -847,14 +885,16 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                         }
                     }
                 } else {
-                    if (!P::kPOverS) wait_p_free();
+                    // (Idle warps wait too: one that did not could get a whole item ahead and find a
+                    // barrier's parity right for the wrong reason.)
+                    wait_p_free();
 #pragma unroll 1
                     for (int c = 0; c < stored; ++c) {
                         uint32_t wv[16];
                         if (c < chunks) {
-                            // Hidden columns take MUFU, whose 2^-inf is exactly 0.
                             float x[32];
-                            logits(x, c);
+                            tmem_ld32(s_addr + c * 32, x);
+                            tmem_wait_ld();
 #pragma unroll
                             for (int e = 0; e < 16; ++e) {
                                 const float2 y = __fadd2_rn(make_float2(x[2 * e], x[2 * e + 1]), nm2);
@@ -880,6 +920,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             if (!ok) break;
 
             // ---- the item's end: O / l to memory ----
+            // (The item is read from the queue again: its numbers would not fit beside the scores.)
+            const Item* e = queue + n % P::kQueue;
+            const int nb_other = e->n[1], e_b = e->b, e_h = e->h[dual ? 0 : t], e_q0 = e->q0[dual ? 0 : t], e_lq = e->si.lq, e_off = e->si.q_off;
             const int last = blk + nb - 1;
             blk += nb;
             wait_for(P::bPVDone + t, last & 1, 330 + t);
@@ -887,7 +930,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             tc_fence_after();
             float l_row = (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y), m_row = m_ref;
             float f_mine = 1.f, f_other = 0.f;
-            const bool merge = dual && k.n[1] > 0;
+            const bool merge = dual && nb_other > 0;
             if (merge) {
                 float2* part = reinterpret_cast<float2*>(smem + P::kPartial);
                 if (t == 1) {
@@ -895,6 +938,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     part[row] = make_float2(m_row, l_row);
                     tc_fence_before();
                     mbar_arrive_warp(bar(P::bPartial));
+                    give_item(n);
                     continue;
                 }
                 wait_for(P::bPartial, shared & 1, 380);
@@ -910,47 +954,56 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 m_row = m_all;
             }
             const float inv = l_row > 0.f ? 1.f / l_row : 0.f;
-            __nv_bfloat16* og = p.out + k.b * p.os[0] + h * p.os[1] + static_cast<int64_t>(k.si.q_off + qi) * p.os[2];
+            // A warp's 32 rows, 32 columns at a time. Four lanes exchange their rows' 16-byte pieces
+            // first, so that a store writes 64 bytes of each of eight rows (a thread's own row straight
+            // to memory is a line of its own for every piece: 4,300 clk for 128 rows of 80, now 3,100).
+            const int r0 = e_q0 + (warp & 3) * 32 + (lane & ~3);
+            __nv_bfloat16* og = p.out + e_b * p.os[0] + e_h * p.os[1] + static_cast<int64_t>(e_off + r0) * p.os[2] + (lane & 3) * 8;
+#pragma unroll 1
+            for (int c = 0; c * 32 < p.dv; ++c) {
+                float o[32];
+                tmem_ld32(o_addr + c * 32, o);
+                if (merge) {
+                    float o1[32];
+                    tmem_ld32(tmem + lane_addr + P::kO + DP + c * 32, o1);
+                    tmem_wait_ld();
 #pragma unroll
-            for (int c = 0; c < DP / 32; ++c) {
-                if (c * 32 < p.dv) {
-                    float o[32];
-                    tmem_ld32(o_addr + c * 32, o);
-                    if (merge) {
-                        float o1[32];
-                        tmem_ld32(tmem + lane_addr + P::kO + DP + c * 32, o1);
-                        tmem_wait_ld();
+                    for (int e = 0; e < 32; ++e) o[e] = fmaf(o1[e], f_other, o[e] * f_mine);
+                } else {
+                    tmem_wait_ld();
+                }
+                if (c * 32 + 32 >= p.dv) {
+                    // O is in registers: the next item's P V may overwrite it.
+                    tc_fence_before();
+                    mbar_arrive_warp(bar(P::bOFree + t));
+                    if (merge) mbar_arrive_warp(bar(P::bOFree + 1));
+                }
+                uint32_t w[4][4];   // [piece][word]; after the exchange [row][word] of piece lane & 3
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) o[e] = fmaf(o1[e], f_other, o[e] * f_mine);
-                    } else {
-                        tmem_wait_ld();
-                    }
-                    if (c * 32 + 32 >= p.dv) {
-                        // O is in registers: the next item's P V may overwrite it.
-                        tc_fence_before();
-                        mbar_arrive_warp(bar(P::bOFree + t));
-                        if (merge) mbar_arrive_warp(bar(P::bOFree + 1));
-                    }
-                    if (real) {
+                for (int e = 0; e < 16; ++e) w[e >> 2][e & 3] = pack_bf16(o[2 * e] * inv, o[2 * e + 1] * inv);
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            uint32_t q[8];
+                for (int x = 1; x < 4; x <<= 1) {
+                    const bool odd = lane & x;
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) q[i] = pack_bf16(o[e * 16 + 2 * i] * inv, o[e * 16 + 2 * i + 1] * inv);
-                            const int left = p.dv - c * 32 - e * 16;   // columns still to write (Dv is a multiple of 8)
-                            if (left >= 16) {
-                                store_32_bytes(og + c * 32 + e * 16, q);
-                            } else if (left >= 8) {
-                                *reinterpret_cast<uint4*>(og + c * 32 + e * 16) = make_uint4(q[0], q[1], q[2], q[3]);
-                            }
+                    for (int a = 0; a < 4; ++a) {
+                        if (a & x) continue;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? w[a][i] : w[a + x][i], x);
+                            if (odd) w[a][i] = got; else w[a + x][i] = got;
                         }
                     }
                 }
+                const bool inside = c * 32 + (lane & 3) * 8 < p.dv;
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    if (inside && r0 + a < e_lq) *reinterpret_cast<uint4*>(og + a * p.os[2] + c * 32) = make_uint4(w[a][0], w[a][1], w[a][2], w[a][3]);
+                }
             }
-            if (real && p.lse) {
-                p.lse[k.b * p.ls[0] + h * p.ls[1] + (k.si.q_off + qi) * p.ls[2]] =
-                    l_row > 0.f ? kLn2 * (m_row + log2f(l_row)) : -INFINITY;
+            if (p.lse && e_q0 + row < e_lq) {
+                p.lse[e_b * p.ls[0] + e_h * p.ls[1] + (e_off + e_q0 + row) * p.ls[2]] = l_row > 0.f ? kLn2 * (m_row + log2f(l_row)) : -INFINITY;
             }
+            give_item(n);
         }
     }
 
@@ -960,6 +1013,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
     __syncthreads();
     if (warp == kMmaWarp) {
         if (*abort_flag) {
+            if (lane == 0) atomicCAS_system(tp.status, 0, *abort_flag);
             const long long t0 = clock64();
             while (clock64() - t0 < 2000000) {
             }

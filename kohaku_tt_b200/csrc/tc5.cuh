@@ -99,23 +99,6 @@ __device__ __forceinline__ bool mbar_wait(
     if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_slow(bar, parity, abort_flag, code, status);
 }
-// The same without a call: for kernels whose warps hold more registers than the calling convention
-// keeps across one (and for those that move registers between warpgroups, where the compiler
-// cannot allocate a call at all).
-__device__ __forceinline__ bool mbar_wait_inline(
-    uint32_t bar, uint32_t parity, volatile int* abort_flag, int code, int* status) {
-    if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
-    const long long t0 = clock64();
-    while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if (clock64() - t0 > kWaitCycles) {
-            *abort_flag = 1;
-            atomicCAS_system(status, 0, code);
-            return false;
-        }
-    }
-}
 
 __device__ __forceinline__ void tma_load_4d(
     uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
