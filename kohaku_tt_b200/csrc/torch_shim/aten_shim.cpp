@@ -600,6 +600,7 @@ struct Attention : torch::autograd::Function<Attention> {
             out = {dq, dk, dv};
         }
         if (at::GradMode::is_enabled()) {   // create_graph: differentiating the gradients is an error, not a silent zero
+            for (Tensor& g : out) g.set_requires_grad(true);   // (a node is only attached to what may need one)
             out = (*std::make_shared<torch::autograd::DelayedError>("kohaku_tt_b200: the gradients of attention are not differentiable", 3))(std::move(out));
         }
         return {out[0], out[1], out[2], Tensor(), Tensor()};
