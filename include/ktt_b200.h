@@ -251,7 +251,8 @@ KTT_B200_API int64_t ktt_b200_sdpa_forward_workspace(const ktt_b200_attn_args* a
  * Launches nothing. */
 KTT_B200_API int ktt_b200_forward_streams_per_sm(void);
 
-/* Bytes of workspace ktt_b200_sdpa_backward needs for the problem (0 on error). */
+/* Bytes of workspace ktt_b200_sdpa_backward needs for the problem (0 on error), its strides among
+ * the arguments: the tcgen05 kernels keep two fp32 per query row there, the others one. */
 KTT_B200_API int64_t ktt_b200_sdpa_backward_workspace(const ktt_b200_attn_args* args);
 /* Backward (dq, dk, dv with the softmax recomputed from lse): ktt_sdpa_train_backward
  * (ktt_capi.h:126-135), bridge::sdpa_varlen_backward, bridge::sdpa_lengths_backward. */

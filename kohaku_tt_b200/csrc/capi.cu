@@ -1,4 +1,5 @@
 // The extern "C" surface: argument checks, kernel choice, counters, error text.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -119,10 +120,9 @@ void delta_layout(const ktt_b200_attn_args* a, int64_t& bs, int64_t& hs, int64_t
 }
 
 // Bytes of it, or of the row terms that stand there in the tcgen05 backward.
-int64_t row_term_bytes(const ktt_b200_attn_args* a, int64_t total) {
-    const int64_t blocks = row_blocks(a->cu_seqlens_q != nullptr, a->total_q, a->batch, a->sq) * a->heads;
-    const int64_t need = total * 4 > blocks * 1024 ? total * 4 : blocks * 1024;
-    return (need + 255) / 256 * 256;
+int64_t row_term_bytes(const AttnParams& p, int64_t total, bool tc5) {
+    const int64_t blocks = tc5 ? row_blocks(p.cu_q != nullptr, p.total_q, p.batch, p.sq) * p.heads : 0;
+    return (std::max(total * 4, blocks * 1024) + 255) / 256 * 256;
 }
 
 __global__ void merge_partials_kernel(
@@ -365,7 +365,9 @@ extern "C" int64_t ktt_b200_sdpa_backward_workspace(const ktt_b200_attn_args* a)
     delta_layout(a, bs, hs, total);
     AttnParams p;
     to_params(a, p);
-    return row_term_bytes(a, total) + backward_partial_bytes(p, backward_group_split(p));
+    const char* why = nullptr;
+    const bool tc5 = a->kernel != KTT_B200_KERNEL_MMA && backward_tc5_takes(p, &why);
+    return row_term_bytes(p, total, tc5) + backward_partial_bytes(p, backward_group_split(p));
 }
 
 __global__ void zero_uncovered_rows_kernel(const AttnParams p) {
@@ -384,9 +386,17 @@ extern "C" int ktt_b200_sdpa_backward(const ktt_b200_attn_args* a, void* stream)
     delta_layout(a, bs, hs, total);
     AttnParams p;
     to_params(a, p);
-    const int64_t delta_bytes = row_term_bytes(a, total);
+    const char* why = nullptr;
+    bool tc5 = a->kernel != KTT_B200_KERNEL_MMA && backward_tc5_takes(p, &why);
+    if (a->kernel == KTT_B200_KERNEL_TC5 && !tc5) {
+        note_call(4);
+        return fail(KTT_B200_ERR_UNSUPPORTED, "sdpa_backward: tcgen05 kernel: %s", why);
+    }
     p.gsplit = backward_group_split(p);
-    const int64_t need = delta_bytes + backward_partial_bytes(p, p.gsplit);
+    const int64_t partial_bytes = backward_partial_bytes(p, p.gsplit);
+    // A workspace sized before the strides were known: the warp-MMA kernels need no more.
+    if (tc5 && a->kernel == KTT_B200_KERNEL_AUTO && a->workspace_bytes < row_term_bytes(p, total, true) + partial_bytes) tc5 = false;
+    const int64_t delta_bytes = row_term_bytes(p, total, tc5), need = delta_bytes + partial_bytes;
     if (!a->workspace || a->workspace_bytes < need) {
         return fail(KTT_B200_ERR_BAD_ARGUMENT, "sdpa_backward: workspace holds %lld bytes, %lld needed",
                     static_cast<long long>(a->workspace_bytes), static_cast<long long>(need));
@@ -399,13 +409,7 @@ extern "C" int ktt_b200_sdpa_backward(const ktt_b200_attn_args* a, void* stream)
         ? reinterpret_cast<int32_t*>(static_cast<unsigned char*>(a->workspace) + delta_bytes + backward_counter_offset(p, p.gsplit))
         : nullptr;
     note_call(2);
-    const char* why = nullptr;
-    const bool tc5 = backward_tc5_takes(p, &why);
-    if (a->kernel == KTT_B200_KERNEL_TC5 && !tc5) {
-        note_call(4);
-        return fail(KTT_B200_ERR_UNSUPPORTED, "sdpa_backward: tcgen05 kernel: %s", why);
-    }
-    if (tc5 && a->kernel != KTT_B200_KERNEL_MMA) {
+    if (tc5) {
         note_call(6);
         return launch_backward_tc5(p, static_cast<cudaStream_t>(stream));
     }
