@@ -33,7 +33,7 @@
 // Two ways to use the two tiles:
 //   pair   A and B are neighbours in the list of (query tile, head) of one K / V head: one
 //          K / V stream serves both, which halves the traffic from L2
-//   dual   (few tiles per SM) A and B are the same query tile, A working on the first half of
+//   dual   (no more tiles than SMs) A and B are the same query tile, A working on the first half of
 //          its key blocks and B on the rest; A's threads then read B's unnormalised O straight
 //          out of tensor memory. The longest tile's serial chain is halved. Always A then B:
 //          the bits do not depend on timing.
@@ -1280,7 +1280,11 @@ int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_
     const int64_t units = static_cast<int64_t>(q_tiles) * group * p.kv_heads * p.batch;   // (query tile, head)
     if (units > 0x3fffffff) return fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 forward: too many query tiles");
     const int sms = sm_count();
-    tp.dual = p.sk > kBN && units <= 6 * static_cast<int64_t>(sms) ? 1 : 0;
+    // Dual halves a tile's chain of blocks but adds a merge and doubles the items: it pays where
+    // tiles would leave SMs without one. (Up to six tiles per SM it cost more than it gave: 16 x 16
+    // heads x 257, D 80: 43 -> 37 us without it, 4 x 16 heads 19 -> 13; 2 x 16 heads x 2048, D 64,
+    // causal mask: 71 -> 58. At 8 heads x 2 x 1024, D 80, 128 tiles, it gives 25 -> 16.)
+    tp.dual = p.sk > kBN && units <= sms ? 1 : 0;
     const int levels = tp.dual ? q_tiles * group : (q_tiles * group + 1) / 2;
     tp.work = levels * p.kv_heads * p.batch;
     tp.by_batch = divisor_of(p.batch);
