@@ -316,7 +316,7 @@ extern "C" int ktt_b200_sdpa_forward(const ktt_b200_attn_args* a, void* stream) 
         note_call(4);
         return fail(KTT_B200_ERR_UNSUPPORTED, "sdpa_forward: tcgen05 kernel: %s", why);
     }
-    if (tc5 && a->kernel != KTT_B200_KERNEL_MMA) {
+    if (tc5 && a->kernel != KTT_B200_KERNEL_MMA && !(a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_preferred(p))) {
         note_call(0);
         const char* why_row = nullptr;
         if (a->kernel != KTT_B200_KERNEL_TC5_WIDE && forward_row_takes(p, &why_row)) {
@@ -330,8 +330,9 @@ extern "C" int ktt_b200_sdpa_forward(const ktt_b200_attn_args* a, void* stream) 
         p.fwd_done_counter = (usable && a->workspace_bytes >= 256) ? static_cast<int32_t*>(a->workspace) + 1 : nullptr;
         return launch_forward_tc5(p, st);
     }
-    // What is left for AUTO: head dims those kernels are not built for and masks with a row per
-    // query. The latter need their workspace; a caller that brings none keeps the warp-MMA kernel.
+    // What is left for AUTO: head dims those kernels are not built for, masks with a row per query
+    // and calls in which this one is the faster. The masks need their workspace; a caller that
+    // brings none keeps the warp-MMA kernel.
     if (a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_takes(p) && (!row_per_query(p) || a->workspace_bytes >= forward_pair_workspace(p))) {
         note_call(0);
         return launch_forward_pair(p, a->workspace, a->workspace_bytes, st);

@@ -1,6 +1,6 @@
-// Forward on the Blackwell tensor path for what the other two tcgen05 kernels are not built for:
-// head dims that are any multiple of 8 up to 128, and masks with a row per query. TMA tile
-// loads, tcgen05.mma with accumulators in tensor memory, online softmax with one thread per
+// Forward on the Blackwell tensor path for what the other two tcgen05 kernels are not built for -
+// head dims that are any multiple of 8 up to 128, and masks with a row per query - and for calls
+// of few keys in which it is the faster (forward_pair_preferred). TMA tile loads, tcgen05.mma with accumulators in tensor memory, online softmax with one thread per
 // query row.
 //
 // A persistent CTA per SM works on two 128-row query tiles at a time, A and B:
@@ -1241,6 +1241,28 @@ bool forward_pair_takes(const AttnParams& p) {
     const char* why;
     return operand_layout(p.q, tq, p.heads, bq, p.qs, s, &why) && operand_layout(p.k, tk, p.kv_heads, bq, p.ks, s, &why) &&
            operand_layout(p.v, tk, p.kv_heads, bq, p.vs, s, &why);
+}
+
+// Head dims 64 and 128 without a mask or with one row of it per (batch, head) have kernels of their
+// own, with one tile per work item and two items at a time on an SM. This one is faster where its
+// pairs fill whole rounds and the keys are few: what it leaves out of a block (columns past the last
+// key, the item arithmetic of all roles but one) weighs most there. Measured on B200, other kernel
+// -> this one: D 64, 520 tiles, 64 keys 17.1 -> 13.0 us, 300 keys 25.1 -> 19.6, 1024 keys 38.4 ->
+// 34.5; D 128, 220 tiles, 256 keys 13.5 -> 11.9, 64 keys 11.1 -> 9.3. The lines:
+//  - as many rounds as the others need, up to three (from the fourth on it is even or slower), and
+//    no last round in which a single tile per SM would run alone and faster (of three rounds that
+//    one weighs less);
+//  - D 64: 1024 keys, with mask terms 320 (at 1024 keys 26.9 -> 27.9);
+//  - D 128: 320 keys in the first round or with mask terms, else 96 (at 200 keys 20.9 -> 21.9).
+bool forward_pair_preferred(const AttnParams& p) {
+    if (p.causal || p.cu_q || p.key_lengths || mask_needs_plan(p) || p.d != p.dv || (p.d != 64 && p.d != 128)) return false;
+    const int64_t sms = sm_count(), group = p.heads / p.kv_heads, planes = static_cast<int64_t>(p.batch) * p.kv_heads;
+    const int64_t per_plane = (p.sq + kBM - 1) / kBM * group, tiles = per_plane * planes, pairs = (per_plane + 1) / 2 * planes;
+    const int64_t rounds = (tiles + 2 * sms - 1) / (2 * sms), last = tiles - (rounds - 1) * 2 * sms;
+    if (rounds > 3 || pairs > rounds * sms || (rounds < 3 && last <= sms)) return false;
+    const bool masked = p.mask_dtype != KTT_B200_MASK_NONE;
+    const int most = p.d == 64 ? (masked ? 320 : 1024) : (rounds == 1 || masked ? 320 : 96);
+    return p.sk <= most && forward_pair_takes(p);
 }
 
 int64_t forward_pair_workspace(const AttnParams& p) {

@@ -41,6 +41,19 @@ def test_head_dims(cuda, b, h, hk, sq, sk, d, dv, causal):
     _check(cuda, *qkv(b, h, hk, sq, sk, d, sq + sk + d, dv=dv), causal=causal)
 
 
+# Calls that other kernels take too: just inside and outside the rounds, tiles and keys between them.
+@pytest.mark.parametrize("h,sq,sk,d,masked", [
+    (37, 512, 96, 64, True), (38, 400, 77, 64, True), (148, 256, 40, 64, False), (50, 300, 320, 64, True),
+    (75, 130, 321, 64, True), (38, 512, 321, 64, False), (149, 256, 33, 128, True), (80, 256, 97, 128, False),
+    (80, 200, 129, 128, True), (112, 512, 64, 128, False),
+])
+def test_few_keys(cuda, h, sq, sk, d, masked):
+    q, k, v = qkv(1, h, h, sq, sk, d, h + sq + sk)
+    keep = torch.rand(1, 1, 1, sk, generator=torch.Generator().manual_seed(h)) > 0.3
+    keep[..., 0] = True
+    _check(cuda, q, k, v, mask=keep if masked else None)
+
+
 def test_head_dim_80_with_key_lengths_and_a_key_mask(cuda):
     q, k, v = qkv(3, 4, 2, 200, 300, 80, 5)
     _check(cuda, q, k, v, lengths=[300, 1, 130])
