@@ -211,7 +211,7 @@ __device__ __forceinline__ void dkv_body(
     };
 
     // Set-up. The producer warp initialises the barriers itself and sends the CTA's first
-    // loads (K, V and the first ring stages; none of them is written by the delta kernel this
+    // loads (K, V and the first ring stages; none of them is written by the row kernel this
     // launch may overlap) while warp 8 allocates tensor memory and the rest wait.
     int issued = 0;
     if (warp == 9) {
@@ -1156,7 +1156,7 @@ int launch_bwd(const AttnParams& p, cudaStream_t stream) {
     const int64_t n_all = n_dkv + static_cast<int64_t>(dq_x) * dq_y * p.batch;
     if (n_all > 0x7fffffff) return fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 backward: too many tiles");
     if (p.gsplit > 1 && !p.dkv_counters) return fail(KTT_B200_ERR_BAD_ARGUMENT, "tcgen05 backward: the group split needs its ticket counters");
-    // Programmatic dependent launch behind the delta kernel: set-up and the first loads of
+    // Programmatic dependent launch behind the row kernel: set-up and the first loads of
     // every CTA of the first wave run while that kernel drains.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(n_all));

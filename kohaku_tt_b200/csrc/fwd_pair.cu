@@ -1,7 +1,7 @@
 // Forward on the Blackwell tensor path for what the other two tcgen05 kernels are not built for -
 // head dims that are any multiple of 8 up to 128, and masks with a row per query - and for calls
-// of few keys in which it is the faster (forward_pair_preferred). TMA tile loads, tcgen05.mma with accumulators in tensor memory, online softmax with one thread per
-// query row.
+// of few keys in which it is the faster (forward_pair_preferred). TMA tile loads, tcgen05.mma with
+// accumulators in tensor memory, online softmax with one thread per query row.
 //
 // A persistent CTA per SM works on two 128-row query tiles at a time, A and B:
 //
