@@ -151,7 +151,8 @@ struct alignas(16) Item {
 static_assert(sizeof(Item) <= 96, "the queue's slots");
 
 // Items of one (batch, K / V head) are neighbours in its list of (query tile, head), longest
-// causal tiles first, heads fastest. Two orders of the items: with the level slowest every deal
+// causal tiles first (else first rows first: a last tile of few rows is then the one without a
+// partner, and its item the short one), heads fastest. Two orders of the items: with the level slowest every deal
 // in rounds hands out similar lengths; `grouped` (needs the counter) keeps all items of one
 // (batch, K / V head) together, so that the items in flight share the K / V of a few heads in L2
 // (measured on a packed 65,536-token batch with 537 MB of K / V: 4.85 -> 0.81 GB of DRAM reads).
@@ -925,13 +926,13 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             const int nb_other = e->n[1], e_b = e->b, e_h = e->h[dual ? 0 : t], e_q0 = e->q0[dual ? 0 : t], e_lq = e->si.lq, e_off = e->si.q_off;
             const int last = blk + nb - 1;
             blk += nb;
-            wait_for(P::bPVDone + t, last & 1, 330 + t);
-            if (!ok) break;
-            tc_fence_after();
             float l_row = (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y), m_row = m_ref;
             float f_mine = 1.f, f_other = 0.f;
             const bool merge = dual && nb_other > 0;
             if (merge) {
+                wait_for(P::bPVDone + t, last & 1, 330 + t);
+                if (!ok) break;
+                tc_fence_after();
                 float2* part = reinterpret_cast<float2*>(smem + P::kPartial);
                 if (t == 1) {
                     // Tile A's threads take this half out of tensor memory and free it.
@@ -954,6 +955,15 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 m_row = m_all;
             }
             const float inv = l_row > 0.f ? 1.f / l_row : 0.f;
+            // (Without a merge the statistics leave while the last P V runs.)
+            if (p.lse && e_q0 + row < e_lq) {
+                p.lse[e_b * p.ls[0] + e_h * p.ls[1] + (e_off + e_q0 + row) * p.ls[2]] = l_row > 0.f ? kLn2 * (m_row + log2f(l_row)) : -INFINITY;
+            }
+            if (!merge) {
+                wait_for(P::bPVDone + t, last & 1, 332 + t);
+                if (!ok) break;
+                tc_fence_after();
+            }
             // A warp's 32 rows, 32 columns at a time. Four lanes exchange their rows' 16-byte pieces
             // first, so that a store writes 64 bytes of each of eight rows (a thread's own row straight
             // to memory is a line of its own for every piece: 4,300 clk for 128 rows of 80, now 3,100).
@@ -999,9 +1009,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 for (int a = 0; a < 4; ++a) {
                     if (inside && r0 + a < e_lq) *reinterpret_cast<uint4*>(og + a * p.os[2] + c * 32) = make_uint4(w[a][0], w[a][1], w[a][2], w[a][3]);
                 }
-            }
-            if (p.lse && e_q0 + row < e_lq) {
-                p.lse[e_b * p.ls[0] + e_h * p.ls[1] + (e_off + e_q0 + row) * p.ls[2]] = l_row > 0.f ? kLn2 * (m_row + log2f(l_row)) : -INFINITY;
             }
             give_item(n);
         }
