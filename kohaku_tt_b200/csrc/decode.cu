@@ -79,6 +79,10 @@ constexpr int kMaxPending = 8;   // stored partials per CTA before their tickets
 #define KTT_DECODE_PAIR_COST 5
 #endif
 constexpr int kPairCost = KTT_DECODE_PAIR_COST;
+// A share is at least this many units: a tile more in a CTA's stream costs less than one partial more
+// to merge at the pair's end. Measured for 1, 2, 3, 4: one sequence of 3,000 keys, 16 heads over 2,
+// D 128: 13.7, 10.7, 10.9, 11.4 us; 1,000 keys, 14 over 2, D 64: 7.85, 7.66, 7.76, 8.14.
+constexpr int kMinUnits = 2;
 constexpr int kMaxCtas = 1024;   // ticket counters in the scratch
 
 // Keys batch b attends over. Append mode: the cached count clamped to [0, sk - 1], plus the
@@ -258,7 +262,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
     }
     // Equal shares of units; this CTA streams the tiles whose unit lies in its share.
     const int total = p.kv_heads * prefix_s[p.batch];
-    const int upc = (total + gridDim.x - 1) / gridDim.x;
+    const int upc = max(static_cast<int>((total + gridDim.x - 1) / gridDim.x), kMinUnits);
     const int first_unit = min(static_cast<int>(blockIdx.x) * upc, total), end_unit = min(first_unit + upc, total);
     const int u0 = 0;
     const int u1 = tiles_before(p, prefix_s, end_unit) - tiles_before(p, prefix_s, first_unit);
@@ -316,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
         // time, every position's loads waited for the previous position's sums: with two
         // pairs to finish that was four trips to L2 in a row behind the slowest stream.)
         const int per_pair = rows * (D / 4);
-        constexpr int kIlp = 2;
+        constexpr int kIlp = 2, kHolders = 4;
         for (int base = 0; base < n * per_pair; base += kIlp * kThreads) {
             bool act[kIlp];
             int r_[kIlp], c4_[kIlp], slot0[kIlp], parts[kIlp], b_[kIlp], hk_[kIlp];
@@ -341,14 +345,16 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
                 sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                 most = max(most, parts[u]);
             }
-            // Running merge in CTA order (deterministic), four holders per round.
-            for (int c0 = 0; c0 < most; c0 += 4) {
-                float ms[kIlp][4], ls[kIlp][4];
-                float4 v[kIlp][4];
+            // Running merge in CTA order (deterministic), kHolders per round with one maximum for the
+            // round. (Eight per round cost the usual pair of two or three holders their idle loads:
+            // 34.7 against 33.0 us on B 64, lengths U[512, 4096], D 128.)
+            for (int c0 = 0; c0 < most; c0 += kHolders) {
+                float ms[kIlp][kHolders], ls[kIlp][kHolders];
+                float4 v[kIlp][kHolders];
 #pragma unroll
                 for (int u = 0; u < kIlp; ++u) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < kHolders; ++j) {
                         // Past the last holder (or an idle position): a repeat of a valid slot, not used.
                         const int slot = slot0[u] + max(min(c0 + j, parts[u] - 1), 0);
                         ms[u][j] = __ldcg(&p.part_m[slot * 16 + r_[u]]);
@@ -358,19 +364,29 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
                 }
 #pragma unroll
                 for (int u = 0; u < kIlp; ++u) {
+                    // The weights do not wait for one another.
+                    float m_new = mm[u];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (c0 + j < parts[u]) {
-                            const float m_new = fmaxf(mm[u], ms[u][j]);
-                            const float base_m = (m_new == -INFINITY) ? 0.f : m_new;
-                            const float fa = fast_exp2(mm[u] - base_m), fb = fast_exp2(ms[u][j] - base_m);
-                            ll[u] = ll[u] * fa + ls[u][j] * fb;
-                            sum[u].x = sum[u].x * fa + v[u][j].x * fb;
-                            sum[u].y = sum[u].y * fa + v[u][j].y * fb;
-                            sum[u].z = sum[u].z * fa + v[u][j].z * fb;
-                            sum[u].w = sum[u].w * fa + v[u][j].w * fb;
-                            mm[u] = m_new;
-                        }
+                    for (int j = 0; j < kHolders; ++j) {
+                        if (c0 + j >= parts[u]) ms[u][j] = -INFINITY;
+                        m_new = fmaxf(m_new, ms[u][j]);
+                    }
+                    const float base_m = (m_new == -INFINITY) ? 0.f : m_new;
+                    const float fa = fast_exp2(mm[u] - base_m);
+                    mm[u] = m_new;
+                    ll[u] *= fa;
+                    sum[u].x *= fa;
+                    sum[u].y *= fa;
+                    sum[u].z *= fa;
+                    sum[u].w *= fa;
+#pragma unroll
+                    for (int j = 0; j < kHolders; ++j) {
+                        const float fb = fast_exp2(ms[u][j] - base_m);
+                        ll[u] = fmaf(ls[u][j], fb, ll[u]);
+                        sum[u].x = fmaf(v[u][j].x, fb, sum[u].x);
+                        sum[u].y = fmaf(v[u][j].y, fb, sum[u].y);
+                        sum[u].z = fmaf(v[u][j].z, fb, sum[u].z);
+                        sum[u].w = fmaf(v[u][j].w, fb, sum[u].w);
                     }
                 }
             }
