@@ -680,6 +680,14 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 kinds = m.kind + piece0;
             }
 
+            // A block's mask term is fetched one block ahead. (The kind of a plan's piece as well cost
+            // more in registers than it gave: 57.1 -> 58.7 us on 2 x 16 heads x 2048, causal mask.)
+            auto term_of = [&](int blk_) {   // (-inf past the last key of the tile: such a block needs no other test)
+                const int key = blk_ * kBN + row;
+                return key < kend ? mask_value(p, k.b, h, 0, static_cast<int64_t>(k.si.k_off) + key) * kLog2e : -INFINITY;
+            };
+            float term_ahead = 0.f;
+            if constexpr (kMask == 1) term_ahead = term_of(it.at);
             for (int j = 0; ok && j < nb; ++j) {
                 const int gb = blk + j;
                 const int block = it.next();
@@ -695,9 +703,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     // gave up elsewhere must not strand the others. Two rows alternate: a row is
                     // written again only after everybody has arrived for the block between.)
                     float* rows = reinterpret_cast<float*>(smem + P::kMaskRow) + (t * 2 + (gb & 1)) * 128;
-                    // (-inf past the last key of the tile: such a block needs no other test.)
-                    const int key = block * kBN + row;
-                    rows[row] = key < kend ? mask_value(p, k.b, h, 0, static_cast<int64_t>(k.si.k_off) + key) * kLog2e : -INFINITY;
+                    rows[row] = term_ahead;
+                    if (j + 1 < nb) term_ahead = term_of(block + 1);
                     mbar_arrive_warp(bar(P::bMask + t));
                     wait_for(P::bMask + t, gb & 1, 340 + t);
                     if (!ok) break;
