@@ -528,7 +528,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     }
                     if (!ok) return;
                     tc_fence_after();
-                    const int keys = min(kBN, (kend - s_block * kBN + 15) & ~15);   // in the MMA's steps of 16
+                    // In the MMA's steps of 16, or in whole chunks where a mask's terms are added to all
+                    // 32 columns of one (`fast` below): what no product has written may be a NaN, which
+                    // a term of -inf does not hide.
+                    constexpr int kRound = kMask == 1 ? 31 : 15;
+                    const int keys = min(kBN, (kend - s_block * kBN + kRound) & ~kRound);
                     const uint64_t kd = k_desc + static_cast<uint32_t>(s_slot * (P::kOperand >> 4));
                     const uint32_t idesc = instr_desc(keys, false);
                     if (d_steps == DP / 16 && keys == kBN) {
@@ -721,7 +725,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 // that is the same for all rows: the scores go into registers once, in straight-line code.
                 // Any other block (the diagonal, the last keys, a mask with a row per query) takes two
                 // loops over 32-column chunks: the first puts the finished logits back in their place.
-                // (Keys past the end of K are zeros from TMA; past a length they are anything.)
+                // (Keys past the end of K are zeros from TMA, and their scores too: the score product covers
+                // every chunk that is read. Past a length they are anything.)
                 const bool fast = kMask == 1 ? !p.causal && (lo >= kBN || (!p.cu_k && kend == p.sk)) && !idle : lo >= kBN && (kMask == 0 || kind == kNoEffect) && !idle;
                 uint4 held = make_uint4(0u, 0u, 0u, 0u);   // plan: this row's visibility bits
                 if (kMask == 2 && kind == kYesNo) held = tp.plan.bits[(piece0 + block) * 32 + lane];

@@ -99,3 +99,24 @@ def test_mask_strides(cuda):
     wide = torch.randn(2, 1, 150, 211, generator=torch.Generator().manual_seed(7)).to(torch.bfloat16)
     _check(cuda, q, k, v, mask=wide[..., 5:208])
     _check(cuda, q, k, v, mask=wide[..., :1])
+
+
+# A last block of 1 to 16 keys past a multiple of 32: the columns up to the next multiple belong to no
+# product of 16, and hold what the kernel before left in tensor memory.
+@pytest.mark.parametrize("d", [64, 80, 128])
+@pytest.mark.parametrize("sk", [1, 16, 77, 129, 240])
+def test_a_key_mask_reads_only_what_the_call_computed(cuda, sk, d):
+    g = torch.Generator().manual_seed(sk)
+    q, k, v = (x.to(cuda) for x in qkv(2, 37, 37, 500, sk, d, sk + d))
+    keep = torch.rand(2, 1, 1, sk, generator=g) > 0.3
+    keep[..., 0] = True
+    keep = keep.to(cuda)
+    # Every score of every SM's two tiles a NaN, and P over them where it shares their columns.
+    poison = [x.to(cuda) for x in qkv(1, 148, 148, 256, 128, 80, 1)]
+    poison[1][:] = math.nan
+    want, want_lse = ops.sdpa_forward(q, k, v, mask=keep)
+    assert rel(want, ao.ruler_dense(q.cpu(), k.cpu(), v.cpu(), mask=keep.cpu())) <= FWD_BOUND
+    for _ in range(3):
+        ops.sdpa_forward(*poison)
+        out, lse = ops.sdpa_forward(q, k, v, mask=keep)
+        assert torch.equal(out, want) and torch.equal(lse, want_lse)
