@@ -1096,7 +1096,7 @@ __global__ void __launch_bounds__(kPlanThreads) mask_plan_kernel(const AttnParam
     __shared__ uint32_t seen[kMaxPlanBlocks];   // per block: 1 floor, 2 zero, 4 anything else
     __shared__ int unsafe;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int g = blockIdx.x, plane = blockIdx.y;
+    const int plane = blockIdx.x, g = blockIdx.y;   // (x: there may be more planes than the 65,535 of y)
     const int pb = plane / m.heads, ph = plane - pb * m.heads;
     const int rr = threadIdx.x >> 5, lane = threadIdx.x & 31;   // row of the group, position in the row
     for (int i = threadIdx.x; i < m.blocks; i += kPlanThreads) seen[i] = 0;
@@ -1212,6 +1212,7 @@ int64_t plan_layout(const AttnParams& p, unsigned char* base, MaskPlan* m) {
     return active + kind + bits + values;
 }
 
+constexpr int64_t kMostTiles = 0x3fffffff;   // (query tile, head) pairs of a call
 constexpr int64_t kHeaderBytes = 256;   // {int32 next item, int32 producers finished}
 
 int sm_count() {
@@ -1256,6 +1257,9 @@ bool forward_pair_takes(const AttnParams& p) {
     // A plan covers the keys whatever a sequence's length, and 131,072 of them.
     if (mask_needs_plan(p) && (p.cu_q || p.key_lengths || p.sk > kMaxPlanBlocks * kBN)) return false;
     if (reinterpret_cast<uintptr_t>(p.out) & 15 || p.os[0] % 8 || p.os[1] % 8 || p.os[2] % 8) return false;
+    // Items are counted in int32; a plan has its 32-row groups in y of its grid.
+    if (static_cast<int64_t>((p.sq + kBM - 1) / kBM) * p.heads * p.batch > kMostTiles) return false;
+    if (mask_needs_plan(p) && (p.sq + 31) / 32 > 65535) return false;
     const int64_t tq = p.cu_q ? p.total_q : p.sq, tk = p.cu_q ? p.total_k : p.sk;
     const int64_t bq = p.cu_q ? 1 : p.batch;
     int64_t s[3];
@@ -1321,7 +1325,7 @@ int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_
     const int group = p.heads / p.kv_heads;
     const int q_tiles = (p.sq + kBM - 1) / kBM;
     const int64_t units = static_cast<int64_t>(q_tiles) * group * p.kv_heads * p.batch;   // (query tile, head)
-    if (units > 0x3fffffff) return fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 forward: too many query tiles");
+    if (units > kMostTiles) return fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 forward: too many query tiles");
     const int sms = sm_count();
     // Dual halves a tile's chain of blocks but adds a merge and doubles the items: it pays where
     // tiles would leave SMs without one. (Up to six tiles per SM it cost more than it gave: 16 x 16
@@ -1349,7 +1353,7 @@ int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_
         const bool vec = p.ms[3] == 1 && (reinterpret_cast<uintptr_t>(p.mask) % (4 * size)) == 0 && p.ms[0] % 4 == 0 && p.ms[1] % 4 == 0 && p.ms[2] % 4 == 0;
         auto plan = p.mask_dtype == KTT_B200_MASK_BOOL ? mask_plan_kernel<KTT_B200_MASK_BOOL> : p.mask_dtype == KTT_B200_MASK_BF16 ? mask_plan_kernel<KTT_B200_MASK_BF16>
                   : p.mask_dtype == KTT_B200_MASK_F16  ? mask_plan_kernel<KTT_B200_MASK_F16>  : mask_plan_kernel<KTT_B200_MASK_F32>;
-        if (int rc = launch_dependent(plan, dim3(m.groups, static_cast<unsigned>(planes)), kPlanThreads, 0, stream, "mask_plan launch", p, tp.plan,
+        if (int rc = launch_dependent(plan, dim3(static_cast<unsigned>(planes), m.groups), kPlanThreads, 0, stream, "mask_plan launch", p, tp.plan,
                                       static_cast<int32_t*>(workspace), vec)) return rc;
     }
     // K / V beyond what L2 keeps (126 MB on B200): the grouped order, which needs the counter.

@@ -120,3 +120,17 @@ def test_a_key_mask_reads_only_what_the_call_computed(cuda, sk, d):
         ops.sdpa_forward(*poison)
         out, lse = ops.sdpa_forward(q, k, v, mask=keep)
         assert torch.equal(out, want) and torch.equal(lse, want_lse)
+
+
+def test_more_mask_planes_than_a_grid_dimension(cuda):
+    # A mask of its own for each of 4,096 x 16 (batch, head) pairs (windows of a bitmap, one key apart).
+    g = torch.Generator(cuda).manual_seed(8)
+    q, k, v = (torch.randn(4096, 16, 200, 80, device=cuda, dtype=torch.bfloat16, generator=g) for _ in range(3))
+    bits = torch.rand(4096 + 16 * 4096 + 200 * 200, device=cuda, generator=g) > 0.4
+    mask = bits.as_strided((4096, 16, 200, 200), (1, 4096, 200, 1))
+    before = ktt.counters()["attention_flash"]
+    out, _ = ops.sdpa_forward(q, k, v, mask=mask)
+    assert ktt.counters()["attention_flash"] == before + 1
+    for b, h in ((0, 0), (2047, 15), (4095, 0), (4095, 14), (4095, 15)):
+        part = [x[b:b + 1, h:h + 1].cpu() for x in (q, k, v, mask)]
+        assert rel(out[b:b + 1, h:h + 1], ao.ruler_dense(*part[:3], mask=part[3])) <= FWD_BOUND
