@@ -844,7 +844,8 @@ Tensor offsets_to_device(const std::vector<int32_t>& cu_q, const std::vector<int
 
 // sdpa_varlen(q, k, v, cu_q, cu_k or None, max_q or None, max_k or None, is_causal, scale), offsets
 // on the host and no mask: the output, or None when the call is not one for the fast path
-// (offsets that break a rule among them: attention.check_offsets then says which).
+// (offsets that break a rule among them: attention.check_offsets then says which; a stream that
+// captures: torch then refuses the copy of the offsets).
 PyObject* py_sdpa_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     const Tensor *q, *k, *v;
@@ -858,6 +859,13 @@ PyObject* py_sdpa_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
         if (!plain(*t) || t->dim() != 3 || t->numel() == 0 || t->scalar_type() != at::kBFloat16 || t->device() != q->device()) Py_RETURN_NONE;
     }
     if (k->size(0) != v->size(0) || k->size(1) != v->size(1) || k->size(2) != q->size(2)) Py_RETURN_NONE;
+    {
+        // A captured copy would read the offsets again at every replay, long after this call's are gone.
+        c10::cuda::CUDAGuard device(q->device());
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        C10_CUDA_CHECK(cudaStreamIsCapturing(at::cuda::getCurrentCUDAStream(), &capture));
+        if (capture != cudaStreamCaptureStatusNone) Py_RETURN_NONE;
+    }
     const bool causal = args[7] == Py_True, same = !given_k || cq == ck;
     if (cq.size() != ck.size() || cq[0] != 0 || ck[0] != 0 || cq.back() != q->size(0) || ck.back() != k->size(0)) Py_RETURN_NONE;
     int32_t longest_q = 0, longest_k = 0;

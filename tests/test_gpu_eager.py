@@ -53,6 +53,20 @@ def test_packed(cuda, monkeypatch, kind):
     _same(*_both(monkeypatch, lambda: _with_grads(call, q, k, v)))
 
 
+@pytest.mark.parametrize("kind", ["list", "cpu"])
+def test_packed_offsets_on_the_host_are_refused_in_a_capture(cuda, kind):
+    # A replay would copy them from memory that is gone.
+    ends = torch.tensor([0, 1, 130, 300], dtype=torch.int32)
+    q, k, v = (x[0].transpose(0, 1).contiguous().to(cuda) for x in qkv(1, 4, 2, 300, 300, 64, 3))
+    want = ktt.sdpa_varlen(q, k, v, ends, is_causal=True)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="capture"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            ktt.sdpa_varlen(q, k, v, ends.tolist() if kind == "list" else ends, is_causal=True)
+    torch.cuda.synchronize()
+    assert torch.equal(ktt.sdpa_varlen(q, k, v, ends, is_causal=True), want)
+
+
 def test_decode_step(cuda, monkeypatch):
     q, k, v = (x.to(cuda) for x in qkv(3, 8, 2, 1, 200, 128, 4))
     kn, vn = k[:, :, :1] * 0.5, v[:, :, :1] * 0.5
