@@ -368,7 +368,13 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
                     float m_new = mm[u];
 #pragma unroll
                     for (int j = 0; j < kHolders; ++j) {
-                        if (c0 + j >= parts[u]) ms[u][j] = -INFINITY;
+                        if (c0 + j >= parts[u]) {
+                            // The values as well: their weight of 0 would make an infinity a NaN.
+                            // (A row sum is finite, or a NaN of the last holder's own. Predicated sums
+                            // instead: 35.3 -> 35.6 us on the batch above; a branch: 34.4 -> 35.1.)
+                            ms[u][j] = -INFINITY;
+                            v[u][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
                         m_new = fmaxf(m_new, ms[u][j]);
                     }
                     const float base_m = (m_new == -INFINITY) ? 0.f : m_new;

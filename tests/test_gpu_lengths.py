@@ -193,3 +193,15 @@ def test_decode_calls_of_different_shapes_share_one_scratch(cuda):
         n = torch.tensor(lengths, dtype=torch.int32, device=cuda)
         out, _ = ops.decode(q.to(cuda), k.to(cuda), v.to(cuda), key_lengths=n)
         assert rel(out, ao.ruler_lengths(q, k, v, lengths)) <= FWD_BOUND, (i, b, h)
+
+
+@pytest.mark.parametrize("n", [130, 700, 1100, 1500, 3000])   # 1 to 24 shares to a pair, four to a round of the merge
+def test_decode_merge_keeps_infinities(cuda, n):
+    q, k, v = qkv(1, 16, 2, 1, n, 128, n)
+    ruler = ao.ruler_lengths(q, k, v, [n])
+    v[0, :, 3, 5] = float("inf")
+    v[0, :, n - 1, 7] = float("-inf")
+    out = ktt.sdpa(q.to(cuda), k.to(cuda), v.to(cuda), key_lengths=[n]).cpu()
+    assert (out[..., 5] == float("inf")).all() and (out[..., 7] == float("-inf")).all()
+    rest = [c for c in range(128) if c not in (5, 7)]
+    assert rel(out[..., rest], ruler[..., rest]) <= FWD_BOUND
