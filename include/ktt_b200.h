@@ -54,6 +54,9 @@ enum {
     KTT_B200_KERNEL_TC5 = 2,  /* TMA + tcgen05/TMEM kernels: head dim 64 / 128 */
     KTT_B200_KERNEL_TC5_WIDE = 3,  /* forward only: the head-dim-128 tcgen05 kernel's design also at
                                       head dim 64, where KERNEL_TC5 picks the two-stream kernel */
+    KTT_B200_KERNEL_PAIR = 4,  /* forward only: the tcgen05 kernel of two query tiles per CTA also where
+                                  AUTO takes another one for faster; a mask with a row per query needs
+                                  its workspace */
 };
 
 /* One attention problem, dense ([B, H, S, D] with arbitrary batch/head/row strides, so

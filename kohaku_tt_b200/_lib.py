@@ -36,7 +36,7 @@ ERR_DEVICE_WAIT = -4
 
 MASK_NONE, MASK_BOOL, MASK_BF16, MASK_F32, MASK_F16 = range(5)
 CAUSAL_NONE, CAUSAL_TOP_LEFT, CAUSAL_BOTTOM_RIGHT = range(3)
-KERNEL_AUTO, KERNEL_MMA, KERNEL_TC5, KERNEL_TC5_WIDE = range(4)
+KERNEL_AUTO, KERNEL_MMA, KERNEL_TC5, KERNEL_TC5_WIDE, KERNEL_PAIR = range(5)
 
 EXPORTS = (
     "ktt_b200_abi_version",

@@ -285,6 +285,14 @@ extern "C" int ktt_b200_sdpa_supported(const ktt_b200_attn_args* a) {
             return 0;
         }
     }
+    if (a->kernel == KTT_B200_KERNEL_PAIR) {
+        AttnParams p;
+        to_params(a, p);
+        if (!forward_pair_takes(p)) {
+            fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 kernel of two tiles: head dims, strides or mask not taken");
+            return 0;
+        }
+    }
     return 1;
 }
 
@@ -316,7 +324,12 @@ extern "C" int ktt_b200_sdpa_forward(const ktt_b200_attn_args* a, void* stream) 
         note_call(4);
         return fail(KTT_B200_ERR_UNSUPPORTED, "sdpa_forward: tcgen05 kernel: %s", why);
     }
-    if (tc5 && a->kernel != KTT_B200_KERNEL_MMA && !(a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_preferred(p))) {
+    const bool wants_pair = a->kernel == KTT_B200_KERNEL_PAIR;
+    if (wants_pair && !forward_pair_takes(p)) {
+        note_call(4);
+        return fail(KTT_B200_ERR_UNSUPPORTED, "sdpa_forward: tcgen05 kernel of two tiles: head dims, strides or mask not taken");
+    }
+    if (tc5 && a->kernel != KTT_B200_KERNEL_MMA && !wants_pair && !(a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_preferred(p))) {
         note_call(0);
         const char* why_row = nullptr;
         if (a->kernel != KTT_B200_KERNEL_TC5_WIDE && forward_row_takes(p, &why_row)) {
@@ -332,8 +345,9 @@ extern "C" int ktt_b200_sdpa_forward(const ktt_b200_attn_args* a, void* stream) 
     }
     // What is left for AUTO: head dims those kernels are not built for, masks with a row per query
     // and calls in which this one is the faster. The masks need their workspace; a caller that
-    // brings none keeps the warp-MMA kernel.
-    if (a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_takes(p) && (!row_per_query(p) || a->workspace_bytes >= forward_pair_workspace(p))) {
+    // brings none keeps the warp-MMA kernel, and so do calls of few rows.
+    if (wants_pair || (a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_takes(p) && (tc5 || forward_pair_pays(p)) &&
+                       (!row_per_query(p) || a->workspace_bytes >= forward_pair_workspace(p)))) {
         note_call(0);
         return launch_forward_pair(p, a->workspace, a->workspace_bytes, st);
     }
@@ -350,8 +364,9 @@ extern "C" int64_t ktt_b200_sdpa_forward_workspace(const ktt_b200_attn_args* a) 
     AttnParams p;
     to_params(a, p);
     const char* why = nullptr;
-    if (forward_tc5_takes(p, &why)) return forward_row_workspace(p);   // the same 256 bytes for both
-    if (a->kernel == KTT_B200_KERNEL_AUTO && forward_pair_takes(p)) return forward_pair_workspace(p);
+    const bool wants_pair = a->kernel == KTT_B200_KERNEL_PAIR;
+    if (!wants_pair && forward_tc5_takes(p, &why)) return forward_row_workspace(p);   // the same 256 bytes for both
+    if ((wants_pair || a->kernel == KTT_B200_KERNEL_AUTO) && forward_pair_takes(p) && (wants_pair || forward_pair_pays(p))) return forward_pair_workspace(p);
     return 0;                                                          // the warp-MMA kernel has no use for one
 }
 

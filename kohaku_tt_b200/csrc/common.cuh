@@ -246,6 +246,7 @@ int forward_row_occupancy();
 // written by the call, which then clears the counter itself.
 bool forward_pair_takes(const AttnParams& p);
 bool forward_pair_preferred(const AttnParams& p);   // over the other tcgen05 kernels, where those take the call too
+bool forward_pair_pays(const AttnParams& p);        // over the warp-MMA kernel, where those do not
 int64_t forward_pair_workspace(const AttnParams& p);
 int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_bytes, cudaStream_t stream);
 // 0, or KTT_B200_ERR_DEVICE_WAIT with the code of the first wait that ran out (cleared).

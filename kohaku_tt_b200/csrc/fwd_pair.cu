@@ -1290,6 +1290,60 @@ bool forward_pair_preferred(const AttnParams& p) {
     return p.sk <= most && forward_pair_takes(p);
 }
 
+// Head dims and masks that only this kernel and the warp-MMA one take: this one unless the estimate below
+// has the other 10 % faster. This one has one CTA of two 128-row tiles per SM, and in front of a mask with
+// a row per query its plan; warp-MMA has four 64-row CTAs per SM. With few rows per (batch, head), or a
+// plan that few heads share, that is the better. Measured on B200, this kernel and warp-MMA, us:
+//   16 x 49 rows and keys, D 32            5.7    4.2     8,192 x 64, D 32                   173    86
+//   512 x 64, a bf16 mask each, D 32      61.3    9.4     8,192 x 64, a bf16 mask each, D 32 920   147
+//   2,048 x 64, D 80                      54     75       512 x 128, D 80                     19    54
+//   512 x 197, one bool mask, D 64        46    124       48 x 520, a bf16 mask each, D 64    85    74
+// The constants are fitted to 13,600 such pairs of times (2 to 3,000 rows, 8 to 2,500 keys, 1 to 65,000
+// (batch, head) pairs, every kind of mask, D 8 to 128): within 10 to 25 % rms of each side. On 1,213 fresh
+// sizes the choice is within 0.5 % of the better side on average, 36 % faster than always this kernel; at
+// worst 1.55 times the better side's time.
+bool forward_pair_pays(const AttnParams& p) {
+    // us. Warp-MMA, a 64-key block of a CTA, by padded head dim (32, 64, 128): when it runs alone on
+    // its SM, and its share of a full one (of the CTA, of 64 rows). This kernel, by padded head dim (64,
+    // 128): a call, an item, a 128-key block of it; a plan's CTA, four blocks of it.
+    // Masks: none, one row, bool, values.
+    struct Warp { float alone, cta, rows; };
+    static constexpr Warp kWarp[3][4] = {{{1.8f, 0.7f, 0.f}, {4.3f, 1.4f, 0.f}, {5.1f, 1.3f, 0.3f}, {5.8f, 1.2f, 1.f}},
+                                         {{3.2f, 1.2f, 0.f}, {5.7f, 1.8f, 0.f}, {6.2f, 1.6f, 0.5f}, {7.1f, 1.7f, 0.9f}},
+                                         {{4.5f, 2.7f, 0.5f}, {7.1f, 3.8f, 0.6f}, {7.6f, 3.6f, 1.3f}, {8.3f, 3.8f, 2.1f}}};
+    struct Pair { float call, item, block, plan, plan_blocks; };
+    static constexpr Pair kPair[2][4] = {{{3.1f, 1.7f, 1.6f, 0.f, 0.f}, {2.6f, 1.5f, 2.5f, 0.f, 0.f}, {4.1f, 3.8f, 1.4f, 1.2f, 3.7f}, {3.6f, 0.f, 5.5f, 0.f, 6.2f}},
+                                         {{3.5f, 1.5f, 2.5f, 0.f, 0.f}, {3.f, 1.6f, 3.1f, 0.f, 0.f}, {4.3f, 4.f, 2.1f, 1.4f, 3.7f}, {3.8f, 0.f, 6.6f, 0.f, 6.2f}}};
+    const bool planned = mask_needs_plan(p);
+    const int kind = p.mask_dtype == KTT_B200_MASK_NONE ? 0 : !planned ? 1 : p.mask_dtype == KTT_B200_MASK_BOOL ? 2 : 3;
+    const int dim = p.d > p.dv ? p.d : p.dv;
+    // (Packed: sequences of the average length.)
+    const int64_t sq = p.cu_q ? p.total_q / p.batch + 1 : p.sq, sk = p.cu_q ? p.total_k / p.batch + 1 : p.sk;
+    const int64_t group = p.heads / p.kv_heads, kv_pairs = static_cast<int64_t>(p.batch) * p.kv_heads;
+    const float sms = static_cast<float>(sm_count());
+
+    const int64_t warp_tiles = (sq + 63) / 64;
+    const Warp& w = kWarp[dim <= 32 ? 0 : dim <= 64 ? 1 : 2][kind];
+    const bool beyond_l2 = 2 * kv_pairs * (group * sq + sk) * (p.d + p.dv) > (96ll << 20);   // then its loads are what it waits for
+    const float share = (w.cta + w.rows * static_cast<float>(sq) / static_cast<float>(64 * warp_tiles)) * (beyond_l2 ? 1.4f : 1.f);
+    const float per_sm = ceilf(static_cast<float>(warp_tiles * group * kv_pairs) / sms), full = ceilf(per_sm / 4.f) - 1.f;
+    const float warp_us = 2.f + static_cast<float>((sk + 63) / 64) * (full * fmaxf(w.alone, 4.f * share) + fmaxf(w.alone, (per_sm - 4.f * full) * share));
+
+    auto rounds = [&](int64_t n) {   // of one per SM; uneven ones overlap
+        const float x = static_cast<float>(n) / sms;
+        return x <= 3.f ? ceilf(x) : x + 0.5f;
+    };
+    const Pair& c = kPair[dim <= 64 ? 0 : 1][kind];
+    const int64_t tiles = (sq + kBM - 1) / kBM * group, blocks = (sk + kBN - 1) / kBN;
+    const bool dual = sk > kBN && tiles * kv_pairs <= sm_count();
+    float pair_us = c.call + rounds((dual ? tiles : (tiles + 1) / 2) * kv_pairs) * (c.item + c.block * static_cast<float>(dual ? (blocks + 1) / 2 : blocks));
+    if (planned) {
+        const int64_t planes = static_cast<int64_t>(p.ms[0] ? p.batch : 1) * (p.ms[1] ? p.heads : 1);
+        pair_us += rounds(planes * ((sq + 31) / 32)) * (c.plan + c.plan_blocks * static_cast<float>((blocks + 3) / 4));
+    }
+    return warp_us > 0.9f * pair_us;
+}
+
 int64_t forward_pair_workspace(const AttnParams& p) {
     MaskPlan m;
     return kHeaderBytes + (mask_needs_plan(p) ? plan_layout(p, nullptr, &m) : 0);

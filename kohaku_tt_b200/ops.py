@@ -22,9 +22,10 @@ _MASK_DTYPES = {
 }
 
 # 'flash' = the TMA + tcgen05 kernels, 'flash_wide' = the head-dim-128 tcgen05 forward's design also
-# at head dim 64 (where 'flash' runs the two-stream kernel), 'mma' = warp MMA.
+# at head dim 64 (where 'flash' runs the two-stream kernel), 'flash_pair' = the tcgen05 forward of
+# two query tiles per CTA wherever it takes the call, 'mma' = warp MMA.
 _KERNELS = {"auto": _lib.KERNEL_AUTO, "mma": _lib.KERNEL_MMA, "flash": _lib.KERNEL_TC5,
-            "flash_wide": _lib.KERNEL_TC5_WIDE}
+            "flash_wide": _lib.KERNEL_TC5_WIDE, "flash_pair": _lib.KERNEL_PAIR}
 
 
 def _kernel_code(kernel):

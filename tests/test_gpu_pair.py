@@ -14,14 +14,14 @@ from tests.gpu_util import FWD_BOUND, LSE_RMS, qkv, rel, rms
 pytestmark = pytest.mark.gpu
 
 
-def _check(cuda, q, k, v, mask=None, causal=False, lengths=None):
-    before = ktt.counters()["attention_flash"]
+def _check(cuda, q, k, v, mask=None, causal=False, lengths=None, kernel="flash_pair", counted="attention_flash"):
+    before = ktt.counters()[counted]
     ln = None if lengths is None else torch.tensor(lengths, dtype=torch.int32, device=cuda)
     out, lse = ops.sdpa_forward(q.to(cuda), k.to(cuda), v.to(cuda), causal=causal, key_lengths=ln,
-                                mask=None if mask is None else mask.to(cuda))
+                                mask=None if mask is None else mask.to(cuda), kernel=kernel)
     torch.cuda.synchronize()
     _lib.device_status()
-    assert ktt.counters()["attention_flash"] == before + 1   # the tcgen05 kernel took it
+    assert ktt.counters()[counted] == before + 1   # the kernel that was meant took it
     if lengths is not None:
         ruler = ao.ruler_lengths(q, k, v, lengths)
     else:
@@ -51,7 +51,18 @@ def test_few_keys(cuda, h, sq, sk, d, masked):
     q, k, v = qkv(1, h, h, sq, sk, d, h + sq + sk)
     keep = torch.rand(1, 1, 1, sk, generator=torch.Generator().manual_seed(h)) > 0.3
     keep[..., 0] = True
-    _check(cuda, q, k, v, mask=keep if masked else None)
+    _check(cuda, q, k, v, mask=keep if masked else None, kernel="auto")
+
+
+# Few rows: the warp-MMA kernel, up to where the tiles fill (both sides of the line).
+@pytest.mark.parametrize("b,h,sq,sk,d,kind,kernel", [
+    (1, 1, 1, 1, 8, None, "mma"), (2, 16, 49, 49, 32, None, "mma"), (64, 16, 64, 64, 32, "bf16", "mma"),
+    (8, 16, 128, 128, 64, "values", "mma"), (2, 16, 16, 16, 80, None, "mma"), (1, 16, 64, 64, 64, "random", "mma"),
+    (2, 16, 144, 144, 32, None, "flash"), (2, 16, 128, 128, 80, None, "flash"), (8, 16, 197, 197, 64, "random", "flash"),
+])
+def test_few_rows(cuda, b, h, sq, sk, d, kind, kernel):
+    q, k, v = qkv(b, h, h, sq, sk, d, sq + sk + d)
+    _check(cuda, q, k, v, mask=_mask(kind, b, h, sq, sk) if kind else None, kernel="auto", counted="attention_" + kernel)
 
 
 def test_head_dim_80_with_key_lengths_and_a_key_mask(cuda):
@@ -114,11 +125,11 @@ def test_a_key_mask_reads_only_what_the_call_computed(cuda, sk, d):
     # Every score of every SM's two tiles a NaN, and P over them where it shares their columns.
     poison = [x.to(cuda) for x in qkv(1, 148, 148, 256, 128, 80, 1)]
     poison[1][:] = math.nan
-    want, want_lse = ops.sdpa_forward(q, k, v, mask=keep)
+    want, want_lse = ops.sdpa_forward(q, k, v, mask=keep, kernel="flash_pair")
     assert rel(want, ao.ruler_dense(q.cpu(), k.cpu(), v.cpu(), mask=keep.cpu())) <= FWD_BOUND
     for _ in range(3):
-        ops.sdpa_forward(*poison)
-        out, lse = ops.sdpa_forward(q, k, v, mask=keep)
+        ops.sdpa_forward(*poison, kernel="flash_pair")
+        out, lse = ops.sdpa_forward(q, k, v, mask=keep, kernel="flash_pair")
         assert torch.equal(out, want) and torch.equal(lse, want_lse)
 
 
@@ -128,9 +139,7 @@ def test_more_mask_planes_than_a_grid_dimension(cuda):
     q, k, v = (torch.randn(4096, 16, 200, 80, device=cuda, dtype=torch.bfloat16, generator=g) for _ in range(3))
     bits = torch.rand(4096 + 16 * 4096 + 200 * 200, device=cuda, generator=g) > 0.4
     mask = bits.as_strided((4096, 16, 200, 200), (1, 4096, 200, 1))
-    before = ktt.counters()["attention_flash"]
-    out, _ = ops.sdpa_forward(q, k, v, mask=mask)
-    assert ktt.counters()["attention_flash"] == before + 1
+    out, _ = ops.sdpa_forward(q, k, v, mask=mask, kernel="flash_pair")
     for b, h in ((0, 0), (2047, 15), (4095, 0), (4095, 14), (4095, 15)):
         part = [x[b:b + 1, h:h + 1].cpu() for x in (q, k, v, mask)]
         assert rel(out[b:b + 1, h:h + 1], ao.ruler_dense(*part[:3], mask=part[3])) <= FWD_BOUND
