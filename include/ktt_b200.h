@@ -123,8 +123,9 @@ typedef struct ktt_b200_attn_args {
      * that those in flight share the K / V of a few (batch, head) pairs (problems whose K / V
      * exceed L2 otherwise re-read them several times). The kernel leaves the counter zero;
      * calls that share a buffer must not overlap on the GPU. A mask with a row per query asks
-     * for more than 256 bytes: a plan of the mask, written by the call, which then also clears
-     * the counter itself (without it such a call runs on the warp-MMA kernel). The
+     * for more than 256 bytes, up to 1 GB: a plan of the mask or of as much of it as fits, written
+     * by the call, which then also clears the counter itself (without it such a call runs on the
+     * warp-MMA kernel). The
      * head-dim-128 kernel also takes 4 to 255 bytes: one int32 the caller zero-fills before EVERY call. */
     void* workspace;
     int64_t workspace_bytes;

@@ -1212,8 +1212,24 @@ int64_t plan_layout(const AttnParams& p, unsigned char* base, MaskPlan* m) {
     return active + kind + bits + values;
 }
 
-constexpr int64_t kMostTiles = 0x3fffffff;   // (query tile, head) pairs of a call
-constexpr int64_t kHeaderBytes = 256;   // {int32 next item, int32 producers finished}
+// A plan is written a part of the call at a time - batch entries, then heads, then query rows - so that it
+// takes at most this much memory however large the mask is.
+constexpr int64_t kMostPlan = 1ll << 30;
+struct PlanPart {
+    int batch, heads, rows;
+};
+
+int64_t plan_bytes(const AttnParams& p, const PlanPart& part) {
+    AttnParams s = p;
+    MaskPlan m;
+    s.batch = part.batch;
+    s.heads = part.heads;
+    s.sq = part.rows;
+    return plan_layout(s, nullptr, &m);
+}
+
+// The smallest part there is: a query tile of one plane.
+PlanPart least_part(const AttnParams& p) { return {p.ms[0] ? 1 : p.batch, p.ms[1] ? 1 : p.heads, p.sq < kBM ? p.sq : kBM}; }
 
 int sm_count() {
     static int sms[64] = {0};
@@ -1226,6 +1242,44 @@ int sm_count() {
     }
     return sms[dev];
 }
+
+// The parts to plan at a time so that a plan fits `room` bytes (or the smallest ones).
+PlanPart plan_part(const AttnParams& p, int64_t room) {
+    PlanPart part = {p.batch, p.heads, p.sq};
+    if (plan_bytes(p, part) <= room) return part;
+    auto cut = [&](int& n, int step) {
+        if (n <= step || plan_bytes(p, part) <= room) return;
+        const int64_t whole = n;
+        n = step;
+        int64_t fit = room / plan_bytes(p, part);   // steps (rounding makes several no larger than their sum)
+        if (fit < 1) fit = 1;
+        // Of the upper half of what fits, the size whose parts leave the fewest SMs idle: 32 heads of 4096 x
+        // 4096 fp32 terms, D 64, at 1 GB in parts of 11 heads 3,292 us, of 9 2,715 (whole 2,570).
+        float least = 0.f;
+        int64_t best = fit;
+        for (int i = 0; i < 16; ++i) {
+            const int64_t steps = fit - fit * i / 32;
+            n = static_cast<int>(steps * step < whole ? steps * step : whole);
+            const int64_t units = static_cast<int64_t>((part.rows + kBM - 1) / kBM) * part.heads * part.batch, sms = sm_count();
+            const float rounds = units <= sms && p.sk > kBN ? 0.5f : static_cast<float>((units + 2 * sms - 1) / (2 * sms));
+            const float cost = rounds * static_cast<float>((whole + n - 1) / n);
+            if (i == 0 || cost < least) {
+                least = cost;
+                best = n;
+            }
+        }
+        n = static_cast<int>(best);
+    };
+    const int group = p.heads / p.kv_heads;
+    if (p.ms[0]) cut(part.batch, 1);
+    if (p.ms[1]) cut(part.heads, group);
+    if (p.ms[1] && part.heads == group) cut(part.heads, 1);   // within the heads of one K / V head
+    cut(part.rows, kBM);
+    return part;
+}
+
+constexpr int64_t kMostTiles = 0x3fffffff;   // (query tile, head) pairs of a call
+constexpr int64_t kHeaderBytes = 256;   // {int32 next item, int32 producers finished}
 
 template <typename Kernel, typename... Args>
 int launch_dependent(Kernel kernel, dim3 grid, int threads, int smem, cudaStream_t stream, const char* what, Args... args) {
@@ -1345,11 +1399,12 @@ bool forward_pair_pays(const AttnParams& p) {
 }
 
 int64_t forward_pair_workspace(const AttnParams& p) {
-    MaskPlan m;
-    return kHeaderBytes + (mask_needs_plan(p) ? plan_layout(p, nullptr, &m) : 0);
+    return kHeaderBytes + (mask_needs_plan(p) ? plan_bytes(p, plan_part(p, kMostPlan)) : 0);
 }
 
-int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
+namespace {
+
+int launch_whole(const AttnParams& p, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
     const char* why = "";
     const int64_t tq = p.cu_q ? p.total_q : p.sq, tk = p.cu_q ? p.total_k : p.sk;
     const int64_t bq = p.cu_q ? 1 : p.batch;
@@ -1396,10 +1451,6 @@ int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_
     const bool planned = mask_needs_plan(p);
     const bool usable = workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
     if (planned) {
-        if (!usable || workspace_bytes < forward_pair_workspace(p)) {
-            return fail(KTT_B200_ERR_BAD_ARGUMENT, "tcgen05 forward: a mask with a row per query needs %lld bytes of workspace",
-                        static_cast<long long>(forward_pair_workspace(p)));
-        }
         plan_layout(p, static_cast<unsigned char*>(workspace) + kHeaderBytes, &tp.plan);
         const MaskPlan& m = tp.plan;
         const int64_t planes = static_cast<int64_t>(m.heads) * (m.batched ? p.batch : 1);
@@ -1424,6 +1475,45 @@ int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_
     const int grid = tp.work < sms ? tp.work : sms;
     if (p.d <= 64 && p.dv <= 64) return launch_pair<64>(p, maps, tp, grid, stream);
     return launch_pair<128>(p, maps, tp, grid, stream);
+}
+
+}  // namespace
+
+int launch_forward_pair(const AttnParams& p, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
+    if (!mask_needs_plan(p)) return launch_whole(p, workspace, workspace_bytes, stream);
+    const int64_t room = workspace_bytes - kHeaderBytes;
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 15) || room < plan_bytes(p, least_part(p))) {
+        return fail(KTT_B200_ERR_BAD_ARGUMENT, "tcgen05 forward: a mask with a row per query needs %lld bytes of workspace, 16-byte aligned",
+                    static_cast<long long>(forward_pair_workspace(p)));
+    }
+    // One part in nearly every call. The next one's plan waits for this one's attention, as it does for
+    // whatever is before it in the stream. (Causal calls take no mask: rows do not depend on the others.)
+    const PlanPart part = plan_part(p, room);
+    const int group = p.heads / p.kv_heads;
+    const int64_t size = p.mask_dtype == KTT_B200_MASK_BOOL ? 1 : p.mask_dtype == KTT_B200_MASK_F32 ? 4 : 2;
+    for (int b = 0; b < p.batch; b += part.batch) {
+        for (int h = 0, heads; h < p.heads; h += heads) {
+            heads = part.heads < p.heads - h ? part.heads : p.heads - h;
+            if (part.heads < group && heads > group - h % group) heads = group - h % group;
+            const int64_t hk = h / group;
+            for (int r = 0; r < p.sq; r += part.rows) {
+                AttnParams s = p;
+                s.batch = part.batch < p.batch - b ? part.batch : p.batch - b;
+                s.heads = heads;
+                s.kv_heads = heads < group ? 1 : heads / group;
+                s.sq = part.rows < p.sq - r ? part.rows : p.sq - r;
+                auto at = [&](const int64_t (&st)[3], int64_t head, int64_t row) { return b * st[0] + head * st[1] + row * st[2]; };
+                s.q += at(p.qs, h, r);
+                s.k += at(p.ks, hk, 0);
+                s.v += at(p.vs, hk, 0);
+                s.out += at(p.os, h, r);
+                if (s.lse) s.lse += at(p.ls, h, r);
+                s.mask = static_cast<const unsigned char*>(p.mask) + (b * p.ms[0] + h * p.ms[1] + r * p.ms[2]) * size;
+                if (int rc = launch_whole(s, workspace, workspace_bytes, stream)) return rc;
+            }
+        }
+    }
+    return 0;
 }
 
 }  // namespace ktt

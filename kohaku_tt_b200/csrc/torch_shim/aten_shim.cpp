@@ -197,13 +197,20 @@ ZeroedPool& decode_pool() {
 }
 
 // The tcgen05 forward's workspace. Without a mask that has a row per query it is the counter the
-// CTAs draw their tiles from, which the kernel leaves zero. A plan of such a mask is as large as
-// the mask and belongs to the call.
+// CTAs draw their tiles from, which the kernel leaves zero. A plan of such a mask is up to 1 GB and
+// belongs to the call; where the device has no room for it the call goes without, to a kernel that
+// reads the mask itself.
 constexpr int64_t kCounterBytes = 256;
 Tensor forward_workspace(const ktt_b200_attn_args& a, const Tensor& like, cudaStream_t stream) {
     const int64_t need = ktt_b200_sdpa_forward_workspace(&a);
     if (need <= 0) return Tensor();
-    if (need > kCounterBytes) return empty_cuda({need}, at::kByte, like);
+    if (need > kCounterBytes) {
+        try {
+            return empty_cuda({need}, at::kByte, like);
+        } catch (const c10::OutOfMemoryError&) {
+            return Tensor();
+        }
+    }
     return forward_pool().get(kCounterBytes, kCounterBytes, like, stream);
 }
 

@@ -148,13 +148,19 @@ def forward_workspace(args, device):
     """The tcgen05 forward's workspace, or None when the kernel that will run uses none. Without
     a mask that has a row per query that is the counter its CTAs draw their tiles from: one
     zero-filled buffer per (device, stream), which the kernel leaves zero, so it is filled
-    once. With such a mask the plan of the mask follows, as large as the mask; it belongs to
-    the call, which clears the counter in front of it itself."""
+    once. With such a mask the plan of the mask follows, up to 1 GB; it belongs to the call,
+    which clears the counter in front of it itself. Where the device has no room for it the
+    call goes without, to a kernel that reads the mask itself."""
     need = _lib.lib().ktt_b200_sdpa_forward_workspace(ctypes.byref(args))
     if need <= 0:
         return None
     if need > _COUNTER_BYTES:
-        buf = torch.empty((need,), dtype=torch.uint8, device=device)
+        try:
+            buf = torch.empty((need,), dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            if args.kernel != _lib.KERNEL_AUTO:
+                raise
+            return None
     else:
         key = (device.index, torch.cuda.current_stream(device).cuda_stream)
         buf = _FORWARD_WORKSPACE.get(key)

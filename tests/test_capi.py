@@ -107,3 +107,18 @@ def test_decode_refusals(built_lib):
     d.heads, d.d = 16, 96
     assert built_lib.ktt_b200_decode(ctypes.byref(d), None) == _lib.ERR_UNSUPPORTED
     assert "head dim 64 or 128" in _lib.last_error()
+
+
+def test_forward_workspace_is_bounded(built_lib):
+    # A mask with a row per query of 40 GB, and a plan of it: 1 GB and the counters.
+    a = _args(batch=16, heads=64, kv_heads=8, sq=4096, sk=4096, d=64, dv=64, mask=4096, mask_dtype=_lib.MASK_F32)
+    a.q = a.k = a.v = a.out = 4096
+    for name in ("q_strides", "out_strides"):
+        getattr(a, name)[:] = (64 * 4096 * 64, 4096 * 64, 64)
+    for name in ("k_strides", "v_strides"):
+        getattr(a, name)[:] = (8 * 4096 * 64, 4096 * 64, 64)
+    a.mask_strides[:] = (64 * 4096 * 4096, 4096 * 4096, 4096, 1)
+    assert 512 << 20 < built_lib.ktt_b200_sdpa_forward_workspace(ctypes.byref(a)) <= (1 << 30) + 256
+    a.sk = 131072   # one plane alone is 2 GB
+    a.mask_strides[:] = (0, 0, 131072, 1)
+    assert 512 << 20 < built_lib.ktt_b200_sdpa_forward_workspace(ctypes.byref(a)) <= (1 << 30) + 256

@@ -1,10 +1,12 @@
 """The forward kernel of two query tiles per CTA (csrc/fwd_pair.cu): head dims it zero-fills and
 masks with a row per query, at the edges of its tiles, against the float64 ruler."""
 
+import ctypes
 import math
 
 import pytest
 import torch
+import torch.nn.functional as F
 
 import kohaku_tt_b200 as ktt
 from kohaku_tt_b200 import _lib, ops
@@ -143,3 +145,56 @@ def test_more_mask_planes_than_a_grid_dimension(cuda):
     for b, h in ((0, 0), (2047, 15), (4095, 0), (4095, 14), (4095, 15)):
         part = [x[b:b + 1, h:h + 1].cpu() for x in (q, k, v, mask)]
         assert rel(out[b:b + 1, h:h + 1], ao.ruler_dense(*part[:3], mask=part[3])) <= FWD_BOUND
+
+
+# The plan of a mask a part of the call at a time: batch entries, K / V heads, heads of one, query rows
+# (the last of them a single one).
+@pytest.mark.parametrize("b,h,hk,sq,kind,parts", [
+    (3, 6, 2, 300, "values", 2), (3, 6, 2, 300, "values", 5), (3, 6, 2, 300, "values", 12), (3, 6, 2, 300, "values", 40),
+    (2, 4, 2, 257, "bf16", 4), (1, 4, 4, 257, "fp16", 8), (2, 2, 1, 257, "additive", 2), (2, 2, 1, 257, "causal", 2),
+])
+def test_parts_of_a_plan(cuda, monkeypatch, b, h, hk, sq, kind, parts):
+    sizes = []
+
+    def workspace(args, device):
+        whole = _lib.lib().ktt_b200_sdpa_forward_workspace(ctypes.byref(args))
+        buf = torch.empty(256 + (whole - 256) // parts, dtype=torch.uint8, device=device)
+        sizes.append(buf.numel())
+        args.workspace, args.workspace_bytes = buf.data_ptr(), buf.numel()
+        return buf
+
+    monkeypatch.setattr(ops, "forward_workspace", workspace)
+    _check(cuda, *qkv(b, h, hk, sq, 200, 64, sq + parts), mask=_mask(kind, b, h, sq, 200))
+    assert sizes
+
+
+def test_a_plan_takes_bounded_memory(cuda):
+    # 1.8 GB if it were whole; and none where the device has no room for it. (No cached segment is left
+    # that has room beside a tensor of this test.)
+    torch.cuda.empty_cache()
+    g = torch.Generator(cuda).manual_seed(3)
+    q, k, v = (torch.randn(128, 16, 400, 80, device=cuda, dtype=torch.bfloat16, generator=g) for _ in range(3))
+    bits = torch.randn(128 + 16 * 128 + 400 * 400, device=cuda, generator=g)
+    mask = bits.as_strided((128, 16, 400, 400), (1, 128, 400, 1))
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    counts = ktt.counters()
+    out, lse = ops.sdpa_forward(q, k, v, mask=mask)
+    assert ktt.counters()["attention_flash"] == counts["attention_flash"] + 1
+    results = out.numel() * 2 + lse.numel() * 4
+    assert torch.cuda.max_memory_allocated() - before <= results + (1025 << 20)
+    for b, h in ((0, 0), (63, 7), (127, 15)):
+        part = [x[b:b + 1, h:h + 1].cpu() for x in (q, k, v, mask)]
+        assert rel(out[b:b + 1, h:h + 1], ao.ruler_dense(*part[:3], mask=part[3])) <= FWD_BOUND
+    for call in (lambda: ops.sdpa_forward(q, k, v, mask=mask)[0], lambda: F.scaled_dot_product_attention(q, k, v, attn_mask=mask)):
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(cuda).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + results + (64 << 20)) / total)
+        counts = ktt.counters()
+        try:
+            again = call()
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        assert ktt.counters()["attention_mma"] == counts["attention_mma"] + 1
+        assert rel(again, out.cpu()) <= FWD_BOUND
+        del again
