@@ -1218,7 +1218,9 @@ int launch_bwd_rows(const AttnParams& p, cudaStream_t stream) {
     const int64_t ncounters = p.dkv_counters ? backward_counter_count(p, p.gsplit) : 0;
     const int padded = (p.sq + 127) / 128 * 128, rows = 256 / (D / 8);
     const int64_t ctas = static_cast<int64_t>(padded / rows) * p.heads * p.batch;
-    const int per = ctas >= 4 * 8 * 148 ? 4 : 1;   // eight CTAs of 256 threads fit an SM
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int per = ctas >= 4 * 8 * static_cast<int64_t>(sms) ? 4 : 1;   // eight CTAs of 256 threads fit an SM
     auto kernel = p.cu_q ? (per == 4 ? bwd_rows_kernel<D, 4, true> : bwd_rows_kernel<D, 1, true>)
                          : (per == 4 ? bwd_rows_kernel<D, 4, false> : bwd_rows_kernel<D, 1, false>);
     kernel<<<dim3(padded / (per * rows), p.heads, p.batch), 256, 0, stream>>>(p, ncounters);

@@ -1,7 +1,8 @@
 // Forward on the Blackwell tensor path for what the other two tcgen05 kernels are not built for -
-// head dims that are any multiple of 8 up to 128, and masks with a row per query - and for calls
-// of few keys in which it is the faster (forward_pair_preferred). TMA tile loads, tcgen05.mma with
-// accumulators in tensor memory, online softmax with one thread per query row.
+// head dims that are any multiple of 8 up to 128, and masks with a row per query, unless the rows are
+// so few that warp-MMA is the faster (forward_pair_pays) - and for calls of few keys in which it is
+// the faster (forward_pair_preferred). TMA tile loads, tcgen05.mma with accumulators in tensor memory,
+// online softmax with one thread per query row.
 //
 // A persistent CTA per SM works on two 128-row query tiles at a time, A and B:
 //
@@ -16,14 +17,13 @@
 //                      and V tiles
 //
 // An item of few blocks runs every role's code once or twice, so the code itself is what such
-// calls are bound by: a third of the instruction fetches miss the cache. Hence one copy of the item
+// calls are bound by: a third of the instruction fetches missed the cache. Hence one copy of the item
 // arithmetic (the producer's), short waits, and loops where a block is not the common one: 94 to
-// 150 KB of instructions became 79 to 105 (16 x 16 heads x 257 rows, D 80: 49 -> 42 us; 2 x 16
-// heads x 2048 x 2048, D 128, a mask of random values: 343 -> 278 us).
+// 150 KB of instructions became 79 to 105, and 16 x 16 heads x 257 rows, D 80, took 42 us where it had
+// taken 49 (a fifth of the fetches still miss there, a tenth on the masked call below).
 //
-// These calls ran on the warp-MMA kernel before (mma.sync, 64-row CTAs). Measured on B200: 16 x
-// 16 heads x 257 rows, D 80: 220 -> 42 us; 2 x 16 heads x 2048, D 64, a causal mask with padding
-// as a bf16 tensor: 577 -> 71 us.
+// Measured on B200, warp-MMA (mma.sync, 64-row CTAs) and this kernel: 16 x 16 heads x 257 rows, D 80,
+// 220 and 36 us; 2 x 16 heads x 2048, D 64, a causal mask with padding as a bf16 tensor, 577 and 57 us.
 //
 // Tensor memory (512 columns): S_A, S_B (128 each); head dims up to 64: P_A, P_B (64 each) and
 // O_A, O_B (64 each), so that the next scores can be computed while P V still reads P; up to 128:
@@ -52,8 +52,6 @@
 // host-visible status word, stops waiting everywhere, frees its tensor memory and exits.
 // Launched with programmatic stream serialization: everything before `griddepcontrol.wait`
 // may overlap the tail of the previous kernel in the stream.
-#include <cstdlib>
-
 #include "tc5.cuh"
 
 namespace ktt {
@@ -93,8 +91,10 @@ struct PairPlan {
     static constexpr int kPStep = kPOverS ? 128 : 64; // from P_A to P_B
     static constexpr int kO = kPOverS ? 256 : 384;    // + DP per tile
     static_assert(kO + 2 * DP <= 512, "tensor memory columns");
-    // Exponentials per 8 pairs that take the FMA-pipe polynomial instead of MUFU.
-    static constexpr int kPolyPairs = 2;   // measured: 0, 1, 2, 3 of 8 take 161, 153, 151, 153 us on 2 x 10 heads x 4096
+    // Exponentials per 8 pairs that take the FMA-pipe polynomial instead of MUFU. Measured, 0, 1, 2, 3
+    // of 8: 36.4, 36.6, 36.1, 37.5 us on 16 x 16 heads x 257, D 80; 57.2, 56.8, 56.9, 58.4 us on 2 x 16
+    // heads x 2048, D 64, a causal mask.
+    static constexpr int kPolyPairs = 2;
     // barriers (8 bytes each); "+ t": tile
     static constexpr int bQFull = 0;                   // + t
     static constexpr int bQFree = 2;                   // + t
@@ -152,10 +152,10 @@ struct alignas(16) Item {
 };
 static_assert(sizeof(Item) <= 96, "the queue's slots");
 
-// Items of one (batch, K / V head) are neighbours in its list of (query tile, head), longest
-// causal tiles first (else first rows first: a last tile of few rows is then the one without a
-// partner, and its item the short one), heads fastest. Two orders of the items: with the level slowest every deal
-// in rounds hands out similar lengths; `grouped` (needs the counter) keeps all items of one
+// Items of one (batch, K / V head) are neighbours in its list of (query tile, head), last rows first
+// (the longest of a causal call), heads fastest; of an odd number of tiles it is the first rows' that
+// has no partner. Two orders of the items: with the level slowest every deal in rounds hands out
+// similar lengths; `grouped` (needs the counter) keeps all items of one
 // (batch, K / V head) together, so that the items in flight share the K / V of a few heads in L2
 // (measured on a packed 65,536-token batch with 537 MB of K / V: 4.85 -> 0.81 GB of DRAM reads).
 __device__ __forceinline__ Item decode_item(const PairParams& tp, int w) {
@@ -1047,11 +1047,14 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
 // ---- masks with a row per query ----------------------------------------------------------
 //
 // One CTA per 32 query rows of a plane walks the keys once, a warp per row, four blocks of 128
-// keys at a time. It is bound by reading the mask once; pieces without values to apply cost
-// nothing further, and what the attention kernel reads back is the bits or values of the pieces
-// that have any. The code is kept small (a type per instance, one row per warp): with four rows
-// per warp and the type looked up per load it was 85 to 106 KB of straight-line instructions that
-// every pass fetched again. A call with 2 x 2048 x 2048 bf16 terms (2 x 16 heads, D 64): 103 -> 75 us.
+// keys at a time. It is not bound by reading the mask once (2 x 2048 x 2048 bf16 terms: 2.6 us of the
+// copy bandwidth; DRAM 12 % busy) but by what it does per term in the few CTAs there are: the ALU
+// pipes of 128 SMs are 71 % busy, and each of four rounds ends at a barrier (16.7 us under ncu with
+// cold caches, about 8 in a stream). Pieces without values to apply cost nothing further, and what
+// the attention kernel reads back is the bits or values of the pieces that have any. The code is kept
+// small (a type per instance, one row per warp): with four rows per warp and the type looked up per
+// load it was 85 to 106 KB of straight-line instructions that every pass fetched again; that call (2 x
+// 16 heads, D 64) 103 -> 75 us.
 //
 // A block is hidden from a group when every term of it is at the floor (-5e5): its weights are
 // exactly 0 as long as each row of the group keeps a key well above the floor. A group with a
@@ -1437,9 +1440,9 @@ int launch_whole(const AttnParams& p, void* workspace, int64_t workspace_bytes, 
     if (units > kMostTiles) return fail(KTT_B200_ERR_UNSUPPORTED, "tcgen05 forward: too many query tiles");
     const int sms = sm_count();
     // Dual halves a tile's chain of blocks but adds a merge and doubles the items: it pays where
-    // tiles would leave SMs without one. (Up to six tiles per SM it cost more than it gave: 16 x 16
-    // heads x 257, D 80: 43 -> 37 us without it, 4 x 16 heads 19 -> 13; 2 x 16 heads x 2048, D 64,
-    // causal mask: 71 -> 58. At 8 heads x 2 x 1024, D 80, 128 tiles, it gives 25 -> 16.)
+    // tiles would leave SMs without one. (Up to six tiles per SM it cost more than it gave, when it was
+    // tried: 16 x 16 heads x 257, D 80: 43 -> 37 us without it, 4 x 16 heads 19 -> 13; 2 x 16 heads x
+    // 2048, D 64, causal mask: 71 -> 58. At 8 heads x 2 x 1024, D 80, 128 tiles, it gives 25 -> 16.)
     tp.dual = p.sk > kBN && units <= sms ? 1 : 0;
     const int levels = tp.dual ? q_tiles * group : (q_tiles * group + 1) / 2;
     tp.work = levels * p.kv_heads * p.batch;
