@@ -164,8 +164,12 @@ def test_parts_of_a_plan(cuda, monkeypatch, b, h, hk, sq, kind, parts):
         return buf
 
     monkeypatch.setattr(ops, "forward_workspace", workspace)
-    _check(cuda, *qkv(b, h, hk, sq, 200, 64, sq + parts), mask=_mask(kind, b, h, sq, 200))
-    assert sizes
+    operands = qkv(b, h, hk, sq, 200, 64, sq + parts)
+    _check(cuda, *operands, mask=_mask(kind, b, h, sq, 200))
+    # Head views of [B, S, H * D], a mask whose rows are a slice of wider ones.
+    views = [x.transpose(1, 2).contiguous().transpose(1, 2) for x in operands]
+    _check(cuda, *views, mask=_mask(kind, b, h, sq, 211)[..., :200])
+    assert len(sizes) == 2
 
 
 def test_a_plan_takes_bounded_memory(cuda):
