@@ -11,6 +11,7 @@
 //                      to tensor memory and rescales O only when the maximum moved by more than
 //                      2^8 (the lazy rescale of ktt_flash/compute.cpp, flash.md "row reference").
 //                      No two threads ever exchange anything inside the loop.
+//                      (kTurns: its exponentials in turn with the same warp of the other tile)
 //   warps 8, 9         issue S = Q K^T and O += P V (P read from tensor memory) of A and of B: while
 //                      one tile is in its exponentials the tensor core serves the other
 //   warp 10            draws the work and hands the items round, TMA loads of Q and of a ring of K
@@ -107,7 +108,8 @@ struct PairPlan {
     static constexpr int bWorkFree = bWorkFull + kQueue;   // + queue slot
     static constexpr int bMask = bWorkFree + kQueue;   // + t: the block's mask terms are written
     static constexpr int bPartial = bMask + 2;         // dual: B's half is final
-    static constexpr int bKVFull = bPartial + 1;       // + ring slot
+    static constexpr int bTurn = bPartial + 1;         // + 4 t + warp: the other tile's warp of this scheduler has had its turn
+    static constexpr int bKVFull = bTurn + 8;          // + ring slot
     static constexpr int bKVEmpty = bKVFull + kSlots;  // + ring slot
     static constexpr int bCount = bKVEmpty + kSlots;
     static_assert(bCount * 8 + 32 <= kBarBytes, "barrier area");
@@ -293,7 +295,10 @@ __device__ __forceinline__ bool wait_one(uint32_t b, uint32_t par, volatile int*
 // ---- the kernel ------------------------------------------------------------------------
 
 // kMask: 0 none, 1 a row per (batch, head), 2 a plan (a row per query).
-template <int DP, int kMask>
+// kTurns: where P overwrites the scores a tile's products and its softmax are one chain, and two tiles that
+// run in step wait for the tensor cores at the same time and then for the exponentials. Taking turns at the
+// exponentials, the products of one run under those of the other.
+template <int DP, int kMask, bool kTurns>
 __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const PairParams tp) {
@@ -643,6 +648,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
         bool ok = true;
         auto wait_for = [&](int b, int parity, int code) { ok = ok && wait_one(bar(b), parity, abort_flag, code); };
         const float sc = p.scale_log2;
+        int turns = 0;      // turns taken so far, the same number by either tile
+        const uint32_t my_turn = bar(P::bTurn + t * 4 + (warp & 3)), their_turn = bar(P::bTurn + (1 - t) * 4 + (warp & 3));
 
         for (int n = 0; ok; ++n) {
             Item k;
@@ -652,6 +659,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 continue;
             }
             // (Selected once: an index that is not a constant would put the item into memory.)
+            const int taking = kTurns ? k.n[1] : 0;   // the blocks both tiles have: B has no more than A
             const int nb = t ? k.n[1] : k.n[0], h = t ? k.h[1] : k.h[0], q0 = t ? k.q0[1] : k.q0[0], kend = t ? k.kend[1] : k.kend[0];
             const int qi = q0 + row;                    // row inside the sequence
             const bool real = qi < k.si.lq;
@@ -860,6 +868,15 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 }
                 const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
 
+                // Tile A goes first: its turn follows B's block before, B's follows A's same block.
+                if (kTurns && (t ? taking > 0 : taking > 0 && j <= taking && turns + j > 0)) {
+                    ok = ok && wait_one(my_turn, (turns + j - 1 + t) & 1, abort_flag, 390 + t);
+                    if (!ok) break;
+                }
+                auto end_turn = [&]() {
+                    if (kTurns && j < taking && lane == 0) mbar_arrive(their_turn);
+                };
+
                 // ---- P = 2^(logit - m) as packed bf16 pairs ----
                 const float2 sc2 = make_float2(fs, fs), nm2 = make_float2(-m_use, -m_use);
                 // P's columns are free once the previous block's P V has read them.
@@ -891,6 +908,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                             wv[e] = pack_bf16(pr.x, pr.y);
                         }
                         if (c == 0) wait_p_free();
+                        if (c == 2) end_turn();   // (the rest of this block runs beside the other's start)
                         tmem_st16(p_addr + c * 16, wv);
                         if (P::kPOverS && (c == 1 || (kMask == 1 && c == 0 && stored == 1))) {
                             // P V may start on the first half of the keys.
@@ -923,6 +941,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                         }
                         tmem_st16(p_addr + c * 16, wv);
                     }
+                    end_turn();
                     tmem_wait_st();
                     tc_fence_before();
                     mbar_arrive_warp(bar(P::kPOverS ? P::bPFull + 2 * t : P::bSFree + t));
@@ -940,6 +959,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             const int nb_other = e->n[1], e_b = e->b, e_h = e->h[dual ? 0 : t], e_q0 = e->q0[dual ? 0 : t], e_lq = e->si.lq, e_off = e->si.q_off;
             const int last = blk + nb - 1;
             blk += nb;
+            turns += taking;
             float l_row = (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y), m_row = m_ref;
             float f_mine = 1.f, f_other = 0.f;
             const bool merge = dual && nb_other > 0;
@@ -1302,7 +1322,15 @@ int launch_dependent(Kernel kernel, dim3 grid, int threads, int smem, cudaStream
 template <int DP>
 int launch_pair(const AttnParams& p, const CUtensorMap (&maps)[3], PairParams& tp, int grid, cudaStream_t stream) {
     using P = PairPlan<DP>;
-    auto kernel = p.mask_dtype == KTT_B200_MASK_NONE ? fwd_pair_kernel<DP, 0> : mask_needs_plan(p) ? fwd_pair_kernel<DP, 2> : fwd_pair_kernel<DP, 1>;
+    auto kernel = mask_needs_plan(p) ? fwd_pair_kernel<DP, 2, false> : p.mask_dtype != KTT_B200_MASK_NONE ? fwd_pair_kernel<DP, 1, false> : fwd_pair_kernel<DP, 0, false>;
+    if constexpr (P::kPOverS) {
+        // Turns, without a mask, from five blocks of keys on: with three, their waits and the code for them
+        // weigh more. Measured, us without and with: D 80, 16 heads x 4096 167 -> 153; D 96, 48 x 1025 52.5 ->
+        // 49.3; D 80, 32 x 2048 causal 46.9 -> 45.0; 128 x 577 44.4 -> 43.3, 128 x 640 42.3 -> 40.4; but 256 x
+        // 257 34.9 -> 35.9, D 128, 10 x 2048 queries x 300 keys 12.7 -> 13.4. (Head dims up to 64, whose scores
+        // are ready in any case: 157 both, 20 x 4096. Masks with a row per query, D 128, 32 x 2048: 68.7 -> 71.1.)
+        if (p.mask_dtype == KTT_B200_MASK_NONE && p.sk > 4 * kBN) kernel = fwd_pair_kernel<DP, 0, true>;
+    }
     if (int rc = ensure_smem(kernel, P::kBytes, "cudaFuncSetAttribute(fwd_pair)")) return rc;
     return launch_dependent(kernel, dim3(grid), kPairThreads, P::kBytes, stream, "fwd_pair launch", maps[0], maps[1], maps[2], tp);
 }

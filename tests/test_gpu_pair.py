@@ -43,6 +43,24 @@ def test_head_dims(cuda, b, h, hk, sq, sk, d, dv, causal):
     _check(cuda, *qkv(b, h, hk, sq, sk, d, sq + sk + d, dv=dv), causal=causal)
 
 
+# The tiles of a CTA take turns from five blocks of keys on: both sides of that line, tiles of unequal
+# length and items in which the second tile has no block or is not there.
+@pytest.mark.parametrize("b,h,hk,sq,sk,d,causal,lengths", [
+    (2, 75, 75, 256, 512, 80, False, None), (2, 75, 75, 256, 513, 80, False, None), (1, 101, 101, 257, 700, 96, True, None),
+    (1, 30, 10, 700, 640, 72, True, None), (3, 50, 50, 129, 1100, 128, False, [1100, 1, 515]), (2, 40, 20, 520, 900, 120, True, [900, 130]),
+])
+def test_turns(cuda, b, h, hk, sq, sk, d, causal, lengths):
+    q, k, v = qkv(b, h, hk, sq, sk, d, sq + sk + d)
+    if lengths is not None and causal:   # (the ruler for lengths is not causal: the plain one on each sequence)
+        out, _ = ops.sdpa_forward(q.to(cuda), k.to(cuda), v.to(cuda), causal=True, kernel="flash_pair",
+                                  key_lengths=torch.tensor(lengths, dtype=torch.int32, device=cuda))
+        for i, n in enumerate(lengths):
+            one = ao.ruler_dense(q[i:i + 1], k[i:i + 1, :, :n], v[i:i + 1, :, :n], causal=True)
+            assert rel(out[i:i + 1], one) <= FWD_BOUND
+        return
+    _check(cuda, q, k, v, causal=causal, lengths=lengths)
+
+
 # Calls that other kernels take too: just inside and outside the rounds, tiles and keys between them.
 @pytest.mark.parametrize("h,sq,sk,d,masked", [
     (37, 512, 96, 64, True), (38, 400, 77, 64, True), (148, 256, 40, 64, False), (50, 300, 320, 64, True),
