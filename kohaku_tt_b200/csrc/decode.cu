@@ -21,7 +21,10 @@
 //             pair's partials (fixed order: deterministic), writes bf16 and puts the
 //             counter back to zero.
 //
-// Scratch: 1024 int32 ticket counters that must be zero before the first call (the kernel
+// Where the pairs are few enough for a cluster of one to eight CTAs each (decode_ranks), none of that is needed:
+// the CTAs of a cluster take the pair's tiles in turn and add their partials up through shared memory.
+//
+// Scratch (shares only): 1024 int32 ticket counters that must be zero before the first call (the kernel
 // leaves them zero), then per slot 16 maxima, 16 sums and 16 x D partial outputs. A pair
 // that spans several CTAs is the last pair of the first of them, so that CTA's index names
 // its counter: the counter area has one size whatever the batch, and calls of different
@@ -29,6 +32,7 @@
 //
 // Semantics are kohakutt.sdpa(q, k, v, key_lengths=) (attention.py:10-23): keys at or past
 // a length contribute nothing, whatever they hold; lengths are clamped to [1, Sk].
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -61,6 +65,7 @@ struct DecodeParams {
     int rope_by_position;
     int32_t* lengths_out;
     long long* trace;   // optional (ktt_b200_set_trace): per CTA, nanosecond stamps of its phases
+    int ranks;          // CTAs of a cluster, which share one pair (decode_kernel<.., true>)
 };
 
 namespace {
@@ -215,7 +220,32 @@ __device__ __forceinline__ int swz(int row, int col) {
     return (row * D + ((((col >> 3) ^ (row & 7))) << 3) + (col & 7)) * 2;
 }
 
-template <int D, int NS, bool kAppend>
+// The CTAs of a cluster meet; what each wrote to its shared memory before is visible to the others after.
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of `addr` (shared memory of this CTA) in CTA `rank` of the cluster, and loads from there.
+__device__ __forceinline__ uint32_t in_rank(uint32_t addr, int rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+// kCluster: a cluster of p.ranks CTAs per (batch, kv head) pair (decode_ranks), rank r of which takes tiles r,
+// r + ranks, ... of it. Which tiles those are does not depend on the length, so the first ones are requested
+// together with it, and the ranks' partials meet in shared memory instead of behind a ticket in L2.
+template <int D, int NS, bool kAppend, bool kCluster>
 __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams p) {
     constexpr int kStage = 2 * kTile * D * 2;  // K then V, bytes
     extern __shared__ __align__(128) unsigned char smem[];
@@ -227,6 +257,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
     int* prefix_s = reinterpret_cast<int*>(fin_l + 16);         // [kMaxBatch + 1]
     int* lens_s = prefix_s + kMaxBatch + 1;                     // [kMaxBatch] clamped lengths
     int* misc = lens_s + kMaxBatch;                       // [8] warp sums, then the pending list
+    float* part_s = reinterpret_cast<float*>(misc + 8 + 6 * kMaxPending + 3);   // kCluster: [16][D] this CTA's partial
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -255,22 +286,37 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     stamp(1);
 
-    scan_lengths<kAppend>(p, prefix_s, lens_s, misc);
-    stamp(2);
-    if (kAppend && blockIdx.x == 0 && p.lengths_out) {
-        for (int b = threadIdx.x; b < p.batch; b += kThreads) p.lengths_out[b] = lens_s[b];
-    }
-    // Equal shares of units; this CTA streams the tiles whose unit lies in its share.
-    const int total = p.kv_heads * prefix_s[p.batch];
-    const int upc = max(static_cast<int>((total + gridDim.x - 1) / gridDim.x), kMinUnits);
-    const int first_unit = min(static_cast<int>(blockIdx.x) * upc, total), end_unit = min(first_unit + upc, total);
-    const int u0 = 0;
-    const int u1 = tiles_before(p, prefix_s, end_unit) - tiles_before(p, prefix_s, first_unit);
-    if (u1 <= 0) return;
-
+    // What this CTA streams: tiles [0, u1) of a walk that starts at `cons`.
     Cursor prod, cons;
-    cursor_seek(p, prefix_s, lens_s, cons, first_unit);
+    int u1, upc = 0, rank = 0;
+    const int u0 = 0;
+    if constexpr (kCluster) {
+        const int pair = static_cast<int>(blockIdx.x) / p.ranks;
+        rank = static_cast<int>(blockIdx.x) - pair * p.ranks;
+        cons.b = pair / p.kv_heads;
+        cons.hk = pair - cons.b * p.kv_heads;
+        cons.tile = rank;
+        cons.len = p.sk;   // what there is in memory, until the length is known
+        u1 = NS;
+    } else {
+        scan_lengths<kAppend>(p, prefix_s, lens_s, misc);
+        stamp(2);
+        if (kAppend && blockIdx.x == 0 && p.lengths_out) {
+            for (int b = threadIdx.x; b < p.batch; b += kThreads) p.lengths_out[b] = lens_s[b];
+        }
+        // Equal shares of units; this CTA streams the tiles whose unit lies in its share.
+        const int total = p.kv_heads * prefix_s[p.batch];
+        upc = max(static_cast<int>((total + gridDim.x - 1) / gridDim.x), kMinUnits);
+        const int first_unit = min(static_cast<int>(blockIdx.x) * upc, total), end_unit = min(first_unit + upc, total);
+        u1 = tiles_before(p, prefix_s, end_unit) - tiles_before(p, prefix_s, first_unit);
+        if (u1 <= 0) return;
+        cursor_seek(p, prefix_s, lens_s, cons, first_unit);
+    }
     prod = cons;
+    auto next = [&](Cursor& c) {
+        if constexpr (kCluster) c.tile += p.ranks;
+        else cursor_next(p, prefix_s, lens_s, c);
+    };
 
     // One normalised output row chunk (4 columns) of (batch b, kv head hk, tile row r).
     auto write_row = [&](int b, int hk, int r, int c4, float4 sum, float mm, float ll) {
@@ -429,12 +475,20 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
     int up = u0;
 #pragma unroll
     for (int s = 0; s < NS - 1; ++s) {
-        if (up < u1) {
+        if (kCluster ? prod.tile * kTile < p.sk : up < u1) {
             issue(prod, s);
-            cursor_next(p, prefix_s, lens_s, prod);
+            next(prod);
             ++up;
         }
         cp_async_commit();
+    }
+    if constexpr (kCluster) {
+        cons.len = clamp_len<kAppend>(p, cons.b);
+        prod.len = cons.len;
+        cons.ntiles = (cons.len + kTile - 1) / kTile;
+        u1 = cons.ntiles > rank ? (cons.ntiles - rank + p.ranks - 1) / p.ranks : 0;
+        if (kAppend && p.lengths_out && rank == 0 && cons.hk == 0 && threadIdx.x == 0) p.lengths_out[cons.b] = cons.len;
+        stamp(2);
     }
 
     uint32_t qa[D / 16][4];
@@ -448,7 +502,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
         // Refill the stage consumed in the previous iteration.
         if (up < u1) {
             issue(prod, (up - u0) % NS);
-            cursor_next(p, prefix_s, lens_s, prod);
+            next(prod);
             ++up;
         }
         cp_async_commit();
@@ -533,6 +587,16 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
         }
 
         const int j0 = cons.tile * kTile + warp * 16;
+        if (kCluster && j0 < cons.len && cons.len < j0 + 16) {
+            // Rows past the length that were requested before it was known: whatever the cache holds there
+            // times a weight of 0 must be 0. (Their scores are replaced.)
+            unsigned char* sV = ring + st * kStage + kTile * D * 2;
+            for (int idx = lane; idx < (j0 + 16 - cons.len) * (D / 8); idx += 32) {
+                const int r = cons.len - cons.tile * kTile + idx / (D / 8);
+                *reinterpret_cast<uint4*>(sV + swz<D>(r, (idx % (D / 8)) * 8)) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            __syncwarp();
+        }
         if (j0 < cons.len) {
             const unsigned char* sK = ring + st * kStage;
             const unsigned char* sV = sK + kTile * D * 2;
@@ -603,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
         }
         __syncwarp();  // all lanes are done with stage `st` before it is refilled
 
-        const bool last_of_pair = cons.tile + 1 == cons.ntiles;
+        const bool last_of_pair = !kCluster && cons.tile + 1 == cons.ntiles;
         if (last_of_pair || u + 1 == u1) {
             const long long fin_t0 = p.trace ? clock64() : 0;
             // Merge the four warps' states in a fixed order (deterministic).
@@ -664,6 +728,12 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
                 return sum;
             };
 
+            if constexpr (kCluster) {
+                for (int idx = threadIdx.x; idx < rows * (D / 4); idx += kThreads) {
+                    reinterpret_cast<float4*>(part_s)[idx] = merged(idx / (D / 4), idx % (D / 4));
+                }
+                break;
+            }
             // Which CTAs hold a piece of this pair?
             const int pair = cons.b * p.kv_heads + cons.hk;
             const int t0 = p.kv_heads * prefix_s[cons.b] + cons.hk * (cons.ntiles + kPairCost);   // the pair's first unit
@@ -700,38 +770,107 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
             fresh = true;
             if (p.trace && threadIdx.x == 0 && blockIdx.x < 1024) p.trace[(64 + blockIdx.x) * 8 + 7] += clock64() - fin_t0;
         }
-        cursor_next(p, prefix_s, lens_s, cons);
+        next(cons);
     }
     cp_async_wait<0>();
-    __syncthreads();
-    stamp(4);
-    if (npend_s[0] > 0) draw_tickets();
+    if constexpr (kCluster) {
+        stamp(4);
+        cluster_meet();
+        // Every rank adds up its share of the output: the partials of the ranks that had a tile, in their order
+        // (deterministic), eight at a time and all of them requested at once.
+        const int parts = min(cons.ntiles, p.ranks), all = rows * (D / 4), share = (all + p.ranks - 1) / p.ranks;
+        const uint32_t at_m = smem_u32(fin_m), at_l = smem_u32(fin_l), at_o = smem_u32(part_s);
+        for (int idx = rank * share + threadIdx.x; idx < min((rank + 1) * share, all); idx += kThreads) {
+            const int r = idx / (D / 4), c4 = idx % (D / 4);
+            float mm = -INFINITY, ll = 0.f;
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c0 = 0; c0 < parts; c0 += 8) {
+                float ms[8], ls[8];
+                float4 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int from = min(c0 + j, parts - 1);   // (past the last one a repeat, not used)
+                    ms[j] = ld_cluster(in_rank(at_m + r * 4, from));
+                    ls[j] = ld_cluster(in_rank(at_l + r * 4, from));
+                    v[j] = ld_cluster4(in_rank(at_o + idx * 16, from));
+                }
+                float m_new = mm;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (c0 + j < parts) m_new = fmaxf(m_new, ms[j]);
+                }
+                const float base = (m_new == -INFINITY) ? 0.f : m_new;
+                const float fa = fast_exp2(mm - base);
+                mm = m_new;
+                ll *= fa;
+                sum.x *= fa;
+                sum.y *= fa;
+                sum.z *= fa;
+                sum.w *= fa;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (c0 + j >= parts) continue;
+                    const float fb = fast_exp2(ms[j] - base);
+                    ll = fmaf(ls[j], fb, ll);
+                    sum.x = fmaf(v[j].x, fb, sum.x);
+                    sum.y = fmaf(v[j].y, fb, sum.y);
+                    sum.z = fmaf(v[j].z, fb, sum.z);
+                    sum.w = fmaf(v[j].w, fb, sum.w);
+                }
+            }
+            write_row(cons.b, cons.hk, r, c4, sum, mm, ll);
+        }
+        cluster_meet();   // nobody's shared memory goes away while another reads it
+    } else {
+        __syncthreads();
+        stamp(4);
+        if (npend_s[0] > 0) draw_tickets();
+    }
     stamp(5);
 }
 
+// CTAs that run at the same time: two per SM (asked for once per device: a small call is bound by its host side).
 int stream_ctas_for_device() {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 2 * 148;
+    int sms = known[dev].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        known[dev].store(sms, std::memory_order_relaxed);
     }
     return 2 * sms;
 }
 
-template <int D, int NS, bool kAppend>
-int launch(const DecodeParams& p, int ctas, cudaStream_t stream) {
-    constexpr int smem = NS * 2 * kTile * D * 2 + (2 * 64 + 32) * 4 + (2 * kMaxBatch + 1 + 8 + 6 * kMaxPending + 1) * 4;
-    if (int rc = ensure_smem(decode_kernel<D, NS, kAppend>, smem, "cudaFuncSetAttribute(decode)")) return rc;
+template <int D, int NS, bool kCluster>
+cudaLaunchConfig_t decode_config(int ctas, int ranks, cudaStream_t stream, cudaLaunchAttribute* attr) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(ctas));
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = NS * 2 * kTile * D * 2 + (2 * 64 + 32) * 4 + (2 * kMaxBatch + 1 + 8 + 6 * kMaxPending + 3) * 4 + (kCluster ? 16 * D * 4 : 0);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    if (kCluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(ranks);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    return cfg;
+}
+
+template <int D, int NS, bool kAppend, bool kCluster>
+int launch(const DecodeParams& p, int ctas, cudaStream_t stream) {
+    auto kernel = decode_kernel<D, NS, kAppend, kCluster>;
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = decode_config<D, NS, kCluster>(ctas, p.ranks, stream, attr);
+    if (int rc = ensure_smem(kernel, static_cast<int>(cfg.dynamicSmemBytes), "cudaFuncSetAttribute(decode)")) return rc;
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, decode_kernel<D, NS, kAppend>, p), "decode launch");
+    ++cfg.numAttrs;
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, p), "decode launch");
 }
 
 // Scratch layout: 1024 ticket counters (int32), then m, l, O partials.
@@ -750,6 +889,50 @@ ScratchLayout scratch_layout(int batch, int kv_heads, int d, int ctas) {
     s.o_bytes = up(static_cast<int64_t>(s.slots) * 16 * d * 4);
     s.total = s.counter_bytes + s.m_bytes + s.l_bytes + s.o_bytes;
     return s;
+}
+
+// Clusters of `ranks` CTAs that run at the same time on the current device (8 to a GPC's 16 to 20 SMs of two
+// CTAs each leave some of them out); asked for once per kernel, size and device.
+template <int D, int NS, bool kAppend>
+int cluster_room(int ranks) {
+    static std::atomic<int> known[64][4];   // by log2 of the ranks; 0: not asked yet, else one more than the answer
+    int dev = 0, log = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    while ((1 << log) < ranks) ++log;
+    int room = known[dev][log].load(std::memory_order_relaxed);
+    if (room == 0) {
+        auto kernel = decode_kernel<D, NS, kAppend, true>;
+        cudaLaunchAttribute attr[1];
+        cudaLaunchConfig_t cfg = decode_config<D, NS, true>(ranks, ranks, nullptr, attr);
+        int n = 0;
+        if (ensure_smem(kernel, static_cast<int>(cfg.dynamicSmemBytes), "cudaFuncSetAttribute(decode)") != 0 ||
+            cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
+        room = n + 1;
+        known[dev][log].store(room, std::memory_order_relaxed);
+    }
+    return room - 1;
+}
+
+// CTAs per (batch, kv head) pair where each pair has a cluster of its own; 0 where the pairs are cut into equal
+// shares. A cluster's partials meet in shared memory, its first tiles are on their way before the length is
+// known, and no CTA has a second pair to end: 5 us less than the shares with their tickets. But a pair is as
+// long as it is, and a cluster of it as slow; with 1,024 keys to a rank that costs at most what it saves.
+// Measured on B200, us, shares and clusters, lengths U[n / 8, n]: 14 heads over 2, D 64, one sequence of 1,024
+// 7.0 and 4.4; 16 over 2, D 128: 1 x 4096 10.5 and 8.5 (8 ranks), 16 x 4096 16.6 and 13.5, 64 x 1024 (2 ranks)
+// 16.8 and 14.2, but 64 x 4096 33.9 and 35.8; 32 over 8, D 128: 8 x 4096 (4 ranks) 21.6 and 20.6, 32 x 1024 (1
+// rank) 22.7 and 21.3; equal lengths 8 x 4096 29.1 and 25.1. Clusters of 16: 8.1 where 8 took 8.9 at most, 12.4
+// where they took 7.4 at worst.
+template <int D, int NS, bool kAppend>
+int decode_ranks(const ktt_b200_decode_args* a) {
+    const int64_t pairs = static_cast<int64_t>(a->batch) * a->kv_heads, ctas = stream_ctas_for_device();
+    for (int ranks = 8; ranks >= 1; ranks /= 2) {
+        if (a->splits > 0 && ranks > a->splits) continue;
+        if (ranks > 1 && (ranks / 2) * kTile >= a->sk) continue;   // half as many have a tile each
+        if (pairs * ranks > ctas) continue;
+        if (cluster_room<D, NS, kAppend>(ranks) < pairs) continue;
+        return a->sk <= 1024 * ranks ? ranks : 0;
+    }
+    return 0;
 }
 
 int decode_ctas(const ktt_b200_decode_args* a) {
@@ -775,6 +958,13 @@ const char* decode_refusal(const ktt_b200_decode_args* a) {
         if (a->q_strides[i] % 2 || a->out_strides[i] % 4) return "q strides must be even and out strides multiples of 4";
     }
     return nullptr;
+}
+
+template <int D, int NS, bool kAppend>
+int run_on(const ktt_b200_decode_args* a, DecodeParams& p, int ctas, cudaStream_t stream) {
+    p.ranks = decode_ranks<D, NS, kAppend>(a);
+    if (p.ranks > 0) return launch<D, NS, kAppend, true>(p, a->batch * a->kv_heads * p.ranks, stream);
+    return launch<D, NS, kAppend, false>(p, ctas, stream);
 }
 
 // Checks, parameter block and launch shared by both entry points; `base` is the scratch.
@@ -822,11 +1012,9 @@ int run_decode(const ktt_b200_decode_args* a, unsigned char* base, const Scratch
         p.rope_stride = app->rope_row_stride;
         p.rope_by_position = app->rope_by_position;
         p.lengths_out = app->lengths_out;
-        if (a->d == 64) return launch<64, 6, true>(p, ctas, st);
-        return launch<128, 3, true>(p, ctas, st);
     }
-    if (a->d == 64) return launch<64, 6, false>(p, ctas, st);
-    return launch<128, 3, false>(p, ctas, st);
+    if (a->d == 64) return app ? run_on<64, 6, true>(a, p, ctas, st) : run_on<64, 6, false>(a, p, ctas, st);
+    return app ? run_on<128, 3, true>(a, p, ctas, st) : run_on<128, 3, false>(a, p, ctas, st);
 }
 
 }  // namespace

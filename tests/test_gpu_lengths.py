@@ -195,6 +195,26 @@ def test_decode_calls_of_different_shapes_share_one_scratch(cuda):
         assert rel(out, ao.ruler_lengths(q, k, v, lengths)) <= FWD_BOUND, (i, b, h)
 
 
+# A cluster per (batch, kv head) pair: 8, 4, 2 and 1 of its CTAs have a tile of 64 keys, the most pairs for each size
+# of it and one more, and both sides of 1,024 keys per CTA (pairs in equal shares). Lengths on the edges of tiles.
+@pytest.mark.parametrize("b,h,hk,sk,d,sq", [
+    (1, 14, 2, 449, 64, 1), (1, 4, 1, 193, 128, 4), (2, 2, 2, 65, 64, 1), (3, 16, 1, 64, 128, 1), (2, 3, 1, 7, 64, 2),
+    (16, 4, 2, 520, 64, 1), (33, 1, 1, 300, 128, 1), (36, 4, 2, 200, 64, 1), (74, 2, 2, 130, 128, 1), (75, 2, 2, 130, 64, 1),
+    (148, 8, 2, 129, 64, 1), (149, 2, 2, 129, 64, 1), (2, 1, 1, 8193, 64, 1), (40, 2, 2, 4097, 64, 1), (150, 1, 1, 1024, 64, 1),
+])
+def test_decode_clusters(cuda, b, h, hk, sk, d, sq):
+    q, k, v = qkv(b, h, hk, sq, sk, d, b + sk)
+    edges = [sk, 1, 64, 65, 63, 16, 17, 128, 129, 448, 512, 513, sk - 1]
+    lengths = [max(1, min(sk, edges[i % len(edges)])) for i in range(b)]
+    out, lse = ops.decode(q.to(cuda), k.to(cuda), v.to(cuda), key_lengths=torch.tensor(lengths, dtype=torch.int32, device=cuda), need_lse=True)
+    assert rel(out, ao.ruler_lengths(q, k, v, lengths)) <= FWD_BOUND
+    for i, n in enumerate(lengths):   # what lies past a length, requested before the length is known, has no part
+        k[i, :, n:] = float("nan")
+        v[i, :, n:] = float("nan")
+    again, lse2 = ops.decode(q.to(cuda), k.to(cuda), v.to(cuda), key_lengths=torch.tensor(lengths, dtype=torch.int32, device=cuda), need_lse=True)
+    assert torch.equal(out, again) and torch.equal(lse, lse2)
+
+
 @pytest.mark.parametrize("n", [130, 700, 1100, 1500, 3000])   # 1 to 24 shares to a pair, four to a round of the merge
 def test_decode_merge_keeps_infinities(cuda, n):
     q, k, v = qkv(1, 16, 2, 1, n, 128, n)
