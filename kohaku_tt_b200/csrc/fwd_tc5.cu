@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(Plan<D>::kThreads, 1) fwd_tc5_kernel(
 
     // The producer warp sets the barriers up itself and goes straight to its first loads;
     // it only arrives at the start-up barrier, the others wait there for it and for the
-    // tensor-memory allocation.
+    // tensor-memory allocation. (A barrier of its own: a producer with few loads reaches the last
+    // __syncthreads while others still wait here, and would count for them a second time.)
     if (warp == P::kMmaWarp + 1) {
       // One barrier per lane: lane i initialises barrier i with its arrival count.
       static_assert(P::bCount <= 32, "one barrier per lane");
@@ -237,11 +238,11 @@ __global__ void __launch_bounds__(Plan<D>::kThreads, 1) fwd_tc5_kernel(
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       fence_async_smem();
       __syncwarp();
-      asm volatile("barrier.cta.arrive 0, %0;" ::"n"(P::kThreads) : "memory");
+      asm volatile("barrier.cta.arrive 1, %0;" ::"n"(P::kThreads) : "memory");
     } else {
       if (warp == P::kMmaWarp) tmem_alloc(smem_u32(tmem_slot), kTmemCols);
       tc_fence_before();
-      asm volatile("barrier.cta.sync 0, %0;" ::"n"(P::kThreads) : "memory");
+      asm volatile("barrier.cta.sync 1, %0;" ::"n"(P::kThreads) : "memory");
       tc_fence_after();
     }
     const uint32_t tmem = *tmem_slot;
