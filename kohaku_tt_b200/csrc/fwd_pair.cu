@@ -1353,6 +1353,108 @@ bool forward_pair_takes(const AttnParams& p) {
            operand_layout(p.v, tk, p.kv_heads, bq, p.vs, s, &why);
 }
 
+// The time at which the last of `machines` is done, when each item goes to the first free one: `cost[i]`
+// us of `count[i]` items, the longest first. Machines that are done at the same time are one group.
+namespace {
+constexpr int kMostLevels = 64;
+float makespan(const float* cost, const int64_t* count, int levels, int64_t machines) {
+    float at[2 * kMostLevels + 2];
+    int64_t of[2 * kMostLevels + 2];
+    int n = 1, first = 0;
+    at[0] = 0.f;
+    of[0] = machines;
+    for (int i = 0; i < levels; ++i) {
+        for (int64_t left = count[i]; left > 0;) {
+            const int64_t take = left < of[first] ? left : of[first];
+            const float done = at[first] + cost[i];
+            left -= take;
+            of[first] -= take;
+            if (of[first] == 0) ++first;
+            int j = n;   // (mostly the last)
+            while (j > first && at[j - 1] > done) --j;
+            if (j > first && at[j - 1] == done) {
+                of[j - 1] += take;
+                continue;
+            }
+            if (n == 2 * kMostLevels + 2) {   // make room at the front; (out of it: the groups are many, and close)
+                if (first == 0) return at[n - 1] > done ? at[n - 1] : done;
+                for (int k = first; k < n; ++k) {
+                    at[k - first] = at[k];
+                    of[k - first] = of[k];
+                }
+                n -= first;
+                j -= first;
+                first = 0;
+            }
+            for (int k = n; k > j; --k) {
+                at[k] = at[k - 1];
+                of[k] = of[k - 1];
+            }
+            at[j] = done;
+            of[j] = take;
+            ++n;
+        }
+    }
+    return at[n - 1];
+}
+
+// Dense calls of head dim 64 or 128 without a mask: whether this kernel's pairs of tiles fill their rounds so
+// much better than the other kernel's tiles (D 64: two halves of a tile's keys at a time, from six tiles per SM
+// on whole tiles in two streams; D 128: whole tiles) that it ends sooner by the estimate below. What a call, an
+// item, a block and, causal, a diagonal cost (us) is fitted to 490 calls of 20 to 1,200 tiles (D 64 within 5 %
+// rms, D 128 within 4 and 6.5): prompts of 1 to 16 sequences, 100 to 4,096 rows, and non-causal ones of 200 to
+// 4,608. The line is 8 % because none of 610 measured calls on this side of it is slower here (at 3 % four were,
+// by up to 5 %); over all of them that is 4.8 % (D 64) and 1.1 % (D 128) of the time, at most 1.3 times: 8 x 14
+// heads over 2 x 512, D 64, causal 19.7 and 15.7 us, 2 x 32 over 8 x 1024 27.7 and 21.8, 20 heads x 1024 20.7 and
+// 18.4; the other way 1 x 14 over 2 x 2048 causal 19.7 and 30.8, 20 heads x 4096 140 and 157.
+bool pair_rounds_better(const AttnParams& p) {
+    struct Fit { float call, item, block, diagonal; };
+    static constexpr Fit kOther[2] = {{2.59f, 2.36f, 1.66f, 0.07f}, {3.62f, 2.55f, 0.95f, 0.42f}};
+    static constexpr Fit kPair[2] = {{2.78f, 2.54f, 1.56f, 0.36f}, {3.55f, 2.43f, 2.20f, 0.67f}};
+    const int wide = p.d == 128 ? 1 : 0, tiles = (p.sq + kBM - 1) / kBM, group = p.heads / p.kv_heads;
+    const int64_t sms = sm_count(), planes = static_cast<int64_t>(p.batch) * p.kv_heads, heads = planes * group, all = heads * tiles;
+    if (tiles > kMostLevels || all > 8 * sms) return false;   // many rounds: the two are even
+    const Fit &o = kOther[wide], &m = kPair[wide];
+    const int shift = p.causal == KTT_B200_CAUSAL_BOTTOM_RIGHT ? p.sk - p.sq : 0;
+    auto blocks_of = [&](int back) {   // of the tile `back` tiles from the last
+        int kend = p.sk;
+        if (p.causal) {
+            const int last = (tiles - back) * kBM;
+            kend = (last < p.sq ? last : p.sq) + shift;
+            kend = kend < 0 ? 0 : kend < p.sk ? kend : p.sk;
+        }
+        return (kend + kBN - 1) / kBN;
+    };
+    float cost[2 * kMostLevels];
+    int64_t count[2 * kMostLevels];
+    const bool halves = !wide && all <= 6 * sms, dual = p.sk > kBN && all <= sms;
+    auto add = [&](const Fit& f, int& n, int blocks, int64_t items) {
+        const float c = f.item + (p.causal ? f.diagonal : 0.f) + f.block * static_cast<float>(blocks);
+        if (n > 0 && cost[n - 1] == c) {
+            count[n - 1] += items;
+            return;
+        }
+        cost[n] = c;
+        count[n++] = items;
+    };
+    int n = 0;
+    for (int t = 0; t < tiles; ++t) add(o, n, halves ? (blocks_of(t) + 1) / 2 : blocks_of(t), heads);
+    const float other = o.call + makespan(cost, count, n, wide || halves ? sms : 2 * sms);
+    n = 0;
+    if (dual) {
+        for (int t = 0; t < tiles; ++t) add(m, n, (blocks_of(t) + 1) / 2, heads);
+    } else {
+        // An item is two neighbours in a plane's list of (tile, head), last rows first.
+        for (int t = 0; t < tiles; ++t) {
+            const int items = ((t + 1) * group + 1) / 2 - (t * group + 1) / 2;   // those whose first tile is one of these
+            if (items > 0) add(m, n, blocks_of(t), planes * items);
+        }
+    }
+    const float pair = m.call + makespan(cost, count, n, sms);
+    return pair < 0.92f * other;
+}
+}  // namespace
+
 // Head dims 64 and 128 without a mask or with one row of it per (batch, head) have kernels of their
 // own, with one tile per work item and two items at a time on an SM. This one is faster where its
 // pairs fill whole rounds and the keys are few: what it leaves out of a block (columns past the last
@@ -1364,8 +1466,11 @@ bool forward_pair_takes(const AttnParams& p) {
 //    one weighs less);
 //  - D 64: 1024 keys, with mask terms 320 (at 1024 keys 26.9 -> 27.9);
 //  - D 128: 320 keys in the first round or with mask terms, else 96 (at 200 keys 20.9 -> 21.9).
+// Without a mask also where its rounds are the better filled ones (pair_rounds_better).
 bool forward_pair_preferred(const AttnParams& p) {
-    if (p.causal || p.cu_q || p.key_lengths || mask_needs_plan(p) || p.d != p.dv || (p.d != 64 && p.d != 128)) return false;
+    if (p.cu_q || p.key_lengths || mask_needs_plan(p) || p.d != p.dv || (p.d != 64 && p.d != 128)) return false;
+    if (p.mask_dtype == KTT_B200_MASK_NONE && pair_rounds_better(p) && forward_pair_takes(p)) return true;
+    if (p.causal) return false;
     const int64_t sms = sm_count(), group = p.heads / p.kv_heads, planes = static_cast<int64_t>(p.batch) * p.kv_heads;
     const int64_t per_plane = (p.sq + kBM - 1) / kBM * group, tiles = per_plane * planes, pairs = (per_plane + 1) / 2 * planes;
     const int64_t rounds = (tiles + 2 * sms - 1) / (2 * sms), last = tiles - (rounds - 1) * 2 * sms;

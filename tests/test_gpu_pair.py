@@ -74,6 +74,16 @@ def test_few_keys(cuda, h, sq, sk, d, masked):
     _check(cuda, q, k, v, mask=keep if masked else None, kernel="auto")
 
 
+# Dense calls without a mask take the kernel whose rounds are the better filled: both sides of that line, causal and
+# not, one and several tiles per item, an odd number of (tile, head)s, lengths that are no multiple of a tile.
+@pytest.mark.parametrize("b,h,hk,sq,sk,d,causal", [
+    (8, 14, 2, 256, 256, 64, True), (1, 14, 2, 1024, 1024, 64, True), (3, 15, 3, 500, 500, 64, True), (9, 9, 3, 385, 385, 64, True),
+    (2, 12, 12, 700, 700, 64, False), (2, 20, 20, 300, 900, 64, False), (8, 16, 16, 200, 200, 128, True), (2, 5, 1, 400, 250, 128, True),
+])
+def test_better_filled_rounds(cuda, b, h, hk, sq, sk, d, causal):
+    _check(cuda, *qkv(b, h, hk, sq, sk, d, b + sq + sk + d), causal=causal, kernel="auto")
+
+
 # Few rows: the warp-MMA kernel, up to where the tiles fill (both sides of the line).
 @pytest.mark.parametrize("b,h,sq,sk,d,kind,kernel", [
     (1, 1, 1, 1, 8, None, "mma"), (2, 16, 49, 49, 32, None, "mma"), (64, 16, 64, 64, 32, "bf16", "mma"),
