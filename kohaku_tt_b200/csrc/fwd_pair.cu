@@ -136,8 +136,9 @@ struct PairParams {
     AttnParams a;
     int* status;
     int dim_of[3][3];     // per operand (q, k, v): tensor-map slot (1..3) of the row, head and batch dims
-    int work;             // items = levels * batch * kv_heads
-    int dual;
+    int work;             // items
+    int duals;            // items from this one on are halves: a tile each, both tiles of the CTA on it (0: all of them)
+    int cut;              // ... of the pairs from this item on, two items each; 0 where every item is a tile
     int* work_counter;    // null: a fixed deal
     int* done_counter;    // with it: the last producer to finish puts both back to zero
     int grouped;          // item order (decode_item)
@@ -147,6 +148,7 @@ struct PairParams {
 
 struct alignas(16) Item {
     int b, hk;                  // b < 0: no more items
+    int dual;                   // A and B are halves of the keys of one tile
     int h[2], q0[2], kend[2];   // per tile; kend: keys any of its rows sees
     int n[2];                   // key blocks per tile (dual: its share); n[0] >= n[1]
     int valid[2];
@@ -163,7 +165,12 @@ static_assert(sizeof(Item) <= 96, "the queue's slots");
 __device__ __forceinline__ Item decode_item(const PairParams& tp, int w) {
     const AttnParams& p = tp.a;
     Item k;
-    int level;
+    int level, only = 0;   // only: which of a pair's tiles a half is of
+    k.dual = w >= tp.duals;
+    if (k.dual && tp.cut) {
+        only = (w - tp.duals) & 1;
+        w = tp.cut + ((w - tp.duals) >> 1);
+    }
     if (tp.grouped) {
         const int plane = div_by(w, tp.by_levels);
         level = w - plane * static_cast<int>(tp.by_levels.d);
@@ -181,7 +188,7 @@ __device__ __forceinline__ Item decode_item(const PairParams& tp, int w) {
     const int units = tiles * group;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-        const int u = tp.dual ? level : 2 * level + t;
+        const int u = !k.dual ? 2 * level + t : tp.cut ? 2 * level + only : level;
         k.valid[t] = u < units;
         const int back = div_by(u, tp.by_group);
         k.h[t] = k.hk * group + (u - back * group);
@@ -191,7 +198,7 @@ __device__ __forceinline__ Item decode_item(const PairParams& tp, int w) {
         k.kend[t] = max(kend, 0);
         k.n[t] = k.valid[t] ? (k.kend[t] + kBN - 1) >> 7 : 0;
     }
-    if (tp.dual) {
+    if (k.dual) {
         k.n[1] = k.n[0] >> 1;
         k.n[0] -= k.n[1];
     }
@@ -247,7 +254,7 @@ struct BlockIter<true> {
 __device__ __forceinline__ void apply_plan(const PairParams& tp, Item& k) {
     int n = 0;
     for (int w = 0; w < tp.plan.words; ++w) n += __popc(active_word(tp, k, w));
-    if (tp.dual) {
+    if (k.dual) {
         k.n[1] = n >> 1;
         k.n[0] = n - k.n[1];
     } else {
@@ -295,10 +302,11 @@ __device__ __forceinline__ bool wait_one(uint32_t b, uint32_t par, volatile int*
 // ---- the kernel ------------------------------------------------------------------------
 
 // kMask: 0 none, 1 a row per (batch, head), 2 a plan (a row per query).
+// kMixed: of the items some are pairs of tiles and some halves of one (last_round_in_halves).
 // kTurns: where P overwrites the scores a tile's products and its softmax are one chain, and two tiles that
 // run in step wait for the tensor cores at the same time and then for the exponentials. Taking turns at the
 // exponentials, the products of one run under those of the other.
-template <int DP, int kMask, bool kTurns>
+template <int DP, int kMask, bool kTurns, bool kMixed>
 __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const PairParams tp) {
@@ -317,6 +325,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + P::kBars + P::bCount * 8 + 8);
     Item* queue = reinterpret_cast<Item*>(smem + P::kItems);   // [kQueue]
     const AttnParams& p = tp.a;
+    const bool all_dual = tp.duals == 0;
 
     if (warp == kProducerWarp) {
         for (int i = lane; i < P::bCount; i += 32) {
@@ -325,9 +334,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             if ((i >= P::bSFree && i < P::bSFree + 2) || (i >= P::bPFull && i < P::bPFull + 4) ||
                 (i >= P::bOFree && i < P::bOFree + 2) || (i >= P::bMask && i < P::bMask + 2) || i == P::bPartial) count = 4;
             if (i >= P::bWorkFree && i < P::bWorkFree + P::kQueue) count = 10;   // the softmax and the MMA warps
-            // Pair: both tiles release every ring tile. Dual: each has one user, but they share Q.
-            if (i >= P::bKVEmpty && !tp.dual) count = 2;
-            if (i == P::bQFree && tp.dual) count = 2;
+            // Pair: both tiles release every ring tile. Dual: each has one user, but they share Q. (Mixed: one
+            // user, or tile A alone, releases twice.)
+            if (i >= P::bKVEmpty && (kMixed || !all_dual)) count = 2;
+            if (i == P::bQFree && (kMixed || all_dual)) count = 2;
             mbar_init(bar(i), count);
         }
         if (lane == 0) {
@@ -350,8 +360,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    const bool dual = tp.dual != 0;
-
     // The producer warp draws the items (from a counter, or the fixed deal of a snake order), works
     // out what they are and hands them to the other roles through a queue in shared memory: one
     // role's divisions and one copy of that code. Positions past the end of a short sequence are
@@ -450,6 +458,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             if (k.n[0] == 0) continue;
             Iter it[2];
             it[0].start(tp, k, 0);
+            const bool dual = kMixed ? k.dual != 0 : all_dual;
             if (dual) it[1].start(tp, k, k.n[0]);
             load_q(k, 0);
             const int entries = dual ? k.n[0] + k.n[1] : k.n[0];
@@ -479,15 +488,13 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
         // What stands between two products is this warp's scalar work, at the pace of one warp
         // beside two in their softmax: no divisions, no state in memory, one vote per pair of waits.
         const int t = warp - kMmaWarp;
-        const uint64_t q_desc = smem_desc(sbase + P::kQ + (tp.dual ? 0 : t) * P::kOperand, 16, 1024);
+        const uint64_t q_descs = smem_desc(sbase + P::kQ + (kMixed || all_dual ? 0 : t) * P::kOperand, 16, 1024);
         const uint64_t k_desc = smem_desc(sbase + P::kRing, 16, 1024);
         const uint64_t v_desc = smem_desc(sbase + P::kRing, P::kTile, 1024);
         const int d_steps = (p.d + 15) >> 4;
         const uint32_t d_s = tmem + t * 128, a_p = tmem + P::kP + t * P::kPStep, d_o = tmem + P::kO + t * DP;
-        const int q_bar = dual ? 0 : t;
-        const int stride = dual ? 4 : 2;    // ring tiles from one of this tile's blocks to its next
         int blk = 0, items = 0;             // this tile's blocks and items so far: parities
-        int q_items = 0;                    // Q tiles so far
+        int q_a = 0, q_b = 0;               // Q tiles so far (mixed: Q_A, Q_B)
         int base = 0, base_lap = 0;         // ring position of the item's first tile
         bool ok = true;
         auto wait_two = [&](uint32_t b0, uint32_t par0, uint32_t b1, uint32_t par1, int code) {
@@ -506,8 +513,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             if (!take_item(n, k, ok)) break;
             give_item(n);
             if (k.n[0] == 0) continue;
+            const bool dual = kMixed ? k.dual != 0 : all_dual;
             const int nb = t ? k.n[1] : k.n[0], kend = t ? k.kend[1] : k.kend[0], klen = k.si.klen;
             const int entries = dual ? k.n[0] + k.n[1] : k.n[0];
+            const int q_bar = dual ? 0 : t, q_items = kMixed && q_bar ? q_b : q_a;
+            const int stride = dual ? 4 : 2;    // ring tiles from one of this tile's blocks to its next
+            const uint64_t q_desc = kMixed ? q_descs + static_cast<uint32_t>((q_bar * P::kOperand) >> 4) : q_descs;
             Iter it;
             it.start(tp, k, dual && t ? k.n[0] : 0);
             int s_slot = base, s_lap = base_lap;    // K of the next score product; V is one further
@@ -555,7 +566,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     }
                     tc_commit(bar(P::bSFull + t));
                     tc_commit(bar(P::bKVEmpty + s_slot));
-                    if (j + 2 == nb) tc_commit(bar(P::bQFree + q_bar));
+                    if (kMixed && dual) tc_commit(bar(P::bKVEmpty + s_slot));
+                    if (j + 2 == nb) {
+                        tc_commit(bar(P::bQFree + q_bar));
+                        if (kMixed && !dual && t == 0) tc_commit(bar(P::bQFree));
+                    }
                     advance(s_slot, s_lap, stride);
                 };
                 auto values = [&]() {
@@ -601,6 +616,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                     }
                     tc_commit(bar(P::bPVDone + t));
                     tc_commit(bar(P::bKVEmpty + v_slot));
+                    if (kMixed && dual) tc_commit(bar(P::bKVEmpty + v_slot));
                     advance(v_slot, v_lap, stride);
                 };
                 if constexpr (P::kPOverS) {
@@ -628,7 +644,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 __syncwarp();
             }
             if (nb > 0) ++items;
-            if (nb > 0 || dual) ++q_items;
+            if (kMixed) {
+                ++q_a;
+                if (!dual && nb > 0 && t) ++q_b;
+            } else if (nb > 0 || dual) {
+                ++q_a;
+            }
             blk += nb;
             // 2 * entries can be several times round the ring.
             for (int left = 2 * entries; left > 0; left -= P::kSlots) advance(base, base_lap, min(left, P::kSlots));
@@ -658,6 +679,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
                 give_item(n);
                 continue;
             }
+            const bool dual = kMixed ? k.dual != 0 : all_dual;
             // (Selected once: an index that is not a constant would put the item into memory.)
             const int taking = kTurns ? k.n[1] : 0;   // the blocks both tiles have: B has no more than A
             const int nb = t ? k.n[1] : k.n[0], h = t ? k.h[1] : k.h[0], q0 = t ? k.q0[1] : k.q0[0], kend = t ? k.kend[1] : k.kend[0];
@@ -956,13 +978,14 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             // ---- the item's end: O / l to memory ----
             // (The item is read from the queue again: its numbers would not fit beside the scores.)
             const Item* e = queue + n % P::kQueue;
-            const int nb_other = e->n[1], e_b = e->b, e_h = e->h[dual ? 0 : t], e_q0 = e->q0[dual ? 0 : t], e_lq = e->si.lq, e_off = e->si.q_off;
+            const bool halves = kMixed ? e->dual != 0 : all_dual;
+            const int nb_other = e->n[1], e_b = e->b, e_h = e->h[halves ? 0 : t], e_q0 = e->q0[halves ? 0 : t], e_lq = e->si.lq, e_off = e->si.q_off;
             const int last = blk + nb - 1;
             blk += nb;
             turns += taking;
             float l_row = (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y), m_row = m_ref;
             float f_mine = 1.f, f_other = 0.f;
-            const bool merge = dual && nb_other > 0;
+            const bool merge = halves && nb_other > 0;
             if (merge) {
                 wait_for(P::bPVDone + t, last & 1, 330 + t);
                 if (!ok) break;
@@ -1322,14 +1345,17 @@ int launch_dependent(Kernel kernel, dim3 grid, int threads, int smem, cudaStream
 template <int DP>
 int launch_pair(const AttnParams& p, const CUtensorMap (&maps)[3], PairParams& tp, int grid, cudaStream_t stream) {
     using P = PairPlan<DP>;
-    auto kernel = mask_needs_plan(p) ? fwd_pair_kernel<DP, 2, false> : p.mask_dtype != KTT_B200_MASK_NONE ? fwd_pair_kernel<DP, 1, false> : fwd_pair_kernel<DP, 0, false>;
+    const bool none = p.mask_dtype == KTT_B200_MASK_NONE, mixed = tp.cut > 0;
+    auto kernel = mask_needs_plan(p) ? fwd_pair_kernel<DP, 2, false, false>
+                : none ? (mixed ? fwd_pair_kernel<DP, 0, false, true> : fwd_pair_kernel<DP, 0, false, false>)
+                       : (mixed ? fwd_pair_kernel<DP, 1, false, true> : fwd_pair_kernel<DP, 1, false, false>);
     if constexpr (P::kPOverS) {
         // Turns, without a mask, from five blocks of keys on: with three, their waits and the code for them
         // weigh more. Measured, us without and with: D 80, 16 heads x 4096 167 -> 153; D 96, 48 x 1025 52.5 ->
         // 49.3; D 80, 32 x 2048 causal 46.9 -> 45.0; 128 x 577 44.4 -> 43.3, 128 x 640 42.3 -> 40.4; but 256 x
         // 257 34.9 -> 35.9, D 128, 10 x 2048 queries x 300 keys 12.7 -> 13.4. (Head dims up to 64, whose scores
         // are ready in any case: 157 both, 20 x 4096. Masks with a row per query, D 128, 32 x 2048: 68.7 -> 71.1.)
-        if (p.mask_dtype == KTT_B200_MASK_NONE && p.sk > 4 * kBN) kernel = fwd_pair_kernel<DP, 0, true>;
+        if (none && p.sk > 4 * kBN) kernel = mixed ? fwd_pair_kernel<DP, 0, true, true> : fwd_pair_kernel<DP, 0, true, false>;
     }
     if (int rc = ensure_smem(kernel, P::kBytes, "cudaFuncSetAttribute(fwd_pair)")) return rc;
     return launch_dependent(kernel, dim3(grid), kPairThreads, P::kBytes, stream, "fwd_pair launch", maps[0], maps[1], maps[2], tp);
@@ -1352,6 +1378,17 @@ bool forward_pair_takes(const AttnParams& p) {
     return operand_layout(p.q, tq, p.heads, bq, p.qs, s, &why) && operand_layout(p.k, tk, p.kv_heads, bq, p.ks, s, &why) &&
            operand_layout(p.v, tk, p.kv_heads, bq, p.vs, s, &why);
 }
+
+namespace {
+// Pairs of equal length in rounds of one per SM, the last of which leaves half of the SMs or more without one:
+// its tiles run as halves, each on an SM of its own.
+bool last_round_in_halves(const AttnParams& p) {
+    if (p.causal || p.cu_q || p.key_lengths || mask_needs_plan(p) || p.sk <= kBN) return false;
+    const int64_t sms = sm_count(), group = p.heads / p.kv_heads, planes = static_cast<int64_t>(p.batch) * p.kv_heads;
+    const int64_t per_plane = (p.sq + kBM - 1) / kBM * group, pairs = (per_plane + 1) / 2 * planes, over = pairs % sms;
+    return per_plane * planes > sms && pairs > sms && over > 0 && 2 * over <= sms;
+}
+}  // namespace
 
 // The time at which the last of `machines` is done, when each item goes to the first free one: `cost[i]`
 // us of `count[i]` items, the longest first. Machines that are done at the same time are one group.
@@ -1448,6 +1485,11 @@ bool pair_rounds_better(const AttnParams& p) {
         for (int t = 0; t < tiles; ++t) {
             const int items = ((t + 1) * group + 1) / 2 - (t * group + 1) / 2;   // those whose first tile is one of these
             if (items > 0) add(m, n, blocks_of(t), planes * items);
+        }
+        if (last_round_in_halves(p)) {   // (all of them are alike)
+            const int64_t over = count[0] % sms;
+            count[0] -= over;
+            add(m, n, (blocks_of(0) + 1) / 2, 2 * over);
         }
     }
     const float pair = m.call + makespan(cost, count, n, sms);
@@ -1576,9 +1618,16 @@ int launch_whole(const AttnParams& p, void* workspace, int64_t workspace_bytes, 
     // tiles would leave SMs without one. (Up to six tiles per SM it cost more than it gave, when it was
     // tried: 16 x 16 heads x 257, D 80: 43 -> 37 us without it, 4 x 16 heads 19 -> 13; 2 x 16 heads x
     // 2048, D 64, causal mask: 71 -> 58. At 8 heads x 2 x 1024, D 80, 128 tiles, it gives 25 -> 16.)
-    tp.dual = p.sk > kBN && units <= sms ? 1 : 0;
-    const int levels = tp.dual ? q_tiles * group : (q_tiles * group + 1) / 2;
+    const bool dual = p.sk > kBN && units <= sms;
+    const int levels = dual ? q_tiles * group : (q_tiles * group + 1) / 2;
     tp.work = levels * p.kv_heads * p.batch;
+    tp.duals = dual ? 0 : tp.work;
+    tp.cut = 0;
+    const int over = last_round_in_halves(p) ? tp.work % sms : 0;
+    if (over) {
+        tp.cut = tp.duals = tp.work - over;
+        tp.work += over;
+    }
     tp.by_batch = divisor_of(p.batch);
     tp.by_kv_heads = divisor_of(p.kv_heads);
     tp.by_group = divisor_of(group);
