@@ -1350,12 +1350,12 @@ int launch_pair(const AttnParams& p, const CUtensorMap (&maps)[3], PairParams& t
                 : none ? (mixed ? fwd_pair_kernel<DP, 0, false, true> : fwd_pair_kernel<DP, 0, false, false>)
                        : (mixed ? fwd_pair_kernel<DP, 1, false, true> : fwd_pair_kernel<DP, 1, false, false>);
     if constexpr (P::kPOverS) {
-        // Turns, without a mask, from five blocks of keys on: with three, their waits and the code for them
+        // Turns, without a mask, for pairs from five blocks of keys on: with three, their waits and the code for them
         // weigh more. Measured, us without and with: D 80, 16 heads x 4096 167 -> 153; D 96, 48 x 1025 52.5 ->
         // 49.3; D 80, 32 x 2048 causal 46.9 -> 45.0; 128 x 577 44.4 -> 43.3, 128 x 640 42.3 -> 40.4; but 256 x
-        // 257 34.9 -> 35.9, D 128, 10 x 2048 queries x 300 keys 12.7 -> 13.4. (Head dims up to 64, whose scores
+        // 257 34.9 -> 35.9, D 128, 10 x 2048 queries x 300 keys 12.7 -> 13.4, and halves, D 80, 8 x 935 14.3 -> 14.6. (Head dims up to 64, whose scores
         // are ready in any case: 157 both, 20 x 4096. Masks with a row per query, D 128, 32 x 2048: 68.7 -> 71.1.)
-        if (none && p.sk > 4 * kBN) kernel = mixed ? fwd_pair_kernel<DP, 0, true, true> : fwd_pair_kernel<DP, 0, true, false>;
+        if (none && tp.duals > 0 && p.sk > 4 * kBN) kernel = mixed ? fwd_pair_kernel<DP, 0, true, true> : fwd_pair_kernel<DP, 0, true, false>;
     }
     if (int rc = ensure_smem(kernel, P::kBytes, "cudaFuncSetAttribute(fwd_pair)")) return rc;
     return launch_dependent(kernel, dim3(grid), kPairThreads, P::kBytes, stream, "fwd_pair launch", maps[0], maps[1], maps[2], tp);
@@ -1450,6 +1450,7 @@ bool pair_rounds_better(const AttnParams& p) {
     static constexpr Fit kPair[2] = {{2.78f, 2.54f, 1.56f, 0.36f}, {3.55f, 2.43f, 2.20f, 0.67f}};
     const int wide = p.d == 128 ? 1 : 0, tiles = (p.sq + kBM - 1) / kBM, group = p.heads / p.kv_heads;
     const int64_t sms = sm_count(), planes = static_cast<int64_t>(p.batch) * p.kv_heads, heads = planes * group, all = heads * tiles;
+    if (all <= sms) return false;                             // one round either way
     if (tiles > kMostLevels || all > 8 * sms) return false;   // many rounds: the two are even
     const Fit &o = kOther[wide], &m = kPair[wide];
     const int shift = p.causal == KTT_B200_CAUSAL_BOTTOM_RIGHT ? p.sk - p.sq : 0;
