@@ -74,6 +74,25 @@ def test_few_keys(cuda, h, sq, sk, d, masked):
     _check(cuda, q, k, v, mask=keep if masked else None, kernel="auto")
 
 
+# Pairs beyond whole rounds of one per SM run as halves: both sides of that line (148 and 149, 222 and 223 pairs), of two
+# and of more rounds, tiles without a partner, two to six blocks of keys (an odd number shares unevenly), a last block
+# of one key, and a mask that leaves a half without a visible key.
+@pytest.mark.parametrize("b,h,hk,sq,sk,d,masked", [
+    (1, 148, 148, 256, 129, 64, False), (1, 149, 149, 256, 129, 64, False), (2, 75, 75, 200, 144, 80, False),
+    (1, 222, 222, 129, 300, 40, False), (1, 223, 223, 129, 300, 40, False), (2, 35, 35, 600, 257, 80, False),
+    (1, 160, 20, 130, 700, 128, False), (5, 30, 30, 256, 513, 96, False), (1, 302, 302, 256, 384, 64, False),
+    (2, 75, 75, 256, 320, 64, True), (1, 150, 150, 150, 290, 128, True), (2, 35, 7, 600, 260, 64, True),
+])
+def test_last_round_in_halves(cuda, b, h, hk, sq, sk, d, masked):
+    q, k, v = qkv(b, h, hk, sq, sk, d, h + sq + sk)
+    keep = None
+    if masked:
+        keep = torch.rand(b, 1, 1, sk, generator=torch.Generator().manual_seed(h)) > 0.3
+        keep[..., 0] = True
+        keep[0, ..., 128:] = False
+    _check(cuda, q, k, v, mask=keep)
+
+
 # Dense calls without a mask take the kernel whose rounds are the better filled: both sides of that line, causal and
 # not, one and several tiles per item, an odd number of (tile, head)s, lengths that are no multiple of a tile.
 @pytest.mark.parametrize("b,h,hk,sq,sk,d,causal", [
