@@ -1,7 +1,7 @@
 // Forward on the Blackwell tensor path for what the other two tcgen05 kernels are not built for -
 // head dims that are any multiple of 8 up to 128, and masks with a row per query, unless the rows are
-// so few that warp-MMA is the faster (forward_pair_pays) - and for calls of few keys in which it is
-// the faster (forward_pair_preferred). TMA tile loads, tcgen05.mma with accumulators in tensor memory,
+// so few that warp-MMA is the faster (forward_pair_pays) - and for calls of few keys, or whose rounds of
+// SMs it fills better, in which it is the faster (forward_pair_preferred). TMA tile loads, tcgen05.mma with accumulators in tensor memory,
 // online softmax with one thread per query row.
 //
 // A persistent CTA per SM works on two 128-row query tiles at a time, A and B:
@@ -17,8 +17,8 @@
 //   warp 10            draws the work and hands the items round, TMA loads of Q and of a ring of K
 //                      and V tiles
 //
-// An item of few blocks runs every role's code once or twice, so the code itself is what such
-// calls are bound by: a third of the instruction fetches missed the cache. Hence one copy of the item
+// An item of few blocks runs every role's code once or twice, and a third of the instruction fetches
+// missed the cache. Hence one copy of the item
 // arithmetic (the producer's), short waits, and loops where a block is not the common one: 94 to
 // 150 KB of instructions became 79 to 105, and 16 x 16 heads x 257 rows, D 80, took 42 us where it had
 // taken 49 (a fifth of the fetches still miss there, a tenth on the masked call below).
@@ -34,7 +34,7 @@
 // Two ways to use the two tiles:
 //   pair   A and B are neighbours in the list of (query tile, head) of one K / V head: one
 //          K / V stream serves both, which halves the traffic from L2
-//   dual   (no more tiles than SMs) A and B are the same query tile, A working on the first half of
+//   dual   (no more tiles than SMs, and the tiles of a last round that leaves half of the SMs idle) A and B are the same query tile, A working on the first half of
 //          its key blocks and B on the rest; A's threads then read B's unnormalised O straight
 //          out of tensor memory. The longest tile's serial chain is halved. Always A then B:
 //          the bits do not depend on timing.
