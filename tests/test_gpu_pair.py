@@ -93,6 +93,23 @@ def test_last_round_in_halves(cuda, b, h, hk, sq, sk, d, masked):
     _check(cuda, q, k, v, mask=keep)
 
 
+# One row behind the last whole tile goes without a tile: both sides of the lines (148 and 150 tiles, one round of pairs
+# and more, a last round of 74 and 75), keys short of, at and past a warp's 32 and a pass of 256, groups of heads, lengths.
+@pytest.mark.parametrize("b,h,hk,sq,sk,d,dv,lengths", [
+    (1, 74, 74, 257, 257, 80, 80, None), (1, 75, 75, 257, 257, 80, 80, None), (2, 74, 74, 257, 32, 64, 64, None), (1, 149, 149, 257, 33, 40, 40, None),
+    (2, 111, 111, 257, 256, 64, 128, None), (1, 223, 223, 257, 1152, 96, 96, None), (1, 223, 223, 257, 1153, 8, 8, None),
+    (2, 80, 40, 129, 31, 120, 24, None), (1, 160, 10, 129, 700, 128, 128, None), (3, 60, 60, 257, 300, 72, 72, [1, 300, 130]),
+])
+def test_last_row_apart(cuda, b, h, hk, sq, sk, d, dv, lengths):
+    q, k, v = qkv(b, h, hk, sq, sk, d, h + sq + sk, dv=dv)
+    _check(cuda, q, k, v, lengths=lengths)
+    # (One row in 257 hardly shows in the whole's error.)
+    ln = None if lengths is None else torch.tensor(lengths, dtype=torch.int32, device=cuda)
+    out, _ = ops.sdpa_forward(q.to(cuda), k.to(cuda), v.to(cuda), key_lengths=ln, kernel="flash_pair")
+    last = q[:, :, -1:]
+    assert rel(out[:, :, -1:], ao.ruler_dense(last, k, v) if lengths is None else ao.ruler_lengths(last, k, v, lengths)) <= FWD_BOUND
+
+
 # Dense calls without a mask take the kernel whose rounds are the better filled: both sides of that line, causal and
 # not, one and several tiles per item, an odd number of (tile, head)s, lengths that are no multiple of a tile.
 @pytest.mark.parametrize("b,h,hk,sq,sk,d,causal", [
