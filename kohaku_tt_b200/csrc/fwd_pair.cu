@@ -109,8 +109,7 @@ struct PairPlan {
     static constexpr int bMask = bWorkFree + kQueue;   // + t: the block's mask terms are written
     static constexpr int bPartial = bMask + 2;         // dual: B's half is final
     static constexpr int bTurn = bPartial + 1;         // + 4 t + warp: the other tile's warp of this scheduler has had its turn
-    static constexpr int bRow = bTurn + 8;             // the softmax warps' parts of a row without a tile
-    static constexpr int bKVFull = bRow + 1;          // + ring slot
+    static constexpr int bKVFull = bTurn + 8;          // + ring slot
     static constexpr int bKVEmpty = bKVFull + kSlots;  // + ring slot
     static constexpr int bCount = bKVEmpty + kSlots;
     static_assert(bCount * 8 + 32 <= kBarBytes, "barrier area");
@@ -143,20 +142,18 @@ struct PairParams {
     int* work_counter;    // null: a fixed deal
     int* done_counter;    // with it: the last producer to finish puts both back to zero
     int grouped;          // item order (decode_item)
-    int rows_from;        // kRows: items from this one on are a query row each, the one behind a head's last whole tile
     Divisor by_batch, by_kv_heads, by_group, by_levels;
     MaskPlan plan;
 };
 
 struct alignas(16) Item {
     int b, hk;                  // b < 0: no more items
-    int dual;                   // 1: A and B are halves of the keys of one tile; kRow: no tile, but row q0[0]
+    int dual;                   // A and B are halves of the keys of one tile
     int h[2], q0[2], kend[2];   // per tile; kend: keys any of its rows sees
     int n[2];                   // key blocks per tile (dual: its share); n[0] >= n[1]
     int valid[2];
     SeqInfo si;
 };
-constexpr int kRow = 2;
 static_assert(sizeof(Item) <= 96, "the queue's slots");
 
 // Items of one (batch, K / V head) are neighbours in its list of (query tile, head), last rows first
@@ -165,28 +162,9 @@ static_assert(sizeof(Item) <= 96, "the queue's slots");
 // similar lengths; `grouped` (needs the counter) keeps all items of one
 // (batch, K / V head) together, so that the items in flight share the K / V of a few heads in L2
 // (measured on a packed 65,536-token batch with 537 MB of K / V: 4.85 -> 0.81 GB of DRAM reads).
-template <bool kRows>
 __device__ __forceinline__ Item decode_item(const PairParams& tp, int w) {
     const AttnParams& p = tp.a;
     Item k;
-    if (kRows && w >= tp.rows_from) {
-        w -= tp.rows_from;
-        const int t = div_by(w, tp.by_kv_heads);
-        k.hk = w - t * p.kv_heads;
-        const int u = div_by(t, tp.by_batch);   // the head of the group
-        k.b = t - u * p.batch;
-        k.si = seq_info(p, k.b);
-        k.dual = kRow;
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            k.h[x] = k.hk * static_cast<int>(tp.by_group.d) + u;
-            k.q0[x] = k.si.lq - 1;
-            k.kend[x] = max(k.si.klen, 0);
-            k.n[x] = 0;
-            k.valid[x] = 1;
-        }
-        return k;
-    }
     int level, only = 0;   // only: which of a pair's tiles a half is of
     k.dual = w >= tp.duals;
     if (k.dual && tp.cut) {
@@ -206,7 +184,7 @@ __device__ __forceinline__ Item decode_item(const PairParams& tp, int w) {
     }
     k.si = seq_info(p, k.b);
     const int group = static_cast<int>(tp.by_group.d);
-    const int tiles = (k.si.lq + (kRows ? 0 : kBM - 1)) >> 7;
+    const int tiles = (k.si.lq + kBM - 1) >> 7;
     const int units = tiles * group;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
@@ -321,130 +299,14 @@ __device__ __forceinline__ bool wait_one(uint32_t b, uint32_t par, volatile int*
     return true;
 }
 
-// ---- a row without a tile ----------------------------------------------------------------
-
-// One query row by the eight softmax warps, without tensor cores. A warp takes 32 keys at a time and keeps an
-// online softmax of its own: DP / 8 lanes read a key's row, 16 bytes each, all loads of K and V together (a thread
-// per key reads 32 lines at a time: 43.3 against 30.4 us on 256 x 257 rows, D 80); partial dot products are summed so
-// that each lane ends with one key's. Then the warps' parts are added up through shared memory, `parts`: float
-// [parity][8][DP + 2]; the parities alternate: what an item wrote is written again only after everybody has
-// arrived for the item between. About 730 instructions per 32 keys: bound by the issue slots and one chain.
-template <int DP>
-__device__ __forceinline__ bool row_alone(const AttnParams& p, const Item& k, float* parts, uint32_t bar, int phase, volatile int* abort_flag) {
-    constexpr int kLanes = DP / 8, kKeys = 32 / kLanes;   // lanes of a key, keys of a load
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = lane & (kLanes - 1), sub = lane / kLanes, keys = k.kend[0];
-    const bool in_d = c * 8 < p.d, in_dv = c * 8 < p.dv;
-    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-    auto pair_of = [](uint32_t u) { return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); };
-    const uint4 qv = in_d ? *reinterpret_cast<const uint4*>(p.q + k.b * p.qs[0] + k.h[0] * p.qs[1] + static_cast<int64_t>(k.q0[0]) * p.qs[2] + c * 8) : none;
-    const __nv_bfloat16* kp = p.k + k.b * p.ks[0] + k.hk * p.ks[1] + c * 8;
-    const __nv_bfloat16* vp = p.v + k.b * p.vs[0] + k.hk * p.vs[1] + c * 8;
-    float m_run = -INFINITY, l_run = 0.f;
-    float2 acc[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll 1
-    for (int first = warp * 32; first < keys; first += 256) {
-        uint4 kv[kLanes], vv[kLanes];
-#pragma unroll
-        for (int i = 0; i < kLanes; ++i) {
-            const int key = first + i * kKeys + sub;
-            kv[i] = in_d && key < keys ? *reinterpret_cast<const uint4*>(kp + static_cast<int64_t>(key) * p.ks[2]) : none;
-        }
-#pragma unroll
-        for (int i = 0; i < kLanes; ++i) {
-            const int key = first + i * kKeys + sub;
-            vv[i] = in_dv && key < keys ? *reinterpret_cast<const uint4*>(vp + static_cast<int64_t>(key) * p.vs[2]) : none;
-        }
-        const float2 q0 = pair_of(qv.x), q1 = pair_of(qv.y), q2 = pair_of(qv.z), q3 = pair_of(qv.w);
-        float s[kLanes];
-#pragma unroll
-        for (int i = 0; i < kLanes; ++i) {
-            float2 x = __fmul2_rn(pair_of(kv[i].x), q0);
-            float2 y = __fmul2_rn(pair_of(kv[i].y), q1);
-            x = __ffma2_rn(pair_of(kv[i].z), q2, x);
-            y = __ffma2_rn(pair_of(kv[i].w), q3, y);
-            s[i] = (x.x + x.y) + (y.x + y.y);
-        }
-#pragma unroll
-        for (int x = kLanes / 2; x > 0; x >>= 1) {
-            const bool upper = lane & x;
-#pragma unroll
-            for (int i = 0; i < x; ++i) {
-                const float got = __shfl_xor_sync(0xffffffffu, upper ? s[i] : s[i + x], x);
-                s[i] = (upper ? s[i + x] : s[i]) + got;
-            }
-        }
-        const float logit = first + c * kKeys + sub < keys ? s[0] * p.scale_log2 : -INFINITY;   // this lane's key
-        float m_new = fmaxf(m_run, logit);
-#pragma unroll
-        for (int x = 16; x > 0; x >>= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, x));
-        const float base = m_new == -INFINITY ? 0.f : m_new;
-        const float back = fast_exp2(m_run - base), w = fast_exp2(logit - base);
-        m_run = m_new;
-        l_run = fmaf(l_run, back, w);   // a lane's own keys
-        const float2 back2 = make_float2(back, back);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[e] = __fmul2_rn(acc[e], back2);
-#pragma unroll
-        for (int i = 0; i < kLanes; ++i) {
-            const float wi = __shfl_sync(0xffffffffu, w, (lane & ~(kLanes - 1)) | i);
-            const float2 w2 = make_float2(wi, wi);
-            acc[0] = __ffma2_rn(pair_of(vv[i].x), w2, acc[0]);
-            acc[1] = __ffma2_rn(pair_of(vv[i].y), w2, acc[1]);
-            acc[2] = __ffma2_rn(pair_of(vv[i].z), w2, acc[2]);
-            acc[3] = __ffma2_rn(pair_of(vv[i].w), w2, acc[3]);
-        }
-    }
-#pragma unroll
-    for (int x = 16; x > 0; x >>= 1) l_run += __shfl_xor_sync(0xffffffffu, l_run, x);
-#pragma unroll
-    for (int x = 16; x >= kLanes; x >>= 1) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            acc[e].x += __shfl_xor_sync(0xffffffffu, acc[e].x, x);
-            acc[e].y += __shfl_xor_sync(0xffffffffu, acc[e].y, x);
-        }
-    }
-    float* part = parts + ((phase & 1) * 8 + warp) * (DP + 2);
-    if (sub == 0) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(part + 2 + c * 8 + e * 2) = acc[e];
-    }
-    if (lane == 0) *reinterpret_cast<float2*>(part) = make_float2(m_run, l_run);
-    mbar_arrive_warp(bar);
-    if (!wait_one(bar, phase & 1, abort_flag, 395)) return false;
-    const int col = threadIdx.x;
-    if (col < p.dv) {
-        part -= warp * (DP + 2);
-        float m[8], m_all = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            m[i] = part[i * (DP + 2)];
-            m_all = fmaxf(m_all, m[i]);
-        }
-        const float base = m_all == -INFINITY ? 0.f : m_all;
-        float l = 0.f, o = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float f = fast_exp2(m[i] - base);
-            l = fmaf(part[i * (DP + 2) + 1], f, l);
-            o = fmaf(part[i * (DP + 2) + 2 + col], f, o);
-        }
-        p.out[k.b * p.os[0] + k.h[0] * p.os[1] + static_cast<int64_t>(k.q0[0]) * p.os[2] + col] = __float2bfloat16_rn(o * (l > 0.f ? 1.f / l : 0.f));
-        if (p.lse && col == 0) p.lse[k.b * p.ls[0] + k.h[0] * p.ls[1] + k.q0[0] * p.ls[2]] = l > 0.f ? kLn2 * (m_all + log2f(l)) : -INFINITY;
-    }
-    return true;
-}
-
 // ---- the kernel ------------------------------------------------------------------------
 
 // kMask: 0 none, 1 a row per (batch, head), 2 a plan (a row per query).
 // kMixed: of the items some are pairs of tiles and some halves of one (last_round_in_halves).
-// kRows: behind the tiles come items of one query row (last_row_apart).
 // kTurns: where P overwrites the scores a tile's products and its softmax are one chain, and two tiles that
 // run in step wait for the tensor cores at the same time and then for the exponentials. Taking turns at the
 // exponentials, the products of one run under those of the other.
-template <int DP, int kMask, bool kTurns, bool kMixed, bool kRows>
+template <int DP, int kMask, bool kTurns, bool kMixed>
 __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const PairParams tp) {
@@ -474,7 +336,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             if (i >= P::bWorkFree && i < P::bWorkFree + P::kQueue) count = 10;   // the softmax and the MMA warps
             // Pair: both tiles release every ring tile. Dual: each has one user, but they share Q. (Mixed: one
             // user, or tile A alone, releases twice.)
-            if (i == P::bRow) count = 8;
             if (i >= P::bKVEmpty && (kMixed || !all_dual)) count = 2;
             if (i == P::bQFree && (kMixed || all_dual)) count = 2;
             mbar_init(bar(i), count);
@@ -573,20 +434,15 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
         // the CTAs out less well at the end.
         const bool ahead = tp.grouped != 0;
         int w_next = ahead ? draw() : 0;
-        bool rows = false;
         for (int n = 0; ok;) {
-            // A row needs no loads, which hold back the drawing of tiles: one at work and one waiting.
-            if (kRows && rows && n >= 2) wait_for(P::bWorkFree + (n - 2) % P::kQueue, ((n - 2) / P::kQueue) & 1, 125);
-            if (!ok) break;
             const int w = ahead ? w_next : draw();
             Item k;
             k.b = -1;
             if (w >= 0) {
                 if (ahead) w_next = draw();
                 if (w >= tp.work) continue;   // the fixed deal's last round
-                k = decode_item<kRows>(tp, w);
+                k = decode_item(tp, w);
                 if (!k.valid[0]) continue;
-                if (kRows && k.dual == kRow) rows = true;
                 if constexpr (kMask == 2) apply_plan(tp, k);
             }
             const int q_slot = n % P::kQueue;
@@ -816,11 +672,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
         int turns = 0;      // turns taken so far, the same number by either tile
         const uint32_t my_turn = bar(P::bTurn + t * 4 + (warp & 3)), their_turn = bar(P::bTurn + (1 - t) * 4 + (warp & 3));
 
-        int n = 0;
-        for (; ok; ++n) {
+        for (int n = 0; ok; ++n) {
             Item k;
             if (!take_item(n, k, ok)) break;
-            if (kRows && k.dual == kRow) break;   // the tiles are done
             if (!(t ? k.valid[1] : k.valid[0])) {
                 give_item(n);
                 continue;
@@ -1215,21 +1069,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) fwd_pair_kernel(
             }
             give_item(n);
         }
-        if constexpr (kRows) {
-            // Rows are the last of the list. (A loop of their own: beside the scores they find no registers.)
-#pragma unroll 1
-            for (int phase = 0; ok; ++n) {
-                Item k;
-                if (!take_item(n, k, ok)) break;
-                if (phase == 0) {   // Both tiles are done with all that the parts are written over.
-                    mbar_arrive_warp(bar(P::bRow));
-                    ok = wait_one(bar(P::bRow), 0, abort_flag, 394);
-                    if (!ok) break;
-                }
-                ok = row_alone<DP>(p, k, reinterpret_cast<float*>(smem + P::kQ), bar(P::bRow), ++phase, abort_flag);
-                if (ok) give_item(n);
-            }
-        }
     }
 
     // Teardown: everyone arrives (all waits above are bounded), then the allocating warp frees
@@ -1507,20 +1346,16 @@ template <int DP>
 int launch_pair(const AttnParams& p, const CUtensorMap (&maps)[3], PairParams& tp, int grid, cudaStream_t stream) {
     using P = PairPlan<DP>;
     const bool none = p.mask_dtype == KTT_B200_MASK_NONE, mixed = tp.cut > 0;
-    const bool rows = tp.rows_from < tp.work;
-    auto kernel = mask_needs_plan(p) ? fwd_pair_kernel<DP, 2, false, false, false>
-                : rows ? fwd_pair_kernel<DP, 0, false, false, true>
-                : none ? (mixed ? fwd_pair_kernel<DP, 0, false, true, false> : fwd_pair_kernel<DP, 0, false, false, false>)
-                       : (mixed ? fwd_pair_kernel<DP, 1, false, true, false> : fwd_pair_kernel<DP, 1, false, false, false>);
+    auto kernel = mask_needs_plan(p) ? fwd_pair_kernel<DP, 2, false, false>
+                : none ? (mixed ? fwd_pair_kernel<DP, 0, false, true> : fwd_pair_kernel<DP, 0, false, false>)
+                       : (mixed ? fwd_pair_kernel<DP, 1, false, true> : fwd_pair_kernel<DP, 1, false, false>);
     if constexpr (P::kPOverS) {
         // Turns, without a mask, for pairs from five blocks of keys on: with three, their waits and the code for them
         // weigh more. Measured, us without and with: D 80, 16 heads x 4096 167 -> 153; D 96, 48 x 1025 52.5 ->
         // 49.3; D 80, 32 x 2048 causal 46.9 -> 45.0; 128 x 577 44.4 -> 43.3, 128 x 640 42.3 -> 40.4; but 256 x
         // 257 34.9 -> 35.9, D 128, 10 x 2048 queries x 300 keys 12.7 -> 13.4, and halves, D 80, 8 x 935 14.3 -> 14.6. (Head dims up to 64, whose scores
         // are ready in any case: 157 both, 20 x 4096. Masks with a row per query, D 128, 32 x 2048: 68.7 -> 71.1.)
-        if (none && tp.duals > 0 && p.sk > 4 * kBN) {
-            kernel = rows ? fwd_pair_kernel<DP, 0, true, false, true> : mixed ? fwd_pair_kernel<DP, 0, true, true, false> : fwd_pair_kernel<DP, 0, true, false, false>;
-        }
+        if (none && tp.duals > 0 && p.sk > 4 * kBN) kernel = mixed ? fwd_pair_kernel<DP, 0, true, true> : fwd_pair_kernel<DP, 0, true, false>;
     }
     if (int rc = ensure_smem(kernel, P::kBytes, "cudaFuncSetAttribute(fwd_pair)")) return rc;
     return launch_dependent(kernel, dim3(grid), kPairThreads, P::kBytes, stream, "fwd_pair launch", maps[0], maps[1], maps[2], tp);
@@ -1545,25 +1380,10 @@ bool forward_pair_takes(const AttnParams& p) {
 }
 
 namespace {
-// One row behind the last whole tile (a class token), where the whole tiles of a K / V head are all in pairs: a tile
-// for that row costs as much as any other, and SMs that the last round of pairs leaves idle can take the rows
-// by CUDA cores instead. Measured, us, a tile for the row -> apart: pairs of one round 96 x 257, D 96 19.0 -> 14.4,
-// 75 x 257 17.2 -> 14.0, 56 x 513 25.4 -> 19.5, 32 x 1025 40.0 -> 30.0; more rounds, the last more than half full:
-// 256 x 257, D 80 34.4 -> 31.9, 384 x 257 48.9 -> 44.7, 128 x 513 39.9 -> 38.7, 96 x 1025 83.8 -> 77.5. Not where the
-// last round runs in halves (150 x 257 24.2 -> 26.2, 64 x 769 39.9 -> 41.8, 80 x 1025 68.2 -> 72.3), nor, beyond one
-// round, from ten blocks of keys on (48 x 1281 57.2 -> 59.5): a row is one chain through its keys.
-bool last_row_apart(const AttnParams& p) {
-    if (p.causal || p.cu_q || p.mask_dtype != KTT_B200_MASK_NONE || p.sq % kBM != 1) return false;
-    const int64_t sms = sm_count(), per_plane = static_cast<int64_t>(p.sq / kBM) * (p.heads / p.kv_heads);
-    const int64_t tiles = per_plane * p.kv_heads * p.batch, pairs = tiles / 2, over = pairs % sms;
-    if (per_plane % 2 || tiles <= sms) return false;
-    return pairs <= sms || ((over == 0 || 2 * over > sms) && p.sk <= 9 * kBN);
-}
-
 // Pairs of equal length in rounds of one per SM, the last of which leaves half of the SMs or more without one:
 // its tiles run as halves, each on an SM of its own.
 bool last_round_in_halves(const AttnParams& p) {
-    if (p.causal || p.cu_q || p.key_lengths || mask_needs_plan(p) || p.sk <= kBN || last_row_apart(p)) return false;
+    if (p.causal || p.cu_q || p.key_lengths || mask_needs_plan(p) || p.sk <= kBN) return false;
     const int64_t sms = sm_count(), group = p.heads / p.kv_heads, planes = static_cast<int64_t>(p.batch) * p.kv_heads;
     const int64_t per_plane = (p.sq + kBM - 1) / kBM * group, pairs = (per_plane + 1) / 2 * planes, over = pairs % sms;
     return per_plane * planes > sms && pairs > sms && over > 0 && 2 * over <= sms;
@@ -1800,9 +1620,7 @@ int launch_whole(const AttnParams& p, void* workspace, int64_t workspace_bytes, 
     // tried: 16 x 16 heads x 257, D 80: 43 -> 37 us without it, 4 x 16 heads 19 -> 13; 2 x 16 heads x
     // 2048, D 64, causal mask: 71 -> 58. At 8 heads x 2 x 1024, D 80, 128 tiles, it gives 25 -> 16.)
     const bool dual = p.sk > kBN && units <= sms;
-    const bool row_apart = last_row_apart(p);
-    const int tiles = row_apart ? q_tiles - 1 : q_tiles;
-    const int levels = dual ? tiles * group : (tiles * group + 1) / 2;
+    const int levels = dual ? q_tiles * group : (q_tiles * group + 1) / 2;
     tp.work = levels * p.kv_heads * p.batch;
     tp.duals = dual ? 0 : tp.work;
     tp.cut = 0;
@@ -1811,8 +1629,6 @@ int launch_whole(const AttnParams& p, void* workspace, int64_t workspace_bytes, 
         tp.cut = tp.duals = tp.work - over;
         tp.work += over;
     }
-    tp.rows_from = tp.work;
-    if (row_apart) tp.work += p.heads * p.batch;
     tp.by_batch = divisor_of(p.batch);
     tp.by_kv_heads = divisor_of(p.kv_heads);
     tp.by_group = divisor_of(group);
