@@ -907,28 +907,6 @@ int cluster_room(int ranks) {
     return room - 1;
 }
 
-// CTAs per (batch, kv head) pair where each pair has a cluster of its own; 0 where the pairs are cut into equal
-// shares. A cluster's partials meet in shared memory, its first tiles are on their way before the length is
-// known, and no CTA has a second pair to end: 5 us less than the shares with their tickets. But a pair is as
-// long as it is, and a cluster of it as slow; with 1,024 keys to a rank that costs at most what it saves.
-// Measured on B200, us, shares and clusters, lengths U[n / 8, n]: 14 heads over 2, D 64, one sequence of 1,024
-// 7.0 and 4.4; 16 over 2, D 128: 1 x 4096 10.5 and 8.5 (8 ranks), 16 x 4096 16.6 and 13.5, 64 x 1024 (2 ranks)
-// 16.8 and 14.2, but 64 x 4096 33.9 and 35.8; 32 over 8, D 128: 8 x 4096 (4 ranks) 21.6 and 20.6, 32 x 1024 (1
-// rank) 22.7 and 21.3; equal lengths 8 x 4096 29.1 and 25.1. Clusters of 16: 8.1 where 8 took 8.9 at most, 12.4
-// where they took 7.4 at worst.
-template <int D, int NS, bool kAppend>
-int decode_ranks(const ktt_b200_decode_args* a) {
-    const int64_t pairs = static_cast<int64_t>(a->batch) * a->kv_heads, ctas = stream_ctas_for_device();
-    for (int ranks = 8; ranks >= 1; ranks /= 2) {
-        if (a->splits > 0 && ranks > a->splits) continue;
-        if (ranks > 1 && (ranks / 2) * kTile >= a->sk) continue;   // half as many have a tile each
-        if (pairs * ranks > ctas) continue;
-        if (cluster_room<D, NS, kAppend>(ranks) < pairs) continue;
-        return a->sk <= 1024 * ranks ? ranks : 0;
-    }
-    return 0;
-}
-
 int decode_ctas(const ktt_b200_decode_args* a) {
     // `splits` bounds the CTAs per (batch, kv head) pair; 0 lets the device size decide.
     int ctas = stream_ctas_for_device();
@@ -938,6 +916,34 @@ int decode_ctas(const ktt_b200_decode_args* a) {
     }
     if (ctas > kMaxCtas) ctas = kMaxCtas;
     return ctas < 1 ? 1 : ctas;
+}
+
+// CTAs per (batch, kv head) pair where each pair has a cluster of its own; 0 where the pairs are cut into equal
+// shares. A cluster's partials meet in shared memory, and no CTA has a second pair to end. But a pair is as long as
+// it is, and a cluster of it as slow, and CTAs that clusters leave out have no share of the work.
+// Measured on B200, us, shares and clusters, lengths U[n / 8, n]: 14 heads over 2, D 64, one sequence of 1,024
+// 7.0 and 5.3; 16 over 2, D 128: 1 x 4096 10.2 and 8.2 (8 ranks), 16 x 4096 16.9 and 14.3, 64 x 1024 (2 ranks) 18.3
+// and 15.5; equal lengths, 32 over 8, D 64, 8 x 3072 (4 ranks) 18.5 and 15.2. The line, 32 over 8, D 128: 160 CTAs in
+// clusters, of 1,024 keys each 17.7 and 20.4 (2 ranks), 18.4 and 21.1 (1 rank), of 768 16.5 and 17.5, 17.8 and 17.5,
+// of 512 13.6 and 13.6, 15.4 and 13.8; 256 CTAs of 1,024 keys 19.7 and 19.6 (4 ranks), 22.6 and 22.6 (2), 23.9 and
+// 22.6 (1); 288 of them, of 700 keys, 20.8 and 17.7. Eight ranks: 2, 16 and 32 pairs of 8,192 keys 12.7 and 11.5, 16.0 and
+// 14.5, 22.1 and 19.8. What it costs where one sequence is long and all others have up to 64 keys: 12.7 and 15.7 at
+// most (8 x 3072, 4 ranks). Clusters of 16: 8.1 where 8 took 8.9 at most, 12.4 where they took 7.4 at worst.
+template <int D, int NS, bool kAppend>
+int decode_ranks(const ktt_b200_decode_args* a) {
+    const int64_t pairs = static_cast<int64_t>(a->batch) * a->kv_heads, ctas = stream_ctas_for_device();
+    for (int ranks = 8; ranks >= 1; ranks /= 2) {
+        if (a->splits > 0 && ranks > a->splits) continue;
+        if (ranks > 1 && (ranks / 2) * kTile >= a->sk) continue;   // half as many have a tile each
+        if (pairs * ranks > ctas) continue;
+        if (cluster_room<D, NS, kAppend>(ranks) < pairs) continue;
+        // Keys of a rank, 1024 at most, and where clusters use fewer CTAs than shares would, as many times fewer
+        // of them. (A rank each: 7 / 6 of that.)
+        const int64_t used = pairs * ranks * (ranks == 1 ? 7 : 6), all = static_cast<int64_t>(decode_ctas(a)) * 6;
+        const int64_t most = 1024 * ranks;
+        return a->sk <= most && (ranks == 8 || a->sk * all <= most * used) ? ranks : 0;
+    }
+    return 0;
 }
 
 const char* decode_refusal(const ktt_b200_decode_args* a) {
