@@ -164,7 +164,8 @@ KTT_B200_API const char* ktt_b200_last_error(void);
 
 /* ktt_counters (ktt_capi.h:24-26) reduced to this path: out[8] = forward calls on the
  * tcgen05 kernel, forward calls on the warp-MMA kernel, backward calls, decode calls,
- * refused calls, device-wait timeouts, backward calls on the tcgen05 kernels, reserved. */
+ * refused calls, device-wait timeouts, backward calls on the tcgen05 kernels, kernels set up
+ * (once per kernel and device, at its first use or before). */
 KTT_B200_API int ktt_b200_counters(int64_t* out8);
 KTT_B200_API int ktt_b200_reset_counters(void);
 
@@ -262,7 +263,8 @@ KTT_B200_API int64_t ktt_b200_sdpa_backward_workspace(const ktt_b200_attn_args* 
  * (ktt_capi.h:126-135), bridge::sdpa_varlen_backward, bridge::sdpa_lengths_backward. */
 KTT_B200_API int ktt_b200_sdpa_backward(const ktt_b200_attn_args* args, void* stream);
 
-/* Split-K decode against a static KV cache. */
+/* Split-K decode against a static KV cache. The first call on a device with a head dim does the one-time
+ * set-up for all calls with that head dim, whatever their size; ktt_b200_decode_append has its own. */
 KTT_B200_API int64_t ktt_b200_decode_scratch_bytes(const ktt_b200_decode_args* args);
 KTT_B200_API int ktt_b200_decode(const ktt_b200_decode_args* args, void* stream);
 
@@ -270,12 +272,13 @@ KTT_B200_API int ktt_b200_decode(const ktt_b200_decode_args* args, void* stream)
  * server that hands out all of the GPU at start-up and gives a plugin only input and
  * output buffers; a decode loop that cannot afford the device-wide stall a cudaMalloc can
  * cause). It has no counterpart in the reference. The split-K partials go to a fixed
- * 4 MiB array inside the library, so args->scratch and args->scratch_bytes are ignored
- * and the call makes no allocation of any kind.
+ * 4 MiB array inside the library (where few pairs have a cluster of CTAs each, they stay on
+ * chip), so args->scratch and args->scratch_bytes are ignored and the call makes no
+ * allocation of any kind.
  *  - A call whose partials exceed 4 MiB (more than 207 (batch, kv head) pairs at head dim
  *    128 on a 148-SM GPU, 696 at head dim 64) is refused with KTT_B200_ERR_UNSUPPORTED.
- *  - The first call on a device does a one-time set-up (address of the array, kernel
- *    attributes); make it before any stream capture.
+ *  - The first call on a device does the one-time set-up for calls of every size (address of the
+ *    array, attributes of all kernels such a call may take); make it before any stream capture.
  *  - Every call on a device uses the same array. It needs no clearing between calls, but
  *    calls that overlap on the GPU (different streams, no ordering) corrupt each other:
  *    keep them on one stream or order them with events.

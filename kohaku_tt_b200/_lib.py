@@ -341,6 +341,7 @@ COUNTER_NAMES = (
     "attention_refused",
     "device_wait_timeouts",
     "attention_backward_flash",
+    "kernel_setups",
 )
 
 

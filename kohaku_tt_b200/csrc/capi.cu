@@ -44,7 +44,7 @@ bool smem_limit_known(const void* kernel, int device) {
 
 void smem_limit_remember(const void* kernel, int device) {
     std::lock_guard<std::mutex> lock(g_smem_mutex);
-    g_smem_done.insert({kernel, device});
+    if (g_smem_done.insert({kernel, device}).second) note_call(7);
 }
 
 namespace {

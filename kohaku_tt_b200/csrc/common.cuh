@@ -196,7 +196,7 @@ __device__ __forceinline__ void cp_async_wait() {
 int fail(int code, const char* fmt, ...);
 int check_cuda(cudaError_t e, const char* what);
 // Counter slots: 0 tcgen05 forward, 1 warp-MMA forward, 2 backward, 3 decode,
-// 4 refused, 5 device-wait timeouts, 6 tcgen05 backward.
+// 4 refused, 5 device-wait timeouts, 6 tcgen05 backward, 7 kernels set up (smem_limit_remember).
 void note_call(int which);
 
 // Raises a kernel's dynamic shared-memory limit once per (kernel, device): the attribute
@@ -206,17 +206,19 @@ bool smem_limit_known(const void* kernel, int device);   // capi.cu
 void smem_limit_remember(const void* kernel, int device);
 
 template <typename K>
-int ensure_smem(K kernel, int bytes, const char* what) {
+cudaError_t raise_smem_limit(K kernel, int bytes) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
     const void* key = reinterpret_cast<const void*>(kernel);
-    if (smem_limit_known(key, dev)) return 0;
-    if (int rc = check_cuda(
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), what)) {
-        return rc;
-    }
-    smem_limit_remember(key, dev);
-    return 0;
+    if (smem_limit_known(key, dev)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) smem_limit_remember(key, dev);
+    return e;
+}
+
+template <typename K>
+int ensure_smem(K kernel, int bytes, const char* what) {
+    return check_cuda(raise_smem_limit(kernel, bytes), what);
 }
 
 // Launchers (one per kernel family).

@@ -36,6 +36,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "kept.h"
 
 namespace ktt {
 
@@ -828,13 +829,11 @@ int stream_ctas_for_device() {
     static std::atomic<int> known[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 2 * 148;
-    int sms = known[dev].load(std::memory_order_relaxed);
-    if (sms == 0) {
-        sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        known[dev].store(sms, std::memory_order_relaxed);
-    }
-    return 2 * sms;
+    const int sms = kept(known[dev], [&]() {
+        int n = 0;
+        return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : -1;
+    });
+    return 2 * (sms > 0 ? sms : 148);
 }
 
 template <int D, int NS, bool kCluster>
@@ -886,25 +885,46 @@ ScratchLayout scratch_layout(int batch, int kv_heads, int d, int ctas) {
 }
 
 // Clusters of `ranks` CTAs that run at the same time on the current device (8 to a GPC's 16 to 20 SMs of two
-// CTAs each leave some of them out); asked for once per kernel, size and device.
+// CTAs each leave some of them out); asked for once per kernel, size and device. -1: there is no answer now, and
+// the call does without clusters.
 template <int D, int NS, bool kAppend>
 int cluster_room(int ranks) {
-    static std::atomic<int> known[64][4];   // by log2 of the ranks; 0: not asked yet, else one more than the answer
+    static std::atomic<int> known[64][4];   // by log2 of the ranks
     int dev = 0, log = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
     while ((1 << log) < ranks) ++log;
-    int room = known[dev][log].load(std::memory_order_relaxed);
-    if (room == 0) {
+    return kept(known[dev][log], [&]() {
         auto kernel = decode_kernel<D, NS, kAppend, true>;
         cudaLaunchAttribute attr[1];
         cudaLaunchConfig_t cfg = decode_config<D, NS, true>(ranks, ranks, nullptr, attr);
         int n = 0;
-        if (ensure_smem(kernel, static_cast<int>(cfg.dynamicSmemBytes), "cudaFuncSetAttribute(decode)") != 0 ||
-            cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
-        room = n + 1;
-        known[dev][log].store(room, std::memory_order_relaxed);
-    }
-    return room - 1;
+        if (raise_smem_limit(kernel, static_cast<int>(cfg.dynamicSmemBytes)) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess) return n;
+        cudaGetLastError();   // not this call's failure
+        return -1;
+    });
+}
+
+// What the calls of one kind need once per device, whatever their size: the limits of both kernels and the room
+// for clusters. Which kernel a call takes depends on its size, so that all of it is done by the first one.
+template <int D, int NS, bool kAppend>
+int decode_set_up() {
+    static std::atomic<int> done[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int rc = 0;
+    kept(done[dev], [&]() {
+        cudaLaunchAttribute attr[1];
+        rc = ensure_smem(decode_kernel<D, NS, kAppend, false>, static_cast<int>(decode_config<D, NS, false>(1, 1, nullptr, attr).dynamicSmemBytes),
+                         "cudaFuncSetAttribute(decode)");
+        int least = rc;
+        for (int ranks = 1; ranks <= 8; ranks *= 2) {
+            const int room = cluster_room<D, NS, kAppend>(ranks);
+            least = room < least ? room : least;
+        }
+        return least < 0 ? -1 : 0;
+    });
+    return rc;
 }
 
 int decode_ctas(const ktt_b200_decode_args* a) {
@@ -962,6 +982,7 @@ const char* decode_refusal(const ktt_b200_decode_args* a) {
 
 template <int D, int NS, bool kAppend>
 int run_on(const ktt_b200_decode_args* a, DecodeParams& p, int ctas, cudaStream_t stream) {
+    if (int rc = decode_set_up<D, NS, kAppend>()) return rc;
     p.ranks = decode_ranks<D, NS, kAppend>(a);
     if (p.ranks > 0) return launch<D, NS, kAppend, true>(p, a->batch * a->kv_heads * p.ranks, stream);
     return launch<D, NS, kAppend, false>(p, ctas, stream);
@@ -1123,8 +1144,8 @@ int static_scratch_address(unsigned char** out) {
 //  - The partials of the call must fit 4 MiB (see kStaticScratchBytes); a larger problem is
 //    refused with KTT_B200_ERR_UNSUPPORTED and a message that names both sizes. Use
 //    ktt_b200_decode with caller scratch for those.
-//  - The first call on each device looks up the array's device address and raises the
-//    kernel's shared-memory limit. Make that first call outside of any stream capture.
+//  - The first call on each device looks up the array's device address and sets up the
+//    kernels of both head dims. Make that first call outside of any stream capture.
 //  - All calls on a device share the one array. Nothing in it has to be cleared between
 //    calls (the array starts zeroed with the module, the ticket counters are put back to
 //    zero by the kernel, every other word is written before it is read), but two calls whose kernels
@@ -1145,5 +1166,6 @@ extern "C" int ktt_b200_decode_static(const ktt_b200_decode_args* a, void* strea
     }
     unsigned char* base = nullptr;
     if (int rc = static_scratch_address(&base)) return rc;
+    if (int rc = a->d == 64 ? decode_set_up<128, 3, false>() : decode_set_up<64, 6, false>()) return rc;   // (the call's own: below)
     return run_decode(a, base, lay, ctas, stream, "decode_static");
 }
