@@ -957,11 +957,11 @@ int decode_ranks(const ktt_b200_decode_args* a) {
         if (ranks > 1 && (ranks / 2) * kTile >= a->sk) continue;   // half as many have a tile each
         if (pairs * ranks > ctas) continue;
         if (cluster_room<D, NS, kAppend>(ranks) < pairs) continue;
-        // Keys of a rank, 1024 at most, and where clusters use fewer CTAs than shares would, as many times fewer
-        // of them. (A rank each: 7 / 6 of that.)
+        // Keys of a rank, 1024 at most, and beyond 512 as many times fewer as clusters use fewer CTAs than shares
+        // would. (A rank each: 7 / 6 of that.)
         const int64_t used = pairs * ranks * (ranks == 1 ? 7 : 6), all = static_cast<int64_t>(decode_ctas(a)) * 6;
         const int64_t most = 1024 * ranks;
-        return a->sk <= most && (ranks == 8 || a->sk * all <= most * used) ? ranks : 0;
+        return a->sk <= most && (ranks == 8 || 2 * a->sk <= most || a->sk * all <= most * used) ? ranks : 0;
     }
     return 0;
 }
