@@ -1652,9 +1652,13 @@ int launch_whole(const AttnParams& p, void* workspace, int64_t workspace_bytes, 
     const bool large = kv_bytes > (96ll << 20);
     // The counter pays when a CTA gets several items; with one or two the fixed deal (longest
     // first, snake order) is as even and saves the trip to the counter before each item's first
-    // load. A workspace of 4 to 255 bytes is one int32 the caller zeroes before every call.
-    const bool header = usable && workspace_bytes >= kHeaderBytes;
-    const bool drawn = header ? tp.work > 2 * static_cast<int64_t>(sms) : workspace && (reinterpret_cast<uintptr_t>(workspace) & 3) == 0 && workspace_bytes >= 4;
+    // load. A workspace of 4 to 255 bytes is one int32 the caller zeroes before every call; not at head
+    // dim 64, where a caller cannot know which kernel takes the call, and the other one has no
+    // use for less than the whole header, 16-byte aligned.
+    const bool narrow = p.d == 64 && p.dv == 64;
+    const bool words = workspace && (reinterpret_cast<uintptr_t>(workspace) & 3) == 0;
+    const bool header = (narrow ? usable : words) && workspace_bytes >= kHeaderBytes;
+    const bool drawn = header ? tp.work > 2 * static_cast<int64_t>(sms) : !narrow && words && workspace_bytes >= 4;
     tp.work_counter = drawn ? static_cast<int*>(workspace) : nullptr;
     tp.done_counter = drawn && header ? static_cast<int*>(workspace) + 1 : nullptr;
     tp.grouped = drawn && large ? 1 : 0;
