@@ -193,8 +193,8 @@ KTT_B200_API int ktt_b200_probe_read(const void* data, int64_t bytes, int32_t* s
 /* Debug dump of one query tile, the counterpart of the reference's FLASH_DUMP build
  * (ktt_flash/program.hpp:56-65, aten_attention.cpp:814-831: `_debug_flash_dump(q, k, v,
  * is_causal, row)`, the intermediate tiles of one query tile row). While a device buffer is
- * set, every head-dim-64 tcgen05 forward launch runs its traced instantiation, and the
- * tile (batch, head, q_tile: rows q_tile * 128 ..) writes out what its row threads hold,
+ * set, AUTO keeps head dim 64 on the two-stream kernel wherever that takes the call, every launch
+ * of which runs its traced instantiation, and the tile (batch, head, q_tile: rows q_tile * 128 ..) writes out what its row threads hold,
  * straight from their registers:
  *   per key block j < max_blocks, KTT_B200_DUMP_BLOCK_FLOATS floats:
  *     x [128][128]   the exponents, logit * scale * log2(e) (+ mask term) - reference, -inf
@@ -216,7 +216,9 @@ KTT_B200_API int ktt_b200_set_dump(float* device_buffer, int32_t batch, int32_t 
 
 /* Profiling zones, the counterpart of the reference's FLASH_PROFILE device zones
  * (ktt_flash/compute.cpp:25-30, program.hpp:56-65): with a device buffer of 64 x 8 int64
- * set, CTA (0, 0, 0) of every tcgen05 forward launch stamps clock64 per key block (slots:
+ * set, AUTO keeps head dims 64 and 128 off the kernel of two tiles per CTA (which writes no
+ * stamps) wherever another tcgen05 kernel takes the call, and
+ * CTA (0, 0, 0) of every launch of those stamps clock64 per key block (slots:
  * S ready, pass 1 done, previous P V done, pass 2 done, P published, MMA lane before the
  * next Q K^T, after the wait for P, after issuing P V), and rows 64 .. 64 + 1023 receive per
  * CTA its start and end on the global nanosecond timer, its SM and its key-block count; the

@@ -1509,8 +1509,10 @@ bool pair_rounds_better(const AttnParams& p) {
 //    one weighs less);
 //  - D 64: 1024 keys, with mask terms 320 (at 1024 keys 26.9 -> 27.9);
 //  - D 128: 320 keys in the first round or with mask terms, else 96 (at 200 keys 20.9 -> 21.9).
-// Without a mask also where its rounds are the better filled ones (pair_rounds_better).
+// Without a mask also where its rounds are the better filled ones (pair_rounds_better). Not while a trace or a dump is
+// asked for, which the other kernels write.
 bool forward_pair_preferred(const AttnParams& p) {
+    if (get_trace_buffer() || (p.d == 64 && get_dump_request().buffer)) return false;
     if (p.cu_q || p.key_lengths || mask_needs_plan(p) || p.d != p.dv || (p.d != 64 && p.d != 128)) return false;
     if (p.mask_dtype == KTT_B200_MASK_NONE && pair_rounds_better(p) && forward_pair_takes(p)) return true;
     if (p.causal) return false;

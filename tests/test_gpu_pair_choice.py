@@ -39,3 +39,34 @@ def test_a_workspace_of_any_size_and_alignment(cuda, b, h, hk, n, d, at, size, f
         if again is not None:
             workspace.fill_(again)
     assert (workspace[at + size:] == fill).all()
+
+
+# A trace and a dump are written by the kernels that took these calls before this one did.
+@pytest.mark.parametrize("b,h,hk,n,sk,d,causal,kernel", [
+    (4, 20, 20, 1000, 1000, 64, True, "fwd_row"), (2, 10, 10, 4096, 77, 64, False, "fwd_row"), (5, 32, 8, 640, 640, 128, True, "fwd_tc5"),
+])
+def test_what_is_traced_stays_with_the_traced_kernels(cuda, b, h, hk, n, sk, d, causal, kernel):
+    q, k, v = (t.to(cuda) for t in qkv(b, h, hk, n, sk, d, n + d))
+    handle = _lib.lib()
+    call = lambda: _forward(q, k, v, causal)
+    assert any("fwd_pair" in x.name for x in launched(call))
+    trace = torch.zeros((64 + 1024) * 8, dtype=torch.int64, device=cuda)
+    handle.ktt_b200_set_trace(trace.data_ptr())
+    try:
+        assert any(kernel in x.name for x in launched(call))
+    finally:
+        handle.ktt_b200_set_trace(None)
+    torch.cuda.synchronize()
+    assert trace[64 * 8] > 0   # the first CTA's start
+    if d == 64:
+        blocks = (sk + 127) // 128
+        dump = torch.full((blocks * (2 * 128 * 128 + 2 * 128) + 128 * 64 + 2 * 128,), float("nan"), device=cuda)
+        assert handle.ktt_b200_set_dump(dump.data_ptr(), b - 1, h - 1, 1, blocks) == 0
+        try:
+            assert any(kernel in x.name for x in launched(call))
+        finally:
+            handle.ktt_b200_set_dump(None, 0, 0, 0, 0)
+        torch.cuda.synchronize()
+        assert dump[-256:].isfinite().all()   # the tile's last maxima and sums
+    assert any("fwd_pair" in x.name for x in launched(call))
+    _lib.device_status()
