@@ -53,6 +53,7 @@
 // host-visible status word, stops waiting everywhere, frees its tensor memory and exits.
 // Launched with programmatic stream serialization: everything before `griddepcontrol.wait`
 // may overlap the tail of the previous kernel in the stream.
+#include "rounds.h"
 #include "tc5.cuh"
 
 namespace ktt {
@@ -1390,51 +1391,7 @@ bool last_round_in_halves(const AttnParams& p) {
 }
 }  // namespace
 
-// The time at which the last of `machines` is done, when each item goes to the first free one: `cost[i]`
-// us of `count[i]` items, the longest first. Machines that are done at the same time are one group.
 namespace {
-constexpr int kMostLevels = 64;
-float makespan(const float* cost, const int64_t* count, int levels, int64_t machines) {
-    float at[2 * kMostLevels + 2];
-    int64_t of[2 * kMostLevels + 2];
-    int n = 1, first = 0;
-    at[0] = 0.f;
-    of[0] = machines;
-    for (int i = 0; i < levels; ++i) {
-        for (int64_t left = count[i]; left > 0;) {
-            const int64_t take = left < of[first] ? left : of[first];
-            const float done = at[first] + cost[i];
-            left -= take;
-            of[first] -= take;
-            if (of[first] == 0) ++first;
-            int j = n;   // (mostly the last)
-            while (j > first && at[j - 1] > done) --j;
-            if (j > first && at[j - 1] == done) {
-                of[j - 1] += take;
-                continue;
-            }
-            if (n == 2 * kMostLevels + 2) {   // make room at the front; (out of it: the groups are many, and close)
-                if (first == 0) return at[n - 1] > done ? at[n - 1] : done;
-                for (int k = first; k < n; ++k) {
-                    at[k - first] = at[k];
-                    of[k - first] = of[k];
-                }
-                n -= first;
-                j -= first;
-                first = 0;
-            }
-            for (int k = n; k > j; --k) {
-                at[k] = at[k - 1];
-                of[k] = of[k - 1];
-            }
-            at[j] = done;
-            of[j] = take;
-            ++n;
-        }
-    }
-    return at[n - 1];
-}
-
 // Dense calls of head dim 64 or 128 without a mask: whether this kernel's pairs of tiles fill their rounds so
 // much better than the other kernel's tiles (D 64: two halves of a tile's keys at a time, from six tiles per SM
 // on whole tiles in two streams; D 128: whole tiles) that it ends sooner by the estimate below. What a call, an

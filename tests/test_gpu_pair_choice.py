@@ -70,3 +70,23 @@ def test_what_is_traced_stays_with_the_traced_kernels(cuda, b, h, hk, n, sk, d, 
         assert dump[-256:].isfinite().all()   # the tile's last maxima and sums
     assert any("fwd_pair" in x.name for x in launched(call))
     _lib.device_status()
+
+
+# On 148 SMs. One round of tiles stays with the kernel of whole tiles; beyond it the kernel whose rounds are better filled
+# takes the call. `kind`: of the paired kernel, turns (head dim 128, five blocks of keys on) and a last round in halves.
+@pytest.mark.parametrize("b,h,hk,n,d,causal,kernel,kind", [
+    (8, 14, 2, 512, 64, True, "pair", "00"), (2, 32, 8, 1024, 64, True, "pair", "00"), (4, 20, 20, 200, 64, True, "pair", "00"),
+    (1, 20, 20, 1024, 64, False, "pair", "00"), (1, 20, 20, 4096, 64, False, "pair", "01"), (2, 20, 20, 1000, 64, False, "pair", "01"),
+    (8, 16, 16, 200, 128, True, "pair", "00"), (8, 14, 2, 640, 128, True, "pair", "10"), (3, 24, 24, 257, 128, False, "pair", "00"),
+    (1, 14, 2, 1024, 64, True, "row", ""), (1, 14, 2, 2048, 64, True, "row", ""), (4, 20, 20, 257, 64, True, "row", ""),
+    (4, 20, 20, 640, 64, False, "row", ""), (8, 14, 2, 1000, 64, True, "row", ""), (1, 37, 37, 512, 64, True, "row", ""),
+    (1, 20, 20, 1024, 128, False, "tc5", ""), (3, 24, 24, 513, 128, False, "tc5", ""), (2, 20, 20, 1024, 128, True, "tc5", ""),
+    (3, 24, 24, 384, 128, True, "tc5", ""), (1, 37, 37, 512, 128, True, "tc5", ""),
+])
+def test_the_kernel_a_call_takes(cuda, b, h, hk, n, d, causal, kernel, kind):
+    q = torch.zeros(b, h, n, d, dtype=torch.bfloat16, device=cuda)
+    k = torch.zeros(b, hk, n, d, dtype=torch.bfloat16, device=cuda)
+    (one,) = [x for x in launched(lambda: _forward(q, k, k, causal)) if "fwd_" in x.name]
+    assert f"fwd_{kernel}_kernel" in one.name
+    if kind:
+        assert f"fwd_pair_kernelILi{d}ELi0ELb{kind[0]}ELb{kind[1]}E" in one.name

@@ -1,8 +1,10 @@
 """Host code of csrc/ that needs no CUDA, compiled by g++ and checked here against plain restatements."""
 
-import os
+import heapq
+import random
 import subprocess
 
+import numpy as np
 import pytest
 
 from kohaku_tt_b200 import _lib
@@ -35,3 +37,37 @@ int main(int argc, char** argv) {
 }
 ''', len(want), *answers)
     assert [int(x) for x in lines[:-1]] == want + [asked]
+
+
+def _list_schedule(cost, count, machines):
+    free = [np.float32(0)] * machines
+    for c, n in zip(cost, count):
+        for _ in range(n):
+            heapq.heapreplace(free, np.float32(free[0] + c))
+    return max(free)
+
+
+# Up to 128 levels (and as many groups of machines), equal and unequal costs, more and fewer items than machines.
+@pytest.mark.parametrize("levels,most,machines,steps", [
+    (1, 400, 148, 1), (4, 60, 148, 3), (64, 40, 148, 1000), (128, 3, 296, 10**6), (128, 30, 148, 10**6), (128, 9, 7, 10**6), (65, 1, 148, 2), (64, 300, 1, 50),
+])
+def test_makespan_is_list_scheduling(tmp_path, levels, most, machines, steps):
+    rng = random.Random(levels * machines)
+    cost = np.array(sorted((rng.randint(1, steps) * 0.37 for _ in range(levels)), reverse=True), dtype=np.float32)
+    count = [rng.randint(0, most) for _ in range(levels)]
+    lines = run(tmp_path, '''
+#include <cstdio>
+#include <cstdlib>
+#include "rounds.h"
+int main(int argc, char** argv) {
+    const int levels = (argc - 2) / 2;
+    static float cost[2 * ktt::kMostLevels];
+    static int64_t count[2 * ktt::kMostLevels];
+    for (int i = 0; i < levels; ++i) {
+        cost[i] = std::strtof(argv[2 + 2 * i], nullptr);
+        count[i] = std::atoll(argv[3 + 2 * i]);
+    }
+    std::printf("%.9g\\n", static_cast<double>(ktt::makespan(cost, count, levels, std::atoll(argv[1]))));
+}
+''', machines, *(x for c, n in zip(cost, count) for x in ("%.9g" % c, n)))
+    assert np.float32(lines[0]) == _list_schedule(cost, count, machines)
