@@ -824,11 +824,17 @@ __global__ void __launch_bounds__(kThreads, 2) decode_kernel(const DecodeParams 
     stamp(5);
 }
 
-// CTAs that run at the same time: two per SM (asked for once per device: a small call is bound by its host side).
-int stream_ctas_for_device() {
-    static std::atomic<int> known[64];
+// The current device, or -1 for one that nothing is kept of. (Asked for once per call: a small call is bound by its
+// host side.)
+int current_device() {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 2 * 148;
+    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? dev : -1;
+}
+
+// CTAs that run at the same time: two per SM.
+int stream_ctas(int dev) {
+    static std::atomic<int> known[64];
+    if (dev < 0) return 2 * 148;
     const int sms = kept(known[dev], [&]() {
         int n = 0;
         return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : -1;
@@ -855,10 +861,9 @@ cudaLaunchConfig_t decode_config(int ctas, int ranks, cudaStream_t stream, cudaL
 
 template <int D, int NS, bool kAppend, bool kCluster>
 int launch(const DecodeParams& p, int ctas, cudaStream_t stream) {
-    auto kernel = decode_kernel<D, NS, kAppend, kCluster>;
+    auto kernel = decode_kernel<D, NS, kAppend, kCluster>;   // (set up: decode_set_up, cluster_room)
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = decode_config<D, NS, kCluster>(ctas, p.ranks, stream, attr);
-    if (int rc = ensure_smem(kernel, static_cast<int>(cfg.dynamicSmemBytes), "cudaFuncSetAttribute(decode)")) return rc;
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
@@ -888,10 +893,10 @@ ScratchLayout scratch_layout(int batch, int kv_heads, int d, int ctas) {
 // CTAs each leave some of them out); asked for once per kernel, size and device. -1: there is no answer now, and
 // the call does without clusters.
 template <int D, int NS, bool kAppend>
-int cluster_room(int ranks) {
+int cluster_room(int dev, int ranks) {
     static std::atomic<int> known[64][4];   // by log2 of the ranks
-    int dev = 0, log = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+    if (dev < 0) return -1;
+    int log = 0;
     while ((1 << log) < ranks) ++log;
     return kept(known[dev][log], [&]() {
         auto kernel = decode_kernel<D, NS, kAppend, true>;
@@ -908,18 +913,19 @@ int cluster_room(int ranks) {
 // What the calls of one kind need once per device, whatever their size: the limits of both kernels and the room
 // for clusters. Which kernel a call takes depends on its size, so that all of it is done by the first one.
 template <int D, int NS, bool kAppend>
-int decode_set_up() {
+int decode_set_up(int dev) {
     static std::atomic<int> done[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     int rc = 0;
-    kept(done[dev], [&]() {
+    auto shares = [&]() {
         cudaLaunchAttribute attr[1];
-        rc = ensure_smem(decode_kernel<D, NS, kAppend, false>, static_cast<int>(decode_config<D, NS, false>(1, 1, nullptr, attr).dynamicSmemBytes),
-                         "cudaFuncSetAttribute(decode)");
-        int least = rc;
+        return rc = ensure_smem(decode_kernel<D, NS, kAppend, false>, static_cast<int>(decode_config<D, NS, false>(1, 1, nullptr, attr).dynamicSmemBytes),
+                                "cudaFuncSetAttribute(decode)");
+    };
+    if (dev < 0) return shares();
+    kept(done[dev], [&]() {
+        int least = shares();
         for (int ranks = 1; ranks <= 8; ranks *= 2) {
-            const int room = cluster_room<D, NS, kAppend>(ranks);
+            const int room = cluster_room<D, NS, kAppend>(dev, ranks);
             least = room < least ? room : least;
         }
         return least < 0 ? -1 : 0;
@@ -929,7 +935,7 @@ int decode_set_up() {
 
 int decode_ctas(const ktt_b200_decode_args* a) {
     // `splits` bounds the CTAs per (batch, kv head) pair; 0 lets the device size decide.
-    int ctas = stream_ctas_for_device();
+    int ctas = stream_ctas(current_device());
     if (a->splits > 0) {
         const int64_t want = static_cast<int64_t>(a->splits) * a->batch * a->kv_heads;
         if (want < ctas) ctas = static_cast<int>(want);
@@ -950,16 +956,16 @@ int decode_ctas(const ktt_b200_decode_args* a) {
 // 14.5, 22.1 and 19.8. What it costs where one sequence is long and all others have up to 64 keys: 12.7 and 15.7 at
 // most (8 x 3072, 4 ranks). Clusters of 16: 8.1 where 8 took 8.9 at most, 12.4 where they took 7.4 at worst.
 template <int D, int NS, bool kAppend>
-int decode_ranks(const ktt_b200_decode_args* a) {
-    const int64_t pairs = static_cast<int64_t>(a->batch) * a->kv_heads, ctas = stream_ctas_for_device();
+int decode_ranks(const ktt_b200_decode_args* a, int shares, int dev) {   // shares: CTAs without clusters (decode_ctas)
+    const int64_t pairs = static_cast<int64_t>(a->batch) * a->kv_heads, ctas = stream_ctas(dev);
     for (int ranks = 8; ranks >= 1; ranks /= 2) {
         if (a->splits > 0 && ranks > a->splits) continue;
         if (ranks > 1 && (ranks / 2) * kTile >= a->sk) continue;   // half as many have a tile each
         if (pairs * ranks > ctas) continue;
-        if (cluster_room<D, NS, kAppend>(ranks) < pairs) continue;
+        if (cluster_room<D, NS, kAppend>(dev, ranks) < pairs) continue;
         // Keys of a rank, 1024 at most, and beyond 512 as many times fewer as clusters use fewer CTAs than shares
         // would. (A rank each: 7 / 6 of that.)
-        const int64_t used = pairs * ranks * (ranks == 1 ? 7 : 6), all = static_cast<int64_t>(decode_ctas(a)) * 6;
+        const int64_t used = pairs * ranks * (ranks == 1 ? 7 : 6), all = static_cast<int64_t>(shares) * 6;
         const int64_t most = 1024 * ranks;
         return a->sk <= most && (ranks == 8 || 2 * a->sk <= most || a->sk * all <= most * used) ? ranks : 0;
     }
@@ -982,8 +988,9 @@ const char* decode_refusal(const ktt_b200_decode_args* a) {
 
 template <int D, int NS, bool kAppend>
 int run_on(const ktt_b200_decode_args* a, DecodeParams& p, int ctas, cudaStream_t stream) {
-    if (int rc = decode_set_up<D, NS, kAppend>()) return rc;
-    p.ranks = decode_ranks<D, NS, kAppend>(a);
+    const int dev = current_device();
+    if (int rc = decode_set_up<D, NS, kAppend>(dev)) return rc;
+    p.ranks = decode_ranks<D, NS, kAppend>(a, ctas, dev);
     if (p.ranks > 0) return launch<D, NS, kAppend, true>(p, a->batch * a->kv_heads * p.ranks, stream);
     return launch<D, NS, kAppend, false>(p, ctas, stream);
 }
@@ -1166,6 +1173,7 @@ extern "C" int ktt_b200_decode_static(const ktt_b200_decode_args* a, void* strea
     }
     unsigned char* base = nullptr;
     if (int rc = static_scratch_address(&base)) return rc;
-    if (int rc = a->d == 64 ? decode_set_up<128, 3, false>() : decode_set_up<64, 6, false>()) return rc;   // (the call's own: below)
+    const int dev = current_device();   // (set up for the call's own head dim: below)
+    if (int rc = a->d == 64 ? decode_set_up<128, 3, false>(dev) : decode_set_up<64, 6, false>(dev)) return rc;
     return run_decode(a, base, lay, ctas, stream, "decode_static");
 }
