@@ -41,6 +41,15 @@ def test_a_workspace_of_any_size_and_alignment(cuda, b, h, hk, n, d, at, size, f
     assert (workspace[at + size:] == fill).all()
 
 
+# Halves of a last round, dealt and drawn (344 items for 148 SMs).
+def test_halves_from_a_counter_and_from_a_fixed_deal(cuda):
+    q, k, v = (t.to(cuda) for t in qkv(1, 20, 20, 4096, 4096, 64, 5))
+    workspace = torch.zeros(256, dtype=torch.uint8, device=cuda)
+    drawn = [_forward(q, k, v, False, workspace) for _ in range(2)]
+    dealt = _forward(q, k, v, False)
+    assert torch.equal(drawn[0], dealt) and torch.equal(drawn[1], dealt) and dealt.isfinite().all()
+
+
 # A trace and a dump are written by the kernels that took these calls before this one did.
 @pytest.mark.parametrize("b,h,hk,n,sk,d,causal,kernel", [
     (4, 20, 20, 1000, 1000, 64, True, "fwd_row"), (2, 10, 10, 4096, 77, 64, False, "fwd_row"), (5, 32, 8, 640, 640, 128, True, "fwd_tc5"),
