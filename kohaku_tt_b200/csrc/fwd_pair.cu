@@ -1397,10 +1397,12 @@ namespace {
 // on whole tiles in two streams; D 128: whole tiles) that it ends sooner by the estimate below. What a call, an
 // item, a block and, causal, a diagonal cost (us) is fitted to 490 calls of 20 to 1,200 tiles (D 64 within 5 %
 // rms, D 128 within 4 and 6.5): prompts of 1 to 16 sequences, 100 to 4,096 rows, and non-causal ones of 200 to
-// 4,608. The line is 8 % because none of 610 measured calls on this side of it is slower here (at 3 % four were,
-// by up to 5 %); over all of them that is 4.8 % (D 64) and 1.1 % (D 128) of the time, at most 1.3 times: 8 x 14
-// heads over 2 x 512, D 64, causal 19.7 and 15.7 us, 2 x 32 over 8 x 1024 27.7 and 21.8, 20 heads x 1024 20.7 and
-// 18.4; the other way 1 x 14 over 2 x 2048 causal 19.7 and 30.8, 20 heads x 4096 140 and 157.
+// 4,608. The fit is of the kernels without halves in a last round and without turns, which the estimate has only the
+// first of: at D 128 from five blocks of keys on a block is 1.90 us, not 2.20, so that calls stay with the other kernel there
+// that this one would take as fast. The line is 8 % because none of 610 calls on this side of it, timed in a graph, was
+// slower here (at 3 % four were, by up to 5 %). Timed as calls, 145 sizes on this side are 1.11 times as fast in the
+// mean, at worst 0.98: 8 x 14 heads over 2 x 512, D 64, causal 19.7 and 15.7 us, 2 x 32 over 8 x 1024 27.7 and 21.8, 20
+// heads x 1024 20.7 and 18.4, x 4096 144 and 131; the other way 1 x 14 over 2 x 2048 causal 19.7 and 30.8.
 bool pair_rounds_better(const AttnParams& p) {
     struct Fit { float call, item, block, diagonal; };
     static constexpr Fit kOther[2] = {{2.59f, 2.36f, 1.66f, 0.07f}, {3.62f, 2.55f, 0.95f, 0.42f}};
